@@ -62,6 +62,17 @@ __device__ __forceinline__ T nbs(const T *__restrict__ so, XQ xq, T qf, Dims3 F,
 	else return nb27<T>(so, xq, qf, F, i, j, k);
 }
 
+template <typename T> struct Vec2;
+template <> struct Vec2<float> { using type = float2; };
+template <> struct Vec2<double> { using type = double2; };
+
+// every pointer a multiple of n bytes
+template <typename... P>
+static bool aligned_to(size_t n, const P *...p)
+{
+	return ((reinterpret_cast<uintptr_t>(p) % n == 0) && ...);
+}
+
 template <typename T>
 struct Load3 {
 	const T *__restrict__ q;
@@ -146,19 +157,184 @@ __global__ void k3_recip(const T *__restrict__ so, T *__restrict__ sor, Dims3 F)
 	sor[F.at1(i, j, k)] = T(1) / SO(i, j, k, KP);
 }
 
-// One colour of BMG3_SymStd_relax_GS (src/3d/ftn/BMG3_SymStd_relax_GS.f90:94-136):
-// colour pts has parities (i, j, k) = bits of pts-1.
-template <typename T>
-__global__ void __launch_bounds__(TX *TY) k3_gs_colour(const T *__restrict__ so, T *__restrict__ q,
-                                                       const T *__restrict__ qf, const T *__restrict__ sor, Dims3 F,
-                                                       int pi, int pj, int pk)
+// Two colours of BMG3_SymStd_relax_GS (src/3d/ftn/BMG3_SymStd_relax_GS.f90:94-136)
+// in one pass: the rows (j, k) of one parity pair, first the points of one
+// x-parity, then the others.  A row's second colour depends on the first only
+// inside the row, and rows of one parity pair do not touch each other, so a
+// block that owns whole rows needs no other block: four launches per sweep.
+// Bound by DRAM: a thread takes the points a = 2t, b = 2t + 1 (0-based) and
+// loads every coefficient of both at once, so a row's operator lines are read
+// once with all of their bytes used.  One colour per launch reads every second
+// point of a row, and each line twice.  The second point's terms that the first
+// colour does not change wait as products in registers (24 of 26), so its sum
+// keeps the reference's order and bits.  Rows longer than 2 W points run in
+// segments from the side whose first colour the second one reads.
+// SECOND_A: b first, then a (the sweep UP, colours 1..8); else a, then b (DOWN).
+template <typename T, bool VEC, bool SECOND_A>
+__global__ void __launch_bounds__(256) k3_gs_rows(const T *__restrict__ so, T *__restrict__ q,
+                                                  const T *__restrict__ qf, const T *__restrict__ sor, Dims3 F, int pj,
+                                                  int pk, int nrj, int nrows, int W)
 {
-	const int i = 2 + pi + 2 * (blockIdx.x * TX + threadIdx.x);
-	const int j = 2 + pj + 2 * (blockIdx.y * TY + threadIdx.y);
-	const int k = 2 + pk + 2 * blockIdx.z;
-	if (i > F.nx + 1 || j > F.ny + 1 || k > F.nz + 1) return;
-	const T acc = nb27<T>(so, Load3<T>{q, F}, QF(i, j, k), F, i, j, k);
-	Q(i, j, k) = acc * sor[F.at1(i, j, k)];
+	using V2 = typename Vec2<T>::type;
+	__shared__ T sh[256];   // first-colour values of the segment
+	__shared__ T edge[256]; // per row: the first-colour value the next segment reads
+	const int r = threadIdx.x / W, t0 = threadIdx.x - r * W;
+	const int row = blockIdx.x * (blockDim.x / W) + r;
+	const int nT = F.nx / 2 + 1, nseg = (nT + W - 1) / W;
+	const int rk = row / nrj, j = 1 + pj + 2 * (row - rk * nrj), k = 1 + pk + 2 * rk;
+	const size_t ps = F.plane(), sl = F.slice();
+	const int p = F.pitch;
+	const size_t base = ((size_t)k * (F.ny + 2) + j) * p;
+	for (int s = 0; s < nseg; ++s) {
+		const int t = (SECOND_A ? s : nseg - 1 - s) * W + t0;
+		const bool live = row < nrows && t < nT;
+		const bool va = live && t >= 1, vb = live && 2 * t + 1 <= F.nx;
+		// terms of the second point (index 0 and 4: its row neighbours), the first point's sum
+		T pr[26], c0 = T(0), c4 = T(0), first = T(0), second = T(0), far = T(0), ds = T(0);
+		if (live) {
+			const size_t o = base + 2 * t;
+			auto pair = [&](const T *x, T &a, T &b) {
+				if constexpr (VEC) {
+					const V2 v = *reinterpret_cast<const V2 *>(x);
+					a = v.x;
+					b = v.y;
+				} else {
+					a = x[0];
+					b = x[1];
+				}
+			};
+			// q of a row: left neighbour of a, a, b, right neighbour of b
+			auto row4 = [&](const T *x, T(&v)[4]) {
+				v[0] = t >= 1 ? x[-1] : T(0);
+				pair(x, v[1], v[2]);
+				v[3] = vb ? x[2] : T(0);
+			};
+			T X[4], ca, cb, acc1, f_a, f_b;
+			const T *S = so + o;
+			auto P = [&](int plane) { return S + (size_t)(plane - 1) * ps; };
+			// one term: coefficient of a and of b, iterates of a and of b
+			auto term = [&](int m, T wa, T xa, T wb, T xb) {
+				if (SECOND_A) {
+					acc1 = acc1 + wb * xb;
+					pr[m] = wa * xa;
+				} else {
+					acc1 = acc1 + wa * xa;
+					pr[m] = wb * xb;
+				}
+			};
+			// coefficient planes at the point, and at its right neighbour
+			auto own = [&](int m, const T *c, int x) {
+				pair(c, ca, cb);
+				term(m, ca, X[1 + x], cb, X[2 + x]);
+			};
+			auto right = [&](int m, const T *c, int x) {
+				ca = c[1];
+				cb = vb ? c[2] : T(0);
+				term(m, ca, X[1 + x], cb, X[2 + x]);
+			};
+			pair(qf + o, f_a, f_b);
+			acc1 = SECOND_A ? f_b : f_a;
+			const T f2 = SECOND_A ? f_a : f_b;
+			const T *qo = q + o;
+			T Y[4];
+			row4(qo, Y);
+			T wa, wb, wr;
+			pair(P(KPW), wa, wb);
+			wr = vb ? P(KPW)[2] : T(0);
+			if (SECOND_A) {  // b: left a (old), right a' (old); a waits for both new b
+				acc1 = acc1 + wb * Y[1];
+				c0 = wa;
+				c4 = wb;
+			} else {  // a: left b (old), right b (old); b waits for both new a
+				acc1 = acc1 + wa * Y[0];
+				c0 = wb;
+				c4 = wr;
+			}
+			row4(qo + p, X);
+			own(1, P(KPNW) + p, -1);
+			own(2, P(KPS) + p, 0);
+			right(3, P(KPSW) + p, 1);
+			if (SECOND_A) acc1 = acc1 + wr * Y[3];
+			else acc1 = acc1 + wb * Y[2];
+			row4(qo - p, X);
+			right(5, P(KPNW), 1);
+			own(6, P(KPS), 0);
+			own(7, P(KPSW), -1);
+			row4(qo - sl, X);
+			own(8, P(KB), 0);
+			own(9, P(KBW), -1);
+			T Z[4];
+#pragma unroll
+			for (int m = 0; m < 4; ++m) Z[m] = X[m];
+			row4(qo + p - sl, X);
+			own(10, P(KBNW) + p, -1);
+			own(11, P(KBN) + p, 0);
+			right(12, P(KBNE) + p, 1);
+#pragma unroll
+			for (int m = 0; m < 4; ++m) X[m] = Z[m];
+			right(13, P(KBE), 1);
+			row4(qo - p - sl, X);
+			right(14, P(KBSE), 1);
+			own(15, P(KBS), 0);
+			own(16, P(KBSW), -1);
+			row4(qo + sl, X);
+			own(17, P(KB) + sl, 0);
+			own(18, P(KBE) + sl, -1);
+#pragma unroll
+			for (int m = 0; m < 4; ++m) Z[m] = X[m];
+			row4(qo + p + sl, X);
+			own(19, P(KBSE) + p + sl, -1);
+			own(20, P(KBS) + p + sl, 0);
+			right(21, P(KBSW) + p + sl, 1);
+#pragma unroll
+			for (int m = 0; m < 4; ++m) X[m] = Z[m];
+			right(22, P(KBW) + sl, 1);
+			row4(qo - p + sl, X);
+			right(23, P(KBNW) + sl, 1);
+			own(24, P(KBN) + sl, 0);
+			own(25, P(KBNE) + sl, -1);
+			T sa, sb;
+			pair(sor + o, sa, sb);
+			// a point outside the interior keeps its value
+			if (SECOND_A) first = vb ? acc1 * sb : Y[2];
+			else first = va ? acc1 * sa : Y[1];
+			second = f2;
+			ds = SECOND_A ? sa : sb;
+			far = SECOND_A ? T(0) : Y[3];
+		}
+		sh[threadIdx.x] = first;
+		__syncthreads();  // the segment's row is read, its first colour formed
+		if (live) {
+			T nl, nr;  // new row neighbours of the second point
+			if (SECOND_A) {
+				nl = t0 > 0 ? sh[threadIdx.x - 1] : edge[r];
+				nr = first;
+			} else {
+				nl = first;
+				nr = t + 1 >= nT ? far : t0 + 1 < W ? sh[threadIdx.x + 1] : edge[r];
+			}
+			second = second + c0 * nl;
+			second = second + pr[1] + pr[2] + pr[3] + c4 * nr;
+#pragma unroll
+			for (int m = 5; m < 26; ++m) second = second + pr[m];
+			second = second * ds;
+			T *qo = q + base + 2 * t;
+			const T na = SECOND_A ? second : first, nb = SECOND_A ? first : second;
+			if (VEC && va && vb) {
+				V2 v;
+				v.x = na;
+				v.y = nb;
+				*reinterpret_cast<V2 *>(qo) = v;
+			} else {
+				if (va) qo[0] = na;
+				if (vb) qo[1] = nb;
+			}
+		}
+		if (nseg > 1) {
+			__syncthreads();  // edge and sh are read
+			if (t0 == (SECOND_A ? W - 1 : 0)) edge[r] = first;
+		}
+	}
 }
 
 // One colour of the seven-point branch of BMG3_SymStd_relax_GS
@@ -186,11 +362,24 @@ int relax_point_3d(const T *so, T *x, const T *b, const T *sor, Dims3 F, int upd
 		}
 		return CDR_OK;
 	}
-	const dim3 blk(TX, TY), grd(ceil_div((F.nx + 1) / 2, TX), ceil_div((F.ny + 1) / 2, TY), (F.nz + 1) / 2);
-	for (int c = 0; c < 8; ++c) {
-		const int pts = updown == CDR_UP ? c + 1 : 8 - c;  // UP 1..8, DOWN 8..1
-		const int bits = pts - 1;
-		k3_gs_colour<T><<<grd, blk, 0, st>>>(so, x, b, sor, F, bits & 1, (bits >> 1) & 1, (bits >> 2) & 1);
+	// colours 1..8 (UP) or 8..1 (DOWN) are the parities (i, j, k), i fastest: pairs
+	// of colours share the rows of one (j, k) parity.  W pairs of points per row and
+	// segment, as many rows to a block of 256 threads as fit; two-element accesses
+	// where rows start aligned.
+	const bool vec = F.pitch % 2 == 0 && aligned_to(2 * sizeof(T), so, x, b, sor);
+	const int W = F.nx / 2 + 1 < 256 ? F.nx / 2 + 1 : 256, R = 256 / W;
+	for (int c = 0; c < 4; ++c) {
+		const int bits = updown == CDR_UP ? c : 3 - c, pj = bits & 1, pk = bits >> 1;
+		const int nrj = (F.ny - pj + 1) / 2, nrows = nrj * ((F.nz - pk + 1) / 2);
+		if (nrows == 0) continue;
+		const int grd = ceil_div(nrows, R), blk = R * W;
+		if (updown == CDR_UP) {
+			if (vec) k3_gs_rows<T, true, true><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			else k3_gs_rows<T, false, true><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
+		} else {
+			if (vec) k3_gs_rows<T, true, false><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			else k3_gs_rows<T, false, false><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
+		}
 		CDR_LAUNCH_CHECK();
 	}
 	return CDR_OK;

@@ -422,3 +422,27 @@ def test_solver3_rejects_bad_nstencil(lib):
     lib.cdr_gpu_settings_default(ctypes.byref(s))
     h = ctypes.c_void_p()
     assert lib.cdr_gpu_solver3_create(ctypes.byref(s), so.ctypes.data, 5, 7, 7, 7, None, ctypes.byref(h)) == 1
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(1, 1, 1), (2, 3, 1), (3, 2, 4), (1, 6, 5), (62, 3, 3), (255, 2, 3), (510, 3, 2),
+                                      (511, 2, 2), (512, 3, 3), (1025, 2, 2)])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_gs3_rows_edges(lib, oracle, nx, ny, nz, extra):
+    """The two-colour row sweep at the edges of its row segments (256 pairs of points), with
+    aligned and unaligned rows, single rows and planes: FP64 bits of the oracle, FP32 within the
+    rounding of its 27-term sums."""
+    so, x, b = make_op3(nx, ny, nz), grid3(nx, ny, nz, 3), grid3(nx, ny, nz, 4)
+    sor = oracle.setup_recip3(so)
+    sor[~np.isfinite(sor)] = 0.0
+    t = __import__("torch")
+    p = nx + 2 + (nx + extra) % 2
+    d64 = [padded(a, p) for a in (so, x, b, sor)]
+    d32 = [a.to(t.float32) for a in d64]
+    xr = x.copy()
+    for updown in (_lib.UP, _lib.DOWN):
+        oracle.relax_gs3(so, xr, b, sor, updown)
+        for d, f in ((d64, lib.cdr_gpu_relax_point_3d_f64), (d32, lib.cdr_gpu_relax_point_3d_f32)):
+            _lib.check(f(ptr(d[0]), 14, ptr(d[1]), ptr(d[2]), ptr(d[3]), nx, ny, nz, p, updown, stream()))
+    assert np.array_equal(unpad(d64[1], nx), xr)
+    # 2 sweeps of 27-term sums: 2 * 30 roundings of 2^-24 on values of the size of x
+    assert np.abs(unpad(d32[1], nx) - xr).max() <= 60 * 2.0 ** -24 * max(np.abs(xr).max(), np.abs(x).max()) * 4
