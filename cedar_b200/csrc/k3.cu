@@ -1030,35 +1030,79 @@ __global__ void k3_cg_factor(const double *__restrict__ so, Dims3 F, double *__r
 	if (info) *info = stt;
 }
 
-// BMG3_SymStd_SOLVE_cg (src/3d/ftn/BMG3_SymStd_SOLVE_cg.f90:105-131) with DPBTRS('U')
-template <typename T>
-__global__ void k3_cg_solve(const double *__restrict__ ab, int ldab, T *__restrict__ q, const T *__restrict__ qf, Dims3 F)
+// BMG3_SymStd_SOLVE_cg (src/3d/ftn/BMG3_SymStd_SOLVE_cg.f90:105-131) with DPBTRS('U').
+// Bound by the chain of 2n quotients, one per unknown and sweep.  The forward
+// sweep runs by columns like the backward one: once unknown i is final, thread m
+// subtracts its term from unknown i + 1 + m, so every unknown still receives its
+// terms in DTBSV's ascending order (the same bits) while a step costs one
+// quotient and one update.  Every thread forms the quotient itself.  WARP: the
+// band has at most 32 entries, one warp runs the steps.  STAGED: the factor fits
+// in shared memory beside the right-hand side.
+template <typename T, bool WARP, bool STAGED>
+__global__ void __launch_bounds__(WARP ? 128 : 1024) k3_cg_solve(const double *__restrict__ ab, int ldab, T *__restrict__ q,
+                                                    const T *__restrict__ qf, Dims3 F)
 {
 	extern __shared__ double xs[];
-	if (threadIdx.x != 0 || blockIdx.x != 0) return;
-	const int kd = F.nx * (F.ny + 1) + 1, n = F.nx * F.ny * F.nz;
-	int kk = 0;
-	for (int k = 2; k <= F.nz + 1; ++k)
-		for (int j = 2; j <= F.ny + 1; ++j)
-			for (int i = 2; i <= F.nx + 1; ++i) xs[kk++] = (double)QF(i, j, k);
-	for (int j = 0; j < n; ++j) {
-		double temp = xs[j];
-		const int i0 = j - kd > 0 ? j - kd : 0;
-		for (int i = i0; i < j; ++i) temp = temp - ab[(size_t)j * ldab + kd + i - j] * xs[i];
-		xs[j] = temp / ab[(size_t)j * ldab + kd];
+	const int kd = ldab - 1, n = F.nx * F.ny * F.nz, tid = threadIdx.x;
+	auto at = [&](int m) -> size_t {  // unknown m, x fastest
+		const int r = m / F.nx;
+		return F.at1(m - r * F.nx + 2, r % F.ny + 2, r / F.ny + 2);
+	};
+	for (int m = tid; m < n; m += blockDim.x) xs[m] = (double)qf[at(m)];
+	const double *A = ab;
+	if (STAGED) {
+		double *sa = xs + n;
+		for (int m = tid; m < n * ldab; m += blockDim.x) sa[m] = ab[m];
+		A = sa;
 	}
-	for (int j = n - 1; j >= 0; --j) {
-		if (xs[j] != 0.0) {
-			xs[j] = xs[j] / ab[(size_t)j * ldab + kd];
-			const double temp = xs[j];
-			const int i1 = j - kd > 0 ? j - kd : 0;
-			for (int i = j - 1; i >= i1; --i) xs[i] = xs[i] - temp * ab[(size_t)j * ldab + kd + i - j];
+	__syncthreads();
+	if (!WARP || tid < 32) {
+		const int nt = WARP ? 32 : blockDim.x;
+		auto sync = [&]() {
+			if (WARP) __syncwarp();
+			else __syncthreads();
+		};
+		auto coef = [&](int r, int c) { return A[(size_t)c * ldab + kd + r - c]; };  // U(r, c), r <= c
+		// the thread's first coefficient and the pivot of the next step load a step ahead
+		double prev = 0.0, d = coef(0, 0), a = tid < kd && 1 + tid < n ? coef(0, 1 + tid) : 0.0;
+		for (int i = 0; i < n; ++i) {
+			const double dn = i + 1 < n ? coef(i + 1, i + 1) : 1.0;
+			const double an = tid < kd && i + 2 + tid < n ? coef(i + 1, i + 2 + tid) : 0.0;
+			const double xi = xs[i] / d;
+			if (tid == 0 && i > 0) xs[i - 1] = prev;
+			if (tid < kd && i + 1 + tid < n) xs[i + 1 + tid] = xs[i + 1 + tid] - a * xi;
+			for (int m = tid + nt; m < kd && i + 1 + m < n; m += nt)
+				xs[i + 1 + m] = xs[i + 1 + m] - coef(i, i + 1 + m) * xi;
+			prev = xi;
+			d = dn;
+			a = an;
+			sync();
 		}
+		if (tid == 0) xs[n - 1] = prev;
+		sync();
+		d = coef(n - 1, n - 1);
+		a = tid < kd && n - 2 - tid >= 0 ? coef(n - 2 - tid, n - 1) : 0.0;
+		for (int j = n - 1; j >= 0; --j) {
+			const double dn = j > 0 ? coef(j - 1, j - 1) : 1.0;
+			const double an = tid < kd && j - 2 - tid >= 0 ? coef(j - 2 - tid, j - 1) : 0.0;
+			const double xj = xs[j];
+			if (tid == 0 && j + 1 < n) xs[j + 1] = prev;
+			prev = xj;
+			if (xj != 0.0) {
+				const double t = xj / d;
+				if (tid < kd && j - 1 - tid >= 0) xs[j - 1 - tid] = xs[j - 1 - tid] - t * a;
+				for (int m = tid + nt; m < kd && j - 1 - m >= 0; m += nt)
+					xs[j - 1 - m] = xs[j - 1 - m] - t * coef(j - 1 - m, j);
+				prev = t;
+			}
+			d = dn;
+			a = an;
+			sync();
+		}
+		if (tid == 0) xs[0] = prev;
 	}
-	kk = 0;
-	for (int k = 2; k <= F.nz + 1; ++k)
-		for (int j = 2; j <= F.ny + 1; ++j)
-			for (int i = 2; i <= F.nx + 1; ++i) Q(i, j, k) = (T)xs[kk++];
+	__syncthreads();
+	for (int m = tid; m < n; m += blockDim.x) q[at(m)] = (T)xs[m];
 }
 
 int setup_cg_3d(const double *so, Dims3 F, double *abd, int *info, cudaStream_t st, int ns)
@@ -1072,12 +1116,20 @@ int setup_cg_3d(const double *so, Dims3 F, double *abd, int *info, cudaStream_t 
 template <typename T>
 int solve_cg_3d(const double *abd, T *x, const T *b, Dims3 F, cudaStream_t st)
 {
-	const size_t sm = sizeof(double) * (size_t)F.nx * F.ny * F.nz;
+	const int n = F.nx * F.ny * F.nz, ldab = cg3_ldab(F), kd = ldab - 1;
+	const size_t sm = sizeof(double) * (size_t)n, staged = sm * (ldab + 1);
 	if (sm > 48 * 1024) {
 		set_error(CDR_ERR_DIM, "coarsest grid %dx%dx%d too large for the direct solve", F.nx, F.ny, F.nz);
 		return CDR_ERR_DIM;
 	}
-	k3_cg_solve<T><<<1, 32, sm, st>>>(abd, F.nx * (F.ny + 1) + 2, x, b, F);
+	const int blk = kd <= 128 ? 128 : kd < 1024 ? (kd + 31) / 32 * 32 : 1024;
+	if (staged <= 48 * 1024) {
+		if (kd <= 32) k3_cg_solve<T, true, true><<<1, blk, staged, st>>>(abd, ldab, x, b, F);
+		else k3_cg_solve<T, false, true><<<1, blk, staged, st>>>(abd, ldab, x, b, F);
+	} else {
+		if (kd <= 32) k3_cg_solve<T, true, false><<<1, blk, sm, st>>>(abd, ldab, x, b, F);
+		else k3_cg_solve<T, false, false><<<1, blk, sm, st>>>(abd, ldab, x, b, F);
+	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
