@@ -144,13 +144,15 @@ int Batch2::setup(bool check)
 			CDR_TRY(setup_recip_2d<double>(F.so, F.sor, df, st, F.ns));
 			if (mixed()) CDR_TRY(convert_f64_f32(F.sor, F.sor32, F.plane() * 2 * nb, st));
 		}
-		if (r == CDR_RELAX_LINE_X || r == CDR_RELAX_LINE_XY) {
-			CDR_TRY(setup_lines_2d<double>(F.so, F.ns, F.sor, df, F.tpitch, CDR_DIR_X, info, st));
-			if (mixed()) CDR_TRY(setup_lines_2d<float>(F.so, F.ns, F.sor32, df, F.tpitch, CDR_DIR_X, info, st));
-		}
-		if (r == CDR_RELAX_LINE_Y || r == CDR_RELAX_LINE_XY) {
-			CDR_TRY(setup_lines_2d<double>(F.so, F.ns, F.sory, df, F.tpitch, CDR_DIR_Y, info, st));
-			if (mixed()) CDR_TRY(setup_lines_2d<float>(F.so, F.ns, F.sory32, df, F.tpitch, CDR_DIR_Y, info, st));
+		const bool lx = r == CDR_RELAX_LINE_X || r == CDR_RELAX_LINE_XY;
+		const bool ly = r == CDR_RELAX_LINE_Y || r == CDR_RELAX_LINE_XY;
+		if (lx || ly) {
+			LineFactors f;
+			if (lx) f.x = F.sor;
+			if (ly) f.y = F.sory;
+			if (lx && mixed()) f.x32 = F.sor32;
+			if (ly && mixed()) f.y32 = F.sory32;
+			CDR_TRY(setup_lines_2d(F.so, F.ns, f, df, F.tpitch, info, st));
 			if (F.yc) CDR_TRY(pack_ylines_2d<double>(F.so, F.ns, F.yc, df, F.tpitch, st));
 		}
 	}

@@ -154,7 +154,7 @@ RECIP_IMPL(float, f32)
 POINT_IMPL(double, f64)
 POINT_IMPL(float, f32)
 
-#define LSETUP_IMPL(T, SUF)                                                                                      \
+#define LSETUP_IMPL(T, SUF, SFX)                                                                                     \
 	int cdr_gpu_setup_lines_2d_##SUF(const double *so, int ns, T *sor, int nx, int ny, int pitch, int tpitch,    \
 	                                 int dir, int *info, cudaStream_t s)                                         \
 	{                                                                                                            \
@@ -162,10 +162,12 @@ POINT_IMPL(float, f32)
 		CDR_TRY(check_ns(ns));                                                                                   \
 		CDR_NONNULL(so); CDR_NONNULL(sor);                                                                       \
 		if (dir != CDR_DIR_X && dir != CDR_DIR_Y) { set_error(CDR_ERR_ARG, "bad dir %d", dir); return CDR_ERR_ARG; } \
-		return setup_lines_2d<T>(so, ns, sor, Dims2{nx, ny, pitch}, tpitch, dir, info, s);                      \
+		LineFactors f;                                                                                                 \
+		(dir == CDR_DIR_X ? f.x##SFX : f.y##SFX) = sor;                                                                \
+		return setup_lines_2d(so, ns, f, Dims2{nx, ny, pitch}, tpitch, info, s);                                       \
 	}
-LSETUP_IMPL(double, f64)
-LSETUP_IMPL(float, f32)
+LSETUP_IMPL(double, f64, )
+LSETUP_IMPL(float, f32, 32)
 
 #define LRELAX_IMPL(T, SUF)                                                                                      \
 	int cdr_gpu_relax_lines_2d_##SUF(const T *so, int ns, T *x, const T *b, const T *sor, int nx, int ny,         \

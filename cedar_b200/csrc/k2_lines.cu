@@ -37,59 +37,135 @@ constexpr int YSMALL_BLOCK = 256;
 
 // ------------------------------------------------------------------ setup
 // BMG2_SymStd_SETUP_lines_{x,y} + DPTTRF: per line d = c, e = -w (x) or -s (y),
-// then e(i) <- e(i)/d(i-1), d(i) <- d(i) - e(i)*e_old(i).  Always FP64; TS is
-// the storage type of the factors.  FP32 factors (the preconditioner's) keep the
-// reciprocal pivots 1/d, formed in FP64 and rounded once, so that the FP32 sweeps
-// multiply instead of divide; FP64 factors keep d, as DPTTRF does.
-template <typename TS, int DIR>
-__global__ void k_lines_setup(const double *__restrict__ so, int ns, TS *__restrict__ sor, Dims2 d, int tpitch,
-                              int *__restrict__ info)
+// then e(i) <- e(i)/d(i-1), d(i) <- d(i) - e(i)*e_old(i).  Always FP64; FP32
+// factors (the preconditioner's) keep the reciprocal pivots 1/d, formed in FP64
+// and rounded once, so that the FP32 sweeps multiply instead of divide; FP64
+// factors keep d, as DPTTRF does.
+//
+// Bound by the recurrence (one quotient per position on the chain), so one
+// launch does every factor array of a level: both directions (grid y) side by
+// side, the FP64 and FP32 copies from one recurrence.  A thread owns a line and
+// loads its operands a chunk of 8 positions ahead of the chain; factors are
+// contiguous along the line and leave as 16-byte stores where they are aligned.
+// One warp per CTA: the few lines of a level spread over the SMs.
+constexpr int LS_CHUNK = 8;
+
+template <bool W64, bool W32, int DIR>
+__device__ __forceinline__ void line_factors(const double *__restrict__ so, int ns, double *__restrict__ f64,
+                                             float *__restrict__ f32, const Dims2 &d, int tpitch, bool vec,
+                                             int *__restrict__ info)
 {
-	const int line = blockIdx.x * blockDim.x + threadIdx.x + 1;
+	const int line = blockIdx.x * 32 + threadIdx.x + 1;
 	const int nl = DIR == CDR_DIR_X ? d.ny : d.nx;
 	const int n = DIR == CDR_DIR_X ? d.nx : d.ny;
 	if (line > nl) return;
 	const size_t ps = d.plane();
 	so += d.bofs(ns * ps);
-	sor += d.bofs(line_factor_size(d, tpitch, DIR));
-	const double *c = so, *off = so + (DIR == CDR_DIR_X ? 1 : 2) * ps;
-	// element at line position p (1..n): grid offset and factor offset
-	auto g = [&](int p) -> size_t { return DIR == CDR_DIR_X ? d.at(p, line) : d.at(line, p); };
-	const size_t fps = DIR == CDR_DIR_X ? ps : (size_t)tpitch * (d.nx + 2);
-	auto fo = [&](int p) -> size_t { return DIR == CDR_DIR_X ? d.at(p, line) : (size_t)line * tpitch + p; };
-	double dprev = c[g(1)];
-	sor[fo(1)] = pivot_store<TS>(dprev);
-	sor[fps + fo(1)] = (TS)(-off[g(1)]);
-	int st = 0;
-	for (int p = 1; p < n; ++p) {
-		if (dprev <= 0.0 && !st) st = p;
-		double ei = -off[g(p + 1)];
-		double e = ei / dprev;
-		double dn = c[g(p + 1)] - e * ei;
-		sor[fps + fo(p + 1)] = (TS)e;
-		sor[fo(p + 1)] = pivot_store<TS>(dn);
-		dprev = dn;
+	const size_t fsize = line_factor_size(d, tpitch, DIR), fps = fsize / 2;
+	const size_t fo = (size_t)line * (DIR == CDR_DIR_X ? d.pitch : tpitch);
+	if (W64) f64 += d.bofs(fsize) + fo;
+	if (W32) f32 += d.bofs(fsize) + fo;
+	// operands of line position p (0: the ghost, read but not used)
+	const size_t g0 = DIR == CDR_DIR_X ? d.at(0, line) : d.at(line, 0), gs = DIR == CDR_DIR_X ? 1 : d.pitch;
+	const double *c = so + g0, *off = so + (DIR == CDR_DIR_X ? 1 : 2) * ps + g0;
+	auto load = [&](int p0, double(&cv)[LS_CHUNK], double(&ov)[LS_CHUNK]) {
+#pragma unroll
+		for (int m = 0; m < LS_CHUNK; ++m) {
+			const bool in = p0 + m <= n;
+			cv[m] = in ? c[(size_t)(p0 + m) * gs] : 0.0;
+			ov[m] = in ? off[(size_t)(p0 + m) * gs] : 0.0;
+		}
+	};
+	double cv[LS_CHUNK], ov[LS_CHUNK], cn[LS_CHUNK], on[LS_CHUNK];
+	load(0, cv, ov);
+	double dprev = 1.0;
+	bool bad = false;
+	for (int p0 = 0; p0 <= n; p0 += LS_CHUNK) {
+		load(p0 + LS_CHUNK, cn, on);
+		double dv[LS_CHUNK], ev[LS_CHUNK];
+#pragma unroll
+		for (int m = 0; m < LS_CHUNK; ++m) {
+			const int p = p0 + m;
+			const double ei = -ov[m];
+			if (p >= 2) {
+				ev[m] = ei / dprev;
+				dv[m] = cv[m] - ev[m] * ei;
+			} else {
+				ev[m] = ei;
+				dv[m] = cv[m];
+			}
+			if (p >= 1 && p <= n) {
+				dprev = dv[m];
+				bad |= dprev <= 0.0;
+			}
+		}
+		if (vec && p0 >= 1 && p0 + LS_CHUNK - 1 <= n) {
+			if (W64) {
+				vstore<double, LS_CHUNK>(f64 + p0, dv);
+				vstore<double, LS_CHUNK>(f64 + fps + p0, ev);
+			}
+			if (W32) {
+				float t[LS_CHUNK];
+#pragma unroll
+				for (int m = 0; m < LS_CHUNK; ++m) t[m] = pivot_store<float>(dv[m]);
+				vstore<float, LS_CHUNK>(f32 + p0, t);
+#pragma unroll
+				for (int m = 0; m < LS_CHUNK; ++m) t[m] = (float)ev[m];
+				vstore<float, LS_CHUNK>(f32 + fps + p0, t);
+			}
+		} else {
+#pragma unroll
+			for (int m = 0; m < LS_CHUNK; ++m) {
+				const int p = p0 + m;
+				if (p < 1 || p > n) continue;
+				if (W64) {
+					f64[p] = dv[m];
+					f64[fps + p] = ev[m];
+				}
+				if (W32) {
+					f32[p] = pivot_store<float>(dv[m]);
+					f32[fps + p] = (float)ev[m];
+				}
+			}
+		}
+#pragma unroll
+		for (int m = 0; m < LS_CHUNK; ++m) {
+			cv[m] = cn[m];
+			ov[m] = on[m];
+		}
 	}
-	if (dprev <= 0.0 && !st) st = n;
-	if (st && info) atomicCAS(info, 0, line);
+	if (bad && info) atomicCAS(info, 0, line);
 }
 
-template <typename TS>
-int setup_lines_2d(const double *so, int nstencil, TS *sor, Dims2 d, int tpitch, int dir, int *info, cudaStream_t st)
+template <bool W64, bool W32>
+__global__ void __launch_bounds__(32) k_lines_setup(const double *__restrict__ so, int ns, LineFactors f, Dims2 d,
+                                                    int tpitch, int dir0, bool vecx, bool vecy, int *__restrict__ info)
 {
-	if (dir == CDR_DIR_Y && tpitch < d.ny + 2) {
+	if (dir0 + (int)blockIdx.y == CDR_DIR_X)
+		line_factors<W64, W32, CDR_DIR_X>(so, ns, f.x, f.x32, d, tpitch, vecx, info);
+	else
+		line_factors<W64, W32, CDR_DIR_Y>(so, ns, f.y, f.y32, d, tpitch, vecy, info);
+}
+
+int setup_lines_2d(const double *so, int nstencil, const LineFactors &f, Dims2 d, int tpitch, int *info, cudaStream_t st)
+{
+	const bool x = f.x || f.x32, y = f.y || f.y32, w64 = f.x || f.y, w32 = f.x32 || f.y32;
+	if (y && tpitch < d.ny + 2) {
 		set_error(CDR_ERR_DIM, "y-line factor pitch %d < ny+2 = %d", tpitch, d.ny + 2);
 		return CDR_ERR_DIM;
 	}
-	const int nl = dir == CDR_DIR_X ? d.ny : d.nx;
-	const dim3 grd(ceil_div(nl, 128), 1, d.nb);
-	if (dir == CDR_DIR_X) k_lines_setup<TS, CDR_DIR_X><<<grd, 128, 0, st>>>(so, nstencil, sor, d, tpitch, info);
-	else k_lines_setup<TS, CDR_DIR_Y><<<grd, 128, 0, st>>>(so, nstencil, sor, d, tpitch, info);
+	// 16-byte stores: line starts, planes and problems a multiple of 4 elements apart
+	auto ok = [](const void *p) { return (uintptr_t)p % 16 == 0; };
+	const bool vecx = d.pitch % 4 == 0 && ok(f.x) && ok(f.x32), vecy = tpitch % 4 == 0 && ok(f.y) && ok(f.y32);
+	const int nl = !y ? d.ny : !x ? d.nx : d.nx > d.ny ? d.nx : d.ny;
+	const dim3 grd(ceil_div(nl, 32), x && y ? 2 : 1, d.nb);
+	const int dir0 = x ? CDR_DIR_X : CDR_DIR_Y;
+	if (w64 && w32) k_lines_setup<true, true><<<grd, 32, 0, st>>>(so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
+	else if (w64) k_lines_setup<true, false><<<grd, 32, 0, st>>>(so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
+	else k_lines_setup<false, true><<<grd, 32, 0, st>>>(so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
-template int setup_lines_2d<double>(const double *, int, double *, Dims2, int, int, int *, cudaStream_t);
-template int setup_lines_2d<float>(const double *, int, float *, Dims2, int, int, int *, cudaStream_t);
 
 // ------------------------------------------------------------------ relax
 // Segmented inclusive scan of affine maps over the tpl threads of a line.

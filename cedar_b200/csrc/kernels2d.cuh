@@ -13,8 +13,14 @@ int setup_recip_2d(const T *so, T *sor, Dims2 d, cudaStream_t st, int nstencil =
 template <typename T>
 int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Dims2 d, int updown, cudaStream_t st,
                    int per = 0);
-template <typename TS>
-int setup_lines_2d(const double *so, int nstencil, TS *sor, Dims2 d, int tpitch, int dir, int *info, cudaStream_t st);
+// Line factors of a level in one launch; null arrays are left out (the FP64 and
+// FP32 arrays of a direction that is wanted must match those of the other).
+struct LineFactors {
+	double *x = nullptr, *y = nullptr;
+	float *x32 = nullptr, *y32 = nullptr;
+};
+int setup_lines_2d(const double *so, int nstencil, const LineFactors &f, Dims2 d, int tpitch, int *info,
+                   cudaStream_t st);
 int lines_prepare();
 // ysync (device, lines_sync_words(d) words, zero before the first use and
 // between uses): y-lines of a single problem sweep both colours in one launch

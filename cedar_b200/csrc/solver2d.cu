@@ -496,16 +496,15 @@ int cdr_gpu_solver::setup()
 		// smoother setup (multilevel::setup_relax_helper, multilevel.h:134-158)
 		switch (s.relaxation) {
 		case CDR_RELAX_POINT: CDR_TRY(setup_recip_2d<double>(F.so, F.sor, F.d, st)); break;
-		case CDR_RELAX_LINE_X:
-			CDR_TRY(setup_lines_2d<double>(F.so, F.ns, F.sor, F.d, F.tpitch, CDR_DIR_X, info, st));
-			break;
-		case CDR_RELAX_LINE_Y:
-			CDR_TRY(setup_lines_2d<double>(F.so, F.ns, F.sory, F.d, F.tpitch, CDR_DIR_Y, info, st));
-			break;
-		case CDR_RELAX_LINE_XY:
-			CDR_TRY(setup_lines_2d<double>(F.so, F.ns, F.sor, F.d, F.tpitch, CDR_DIR_X, info, st));
-			CDR_TRY(setup_lines_2d<double>(F.so, F.ns, F.sory, F.d, F.tpitch, CDR_DIR_Y, info, st));
-			break;
+		default: {
+			const bool lx = s.relaxation != CDR_RELAX_LINE_Y, ly = s.relaxation != CDR_RELAX_LINE_X;
+			LineFactors f;
+			if (lx) f.x = F.sor;
+			if (ly) f.y = F.sory;
+			if (lx && mixed()) f.x32 = F.sor32;
+			if (ly && mixed()) f.y32 = F.sory32;
+			CDR_TRY(setup_lines_2d(F.so, F.ns, f, F.d, F.tpitch, info, st));
+		}
 		}
 		if (F.ypk) CDR_TRY(pack_ylines_2d<double>(F.so, F.ns, F.sory + F.ysize(), F.d, F.tpitch, st));
 	}
@@ -523,19 +522,7 @@ int cdr_gpu_solver::setup()
 			if (F.dg32) CDR_TRY(rowsum_excess_2d(F.so, F.ns, F.dg32, F.d, st));
 			if (l > 0) CDR_TRY(convert_f64_f32(F.ci, F.ci32, F.d.plane() * 8, st));
 			if (l + 1 == L()) continue;
-			switch (s.relaxation) {
-			case CDR_RELAX_POINT: CDR_TRY(convert_f64_f32(F.sor, F.sor32, F.d.plane(), st)); break;
-			case CDR_RELAX_LINE_X:
-				CDR_TRY(setup_lines_2d<float>(F.so, F.ns, F.sor32, F.d, F.tpitch, CDR_DIR_X, info, st));
-				break;
-			case CDR_RELAX_LINE_Y:
-				CDR_TRY(setup_lines_2d<float>(F.so, F.ns, F.sory32, F.d, F.tpitch, CDR_DIR_Y, info, st));
-				break;
-			case CDR_RELAX_LINE_XY:
-				CDR_TRY(setup_lines_2d<float>(F.so, F.ns, F.sor32, F.d, F.tpitch, CDR_DIR_X, info, st));
-				CDR_TRY(setup_lines_2d<float>(F.so, F.ns, F.sory32, F.d, F.tpitch, CDR_DIR_Y, info, st));
-				break;
-			}
+			if (s.relaxation == CDR_RELAX_POINT) CDR_TRY(convert_f64_f32(F.sor, F.sor32, F.d.plane(), st));
 			if (F.ypk) CDR_TRY(pack_ylines_2d<float>(F.so32, F.ns, F.sory32 + F.ysize(), F.d, F.tpitch, st));
 		}
 	}

@@ -554,3 +554,29 @@ def test_packed_y_couplings_sweep_bitwise(lib, precision, nx, ny, ns):
                                               err_msg="pair: cap %d updown %d flags %d" % (cap, updown, flags))
     assert int(sync.abs().sum().item()) == 0
     assert lib.cdr_gpu_lines_stream_status(stream()) == 0
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (7, 9), (8, 15), (16, 17), (33, 24), (40, 70)])
+@pytest.mark.parametrize("extra", [0, 1, 6])
+def test_line_factors_chunk_edges(lib, oracle, nx, ny, extra):
+    """Line factors at the edges of the kernel's chunks of 8 positions and blocks of 32 lines, with
+    rows on and off the 16-byte stores' alignment: FP64 bits of the oracle, FP32 its rounded values
+    (reciprocal pivots), nothing written outside the interior positions."""
+    import torch
+    so = make_op(nx, ny, 5)
+    p, tp = -(-(nx + 2) // 8) * 8 + extra, -(-(ny + 2) // 8) * 8 + extra
+    dso = padded(so, p)
+    for direction, ref in ((_lib.DIR_X, oracle.setup_lines_x(so)[0]), (_lib.DIR_Y, oracle.setup_lines_y(so)[0])):
+        rows, n, width = (ny, nx, p) if direction == _lib.DIR_X else (nx, ny, tp)
+        inner = (slice(None), slice(1, rows + 1), slice(1, n + 1))
+        for dt, f in ((torch.float64, lib.cdr_gpu_setup_lines_2d_f64), (torch.float32, lib.cdr_gpu_setup_lines_2d_f32)):
+            out = torch.full((2, rows + 2, width), -7.0, dtype=dt, device="cuda")
+            _lib.check(f(ptr(dso), 5, ptr(out), nx, ny, p, tp, direction, None, stream()))
+            want = ref[inner].copy()
+            if dt == torch.float32:
+                want[0] = 1.0 / want[0]
+                want = want.astype(np.float32).astype(np.float64)
+            got = host(out)
+            assert np.array_equal(got[inner], want)
+            got[inner] = -7.0
+            assert (got == -7.0).all()
