@@ -10,6 +10,8 @@
 // Kernel bodies address arrays with the reference's 1-based (I, J, K) through
 // the macros below and keep its operand order, so they reproduce its bits
 // (the library is built without FMA contraction).
+
+#include "k2_bulk.cuh"
 #include "k2_point.cuh"
 #include "kernels3d.cuh"
 
@@ -123,10 +125,495 @@ __global__ void __launch_bounds__(1024) k3_norm_finish(const double *__restrict_
 	}
 }
 
+// ----------------------------------------------------------------- smoother
+// BMG3_SymStd_SETUP_recip (src/3d/ftn/BMG3_SymStd_SETUP_recip.f90:63-69)
+template <typename T>
+__global__ void k3_recip(const T *__restrict__ so, T *__restrict__ sor, Dims3 F)
+{
+	const int i = blockIdx.x * TX + threadIdx.x + 2, j = blockIdx.y * TY + threadIdx.y + 2, k = blockIdx.z + 2;
+	if (i > F.nx + 1 || j > F.ny + 1) return;
+	sor[F.at1(i, j, k)] = T(1) / SO(i, j, k, KP);
+}
+
+// The points a = 2t, b = 2t + 1 (0-based) of a row: the sum of the colour swept
+// first, and the second point's terms, held as products (in nb27's order) until
+// its row neighbours (terms 0 and 4, coefficients c0 and c4) have their new values.
+template <typename T>
+struct GsPair {
+	T pr[26], c0, c4, first, rhs, ds;
+};
+
+// crow(plane, dj, dk) and qrow(dj, dk) point at element a of an operator row and
+// of the iterate's rows around (j, k); qf and sor at element a of b and 1/c.
+// SECOND_A: b first, then a (the sweep UP, colours 1..8); else a, then b (DOWN).
+// t >= 1: a has a left neighbour; vb: b is an interior point.
+template <typename T, bool VEC, bool SECOND_A, typename CR, typename QR>
+__device__ __forceinline__ void gs_pair_terms(CR crow, QR qrow, const T *qf, const T *sor, int t, bool va, bool vb,
+                                              GsPair<T> &g, T &far)
+{
+	using V2 = typename Vec2<T>::type;
+	auto pair = [&](const T *x, T &a, T &b) {
+		if constexpr (VEC) {
+			const V2 v = *reinterpret_cast<const V2 *>(x);
+			a = v.x;
+			b = v.y;
+		} else {
+			a = x[0];
+			b = x[1];
+		}
+	};
+	auto row4 = [&](const T *x, T(&v)[4]) {  // left neighbour of a, a, b, right neighbour of b
+		v[0] = t >= 1 ? x[-1] : T(0);
+		pair(x, v[1], v[2]);
+		v[3] = vb ? x[2] : T(0);
+	};
+	T X[4] = {}, Y[4], Z[4], ca, cb, fa, fb, wa, wb, wr, sa, sb;
+	pair(qf, fa, fb);
+	T acc = SECOND_A ? fb : fa;
+	// one term: coefficients of a and of b, iterates of a and of b
+	auto term = [&](int m, T ka, T xa, T kb, T xb) {
+		if (SECOND_A) {
+			acc = acc + kb * xb;
+			g.pr[m] = ka * xa;
+		} else {
+			acc = acc + ka * xa;
+			g.pr[m] = kb * xb;
+		}
+	};
+	// coefficient planes at the point, and at its right neighbour; x: the
+	// neighbour's offset along the row
+	auto own = [&](int m, const T *c, int x) {
+		pair(c, ca, cb);
+		term(m, ca, X[1 + x], cb, X[2 + x]);
+	};
+	auto right = [&](int m, const T *c, int x) {
+		ca = c[1];
+		cb = vb ? c[2] : T(0);
+		term(m, ca, X[1 + x], cb, X[2 + x]);
+	};
+	auto use = [&](const T(&v)[4]) {
+#pragma unroll
+		for (int m = 0; m < 4; ++m) X[m] = v[m];
+	};
+	row4(qrow(0, 0), Y);
+	const T *pw = crow(KPW, 0, 0);
+	pair(pw, wa, wb);
+	wr = vb ? pw[2] : T(0);
+	if (SECOND_A) {  // b: left a (old), right a' (old); a waits for both new b
+		acc = acc + wb * Y[1];
+		g.c0 = wa;
+		g.c4 = wb;
+	} else {  // a: left b (old), right b (old); b waits for both new a
+		acc = acc + wa * Y[0];
+		g.c0 = wb;
+		g.c4 = wr;
+	}
+	row4(qrow(1, 0), X);
+	own(1, crow(KPNW, 1, 0), -1);
+	own(2, crow(KPS, 1, 0), 0);
+	right(3, crow(KPSW, 1, 0), 1);
+	if (SECOND_A) acc = acc + wr * Y[3];
+	else acc = acc + wb * Y[2];
+	row4(qrow(-1, 0), X);
+	right(5, crow(KPNW, 0, 0), 1);
+	own(6, crow(KPS, 0, 0), 0);
+	own(7, crow(KPSW, 0, 0), -1);
+	row4(qrow(0, -1), Z);
+	use(Z);
+	own(8, crow(KB, 0, 0), 0);
+	own(9, crow(KBW, 0, 0), -1);
+	row4(qrow(1, -1), X);
+	own(10, crow(KBNW, 1, 0), -1);
+	own(11, crow(KBN, 1, 0), 0);
+	right(12, crow(KBNE, 1, 0), 1);
+	use(Z);
+	right(13, crow(KBE, 0, 0), 1);
+	row4(qrow(-1, -1), X);
+	right(14, crow(KBSE, 0, 0), 1);
+	own(15, crow(KBS, 0, 0), 0);
+	own(16, crow(KBSW, 0, 0), -1);
+	row4(qrow(0, 1), Z);
+	use(Z);
+	own(17, crow(KB, 0, 1), 0);
+	own(18, crow(KBE, 0, 1), -1);
+	row4(qrow(1, 1), X);
+	own(19, crow(KBSE, 1, 1), -1);
+	own(20, crow(KBS, 1, 1), 0);
+	right(21, crow(KBSW, 1, 1), 1);
+	use(Z);
+	right(22, crow(KBW, 0, 1), 1);
+	row4(qrow(-1, 1), X);
+	right(23, crow(KBNW, 0, 1), 1);
+	own(24, crow(KBN, 0, 1), 0);
+	own(25, crow(KBNE, 0, 1), -1);
+	pair(sor, sa, sb);
+	// a point outside the interior keeps its value
+	if (SECOND_A) g.first = vb ? acc * sb : Y[2];
+	else g.first = va ? acc * sa : Y[1];
+	g.rhs = SECOND_A ? fa : fb;
+	g.ds = SECOND_A ? sa : sb;
+	far = Y[3];
+}
+
+// the second point, given the new values of its row neighbours
+template <typename T>
+__device__ __forceinline__ T gs_pair_second(const GsPair<T> &g, T left, T right)
+{
+	T v = g.rhs + g.c0 * left;
+	v = v + g.pr[1] + g.pr[2] + g.pr[3] + g.c4 * right;
+#pragma unroll
+	for (int m = 5; m < 26; ++m) v = v + g.pr[m];
+	return v * g.ds;
+}
+
+template <typename T, bool VEC>
+__device__ __forceinline__ void gs_pair_store(T *qo, T a, T b, bool va, bool vb)
+{
+	if (VEC && va && vb) {
+		typename Vec2<T>::type v;
+		v.x = a;
+		v.y = b;
+		*reinterpret_cast<typename Vec2<T>::type *>(qo) = v;
+	} else {
+		if (va) qo[0] = a;
+		if (vb) qo[1] = b;
+	}
+}
+
+// Two colours of BMG3_SymStd_relax_GS (src/3d/ftn/BMG3_SymStd_relax_GS.f90:94-136)
+// in one pass: the rows (j, k) of one parity pair, first the points of one
+// x-parity, then the others.  A row's second colour depends on the first only
+// inside the row, and rows of one parity pair do not touch each other, so a
+// block that owns whole rows needs no other block: four launches per sweep.
+// Bound by latency and DRAM: a thread takes a pair of points and loads every
+// coefficient of both at once, so a row's operator lines are read once with all
+// of their bytes used (one colour per launch reads every second point of a row,
+// and each line twice), and the second point's terms wait as products, so that
+// its sum keeps the reference's order and bits.  Rows longer than 2 W points run
+// in segments from the side whose first colour the second one reads.
+template <typename T, bool VEC, bool SECOND_A>
+__global__ void __launch_bounds__(256) k3_gs_rows(const T *__restrict__ so, T *__restrict__ q,
+                                                  const T *__restrict__ qf, const T *__restrict__ sor, Dims3 F, int pj,
+                                                  int pk, int nrj, int nrows, int W)
+{
+	__shared__ T sh[256];    // first-colour values of the segment
+	__shared__ T edge[256];  // per row: the first-colour value the next segment reads
+	const int r = threadIdx.x / W, t0 = threadIdx.x - r * W;
+	const int row = blockIdx.x * (blockDim.x / W) + r;
+	const int nT = F.nx / 2 + 1, nseg = (nT + W - 1) / W;
+	const int rk = row / nrj, j = 1 + pj + 2 * (row - rk * nrj), k = 1 + pk + 2 * rk;
+	const size_t ps = F.plane(), sl = F.slice();
+	const int p = F.pitch;
+	const size_t base = ((size_t)k * (F.ny + 2) + j) * p;
+	for (int s = 0; s < nseg; ++s) {
+		const int t = (SECOND_A ? s : nseg - 1 - s) * W + t0;
+		const bool live = row < nrows && t < nT;
+		const bool va = live && t >= 1, vb = live && 2 * t + 1 <= F.nx;
+		const size_t o = base + 2 * t;
+		GsPair<T> g;
+		T far = T(0);
+		g.first = T(0);
+		if (live)
+			gs_pair_terms<T, VEC, SECOND_A>(
+			    [&](int plane, int dj, int dk) { return so + (size_t)(plane - 1) * ps + o + dj * p + dk * sl; },
+			    [&](int dj, int dk) { return q + o + (ptrdiff_t)dj * p + (ptrdiff_t)dk * (ptrdiff_t)sl; }, qf + o, sor + o, t,
+			    va, vb, g, far);
+		sh[threadIdx.x] = g.first;
+		__syncthreads();  // the segment's row is read, its first colour formed
+		if (live) {
+			T left, right;  // new row neighbours of the second point
+			if (SECOND_A) {
+				left = t0 > 0 ? sh[threadIdx.x - 1] : edge[r];
+				right = g.first;
+			} else {
+				left = g.first;
+				right = t + 1 >= nT ? far : t0 + 1 < W ? sh[threadIdx.x + 1] : edge[r];
+			}
+			const T second = gs_pair_second<T>(g, left, right);
+			gs_pair_store<T, VEC>(q + o, SECOND_A ? second : g.first, SECOND_A ? g.first : second, va, vb);
+		}
+		if (nseg > 1) {
+			__syncthreads();  // edge and sh are read
+			if (t0 == (SECOND_A ? W - 1 : 0)) edge[r] = g.first;
+		}
+	}
+}
+
+// --------------------------------------------------------------- staged rows
+// The sweep and the residual of a row read 36 rows: with loads into registers
+// they are bound by latency (159^3 FP32: 22 warps per SM, DRAM at 55 % of peak).
+// Where rows start on 16 bytes, a block takes one row and its 36 input rows arrive
+// in shared memory by 16-byte asynchronous copies, all in flight at once and
+// without registers; several blocks to an SM overlap copies and arithmetic.
+// the 25 operator rows of a row's terms, in shared-memory order
+struct Row27 {
+	int plane, dj, dk;
+};
+constexpr int GS_OPS = 25, GS_ROWS = GS_OPS + 2 + 9;  // then b, 1/c and the iterate's nine rows
+__host__ __device__ constexpr Row27 gs_op(int m)
+{
+	constexpr Row27 t[GS_OPS] = {
+	    {KPW, 0, 0},  {KPNW, 0, 0}, {KPS, 0, 0},  {KPSW, 0, 0}, {KB, 0, 0},   {KBW, 0, 0},  {KBE, 0, 0},
+	    {KBSE, 0, 0}, {KBS, 0, 0},  {KBSW, 0, 0}, {KPNW, 1, 0}, {KPS, 1, 0},  {KPSW, 1, 0}, {KBNW, 1, 0},
+	    {KBN, 1, 0},  {KBNE, 1, 0}, {KB, 0, 1},   {KBE, 0, 1},  {KBW, 0, 1},  {KBNW, 0, 1}, {KBN, 0, 1},
+	    {KBNE, 0, 1}, {KBSE, 1, 1}, {KBS, 1, 1},  {KBSW, 1, 1}};
+	return t[m];
+}
+__host__ __device__ constexpr int gs_op_index(int plane, int dj, int dk)
+{
+	for (int m = 0; m < GS_OPS; ++m)
+		if (gs_op(m).plane == plane && gs_op(m).dj == dj && gs_op(m).dk == dk) return m;
+	return -1;
+}
+
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// 16-byte chunks of a staged row
+template <typename T>
+__host__ __device__ __forceinline__ int staged_chunks(Dims3 F)
+{
+	constexpr int VPC = 16 / sizeof(T);
+	return (F.nx + 2 + VPC - 1) / VPC;
+}
+
+// Copies of the row at `base` (element offset of (j, k)): rl elements apart in
+// shared memory; slot GS_OPS holds qf's row, slot GS_OPS + 1 the row of `extra`.
+template <typename T>
+__device__ __forceinline__ void stage_rows(T *rows, int nch, const T *__restrict__ so, const T *q,
+                                           const T *__restrict__ qf, const T *__restrict__ extra, size_t base, Dims3 F)
+{
+	constexpr int VPC = 16 / sizeof(T);
+	const size_t ps = F.plane(), sl = F.slice();
+	const int p = F.pitch, rl = nch * VPC;
+	for (int c = threadIdx.x; c < nch; c += blockDim.x) {
+		const T *src = so + base + c * VPC, *qs = q + base + c * VPC;
+		T *dst = rows + c * VPC;
+#pragma unroll
+		for (int m = 0; m < GS_OPS; ++m) {
+			const Row27 r = gs_op(m);
+			cp_async16(dst + m * rl, src + (size_t)(r.plane - 1) * ps + r.dj * p + r.dk * sl);
+		}
+		cp_async16(dst + GS_OPS * rl, qf + base + c * VPC);
+		cp_async16(dst + (GS_OPS + 1) * rl, extra + base + c * VPC);
+#pragma unroll
+		for (int m = 0; m < 9; ++m)
+			cp_async16(dst + (GS_OPS + 2 + m) * rl,
+			           qs + (ptrdiff_t)(m % 3 - 1) * p + (ptrdiff_t)(m / 3 - 1) * (ptrdiff_t)sl);
+	}
+	asm volatile("cp.async.wait_all;\n" ::: "memory");
+	__syncthreads();
+}
+
+// k3_gs_rows with the row staged; block = row.
+template <typename T, bool SECOND_A>
+__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)
+    k3_gs_staged(const T *__restrict__ so, T *__restrict__ q, const T *__restrict__ qf, const T *__restrict__ sor,
+                 Dims3 F, int pj, int pk, int nrj)
+{
+	extern __shared__ __align__(16) unsigned char k3_raw[];
+	T *rows = reinterpret_cast<T *>(k3_raw);
+	const int nch = staged_chunks<T>(F), rl = nch * (16 / (int)sizeof(T)), t = threadIdx.x;
+	const int rk = blockIdx.x / nrj, j = 1 + pj + 2 * (blockIdx.x - rk * nrj), k = 1 + pk + 2 * rk;
+	const size_t base = ((size_t)k * (F.ny + 2) + j) * F.pitch;
+	stage_rows<T>(rows, nch, so, q, qf, sor, base, F);
+	const bool live = t < F.nx / 2 + 1, va = live && t >= 1, vb = live && 2 * t + 1 <= F.nx;
+	T *center = rows + (GS_OPS + 2 + 4) * rl;
+	GsPair<T> g;
+	if (live) {
+		T far;
+		gs_pair_terms<T, true, SECOND_A>(
+		    [&](int plane, int dj, int dk) { return rows + gs_op_index(plane, dj, dk) * rl + 2 * t; },
+		    [&](int dj, int dk) { return rows + (GS_OPS + 2 + 3 * (dk + 1) + dj + 1) * rl + 2 * t; },
+		    rows + GS_OPS * rl + 2 * t, rows + (GS_OPS + 1) * rl + 2 * t, t, va, vb, g, far);
+		// the first colour goes into the staged row: no thread's first sum reads these points
+		if (SECOND_A ? vb : va) center[2 * t + (SECOND_A ? 1 : 0)] = g.first;
+	}
+	__syncthreads();
+	if (va || vb) {
+		T second = T(0);
+		if (SECOND_A && va) second = gs_pair_second<T>(g, center[2 * t - 1], center[2 * t + 1]);
+		if (!SECOND_A && vb) second = gs_pair_second<T>(g, center[2 * t], center[2 * t + 2]);
+		gs_pair_store<T, true>(q + base + 2 * t, SECOND_A ? second : g.first, SECOND_A ? g.first : second, va, vb);
+	}
+}
+
+// r = b - A x (27-point) of the points a = 2t, b = 2t + 1 of a staged row, in
+// the order of nb27
+template <typename T>
+__device__ __forceinline__ void residual_pair(const T *rows, int rl, int t, bool vb, T &ra, T &rb)
+{
+	using V2 = typename Vec2<T>::type;
+	const T *r0 = rows + 2 * t;
+	auto pair = [&](const T *x, T &a, T &b) {
+		const V2 v = *reinterpret_cast<const V2 *>(x);
+		a = v.x;
+		b = v.y;
+	};
+	T X[4] = {}, Y[4], Z[4], ca, cb;
+	auto row4 = [&](int dj, int dk, T(&v)[4]) {
+		const T *x = r0 + (GS_OPS + 2 + 3 * (dk + 1) + dj + 1) * rl;
+		v[0] = t >= 1 ? x[-1] : T(0);
+		pair(x, v[1], v[2]);
+		v[3] = vb ? x[2] : T(0);
+	};
+	auto own = [&](int plane, int dj, int dk, int x) {
+		pair(r0 + gs_op_index(plane, dj, dk) * rl, ca, cb);
+		ra = ra + ca * X[1 + x];
+		rb = rb + cb * X[2 + x];
+	};
+	auto right = [&](int plane, int dj, int dk, int x) {
+		const T *c = r0 + gs_op_index(plane, dj, dk) * rl;
+		ra = ra + c[1] * X[1 + x];
+		rb = rb + (vb ? c[2] : T(0)) * X[2 + x];
+	};
+	auto use = [&](const T(&v)[4]) {
+#pragma unroll
+		for (int m = 0; m < 4; ++m) X[m] = v[m];
+	};
+	pair(r0 + GS_OPS * rl, ra, rb);
+	row4(0, 0, Y);
+	use(Y);
+	own(KPW, 0, 0, -1);
+	row4(1, 0, X);
+	own(KPNW, 1, 0, -1);
+	own(KPS, 1, 0, 0);
+	right(KPSW, 1, 0, 1);
+	use(Y);
+	right(KPW, 0, 0, 1);
+	row4(-1, 0, X);
+	right(KPNW, 0, 0, 1);
+	own(KPS, 0, 0, 0);
+	own(KPSW, 0, 0, -1);
+	row4(0, -1, Z);
+	use(Z);
+	own(KB, 0, 0, 0);
+	own(KBW, 0, 0, -1);
+	row4(1, -1, X);
+	own(KBNW, 1, 0, -1);
+	own(KBN, 1, 0, 0);
+	right(KBNE, 1, 0, 1);
+	use(Z);
+	right(KBE, 0, 0, 1);
+	row4(-1, -1, X);
+	right(KBSE, 0, 0, 1);
+	own(KBS, 0, 0, 0);
+	own(KBSW, 0, 0, -1);
+	row4(0, 1, Z);
+	use(Z);
+	own(KB, 0, 1, 0);
+	own(KBE, 0, 1, -1);
+	row4(1, 1, X);
+	own(KBSE, 1, 1, -1);
+	own(KBS, 1, 1, 0);
+	right(KBSW, 1, 1, 1);
+	use(Z);
+	right(KBW, 0, 1, 1);
+	row4(-1, 1, X);
+	right(KBNW, 0, 1, 1);
+	own(KBN, 0, 1, 0);
+	own(KBNE, 0, 1, -1);
+	pair(r0 + (GS_OPS + 1) * rl, ca, cb);
+	ra = ra - ca * Y[1];
+	rb = rb - cb * Y[2];
+}
+
+// k3_residual with the rows staged: a block walks rows (NORM: at most 2048
+// blocks, one partial sum each).  TO: type of the stored residual.
+template <typename T, typename TO, bool NORM>
+__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)
+    k3_residual_staged(const T *__restrict__ so, const T *__restrict__ q, const T *__restrict__ qf, TO *__restrict__ res,
+                       Dims3 F, double *__restrict__ partial)
+{
+	extern __shared__ __align__(16) unsigned char k3_raw[];
+	__shared__ double sh[16];
+	T *rows = reinterpret_cast<T *>(k3_raw);
+	const int nch = staged_chunks<T>(F), rl = nch * (16 / (int)sizeof(T)), t = threadIdx.x;
+	const bool live = t < F.nx / 2 + 1, va = live && t >= 1, vb = live && 2 * t + 1 <= F.nx;
+	const int nrows = F.ny * F.nz;
+	double acc = 0.0;
+	for (int row = blockIdx.x; row < nrows; row += gridDim.x) {
+		const int k = row / F.ny + 1, j = row - (k - 1) * F.ny + 1;
+		const size_t base = ((size_t)k * (F.ny + 2) + j) * F.pitch;
+		stage_rows<T>(rows, nch, so, q, qf, so, base, F);
+		if (live) {
+			T ra, rb;
+			residual_pair<T>(rows, rl, t, vb, ra, rb);
+			gs_pair_store<TO, true>(res + base + 2 * t, (TO)ra, (TO)rb, va, vb);
+			if (NORM) {
+				if (va) acc += (double)ra * (double)ra;
+				if (vb) acc += (double)rb * (double)rb;
+			}
+		}
+		__syncthreads();  // the staged rows are read
+	}
+	if (NORM) {
+		for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+		if ((t & 31) == 0) sh[t >> 5] = acc;
+		__syncthreads();
+		if (t == 0) {
+			double v = 0.0;
+			for (int w = 0; w < (int)blockDim.x / 32; ++w) v += sh[w];
+			partial[blockIdx.x] = v;
+		}
+	}
+}
+
+// Shared memory of a staged row, and whether a level's rows can be staged: one
+// row to a block, two blocks to an SM at the least, rows on 16 bytes.  The
+// sweep is faster so at every size but a narrow middle: 31^3 FP32 15.0 -> 9.3 us
+// a sweep, 95^3 19.8 -> 21.8 (L2 holds the level), 127^3 56.7 -> 44.1, 255^3
+// 445 -> 363; FP64 31^3 17.6 -> 10.9, 63^3 18.0 -> 20.1, 191^3 444 -> 317.
+constexpr size_t kStageSmemMax = 104 * 1024;
+template <typename T>
+static size_t staged_smem(Dims3 F)
+{
+	return (size_t)GS_ROWS * staged_chunks<T>(F) * 16;
+}
+template <typename T, typename... P>
+static bool staged_ok(Dims3 F, const P *...p)
+{
+	return F.pitch % (16 / (int)sizeof(T)) == 0 && F.nx / 2 + 1 <= 512 &&
+	       staged_smem<T>(F) <= kStageSmemMax && aligned_to(16, p...);
+}
+static int staged_block(Dims3 F) { return (F.nx / 2 + 1 + 31) / 32 * 32; }
+// opts a staged kernel into its dynamic shared memory
+static int staged_opt_in(const void *fn, size_t smem)
+{
+	if (smem > 40 * 1024)
+		CDR_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStageSmemMax));
+	return CDR_OK;
+}
+
+// the staged residual of a 27-point level; norm_out as in residual_3d
+template <typename T, typename TO>
+static int residual_staged(const T *so, const T *x, const T *b, TO *r, Dims3 F, double *norm_out, double *partial,
+                           cudaStream_t st)
+{
+	const size_t smem = staged_smem<T>(F);
+	const int nrows = F.ny * F.nz, blk = staged_block(F);
+	if (norm_out) {
+		const int nb = nrows < 2048 ? nrows : 2048;
+		CDR_TRY(staged_opt_in((const void *)k3_residual_staged<T, TO, true>, smem));
+		k3_residual_staged<T, TO, true><<<nb, blk, smem, st>>>(so, x, b, r, F, partial);
+		CDR_LAUNCH_CHECK();
+		k3_norm_finish<<<1, 1024, 0, st>>>(partial, nb, norm_out);
+	} else {
+		CDR_TRY(staged_opt_in((const void *)k3_residual_staged<T, TO, false>, smem));
+		k3_residual_staged<T, TO, false><<<nrows, blk, smem, st>>>(so, x, b, r, F, nullptr);
+	}
+	CDR_LAUNCH_CHECK();
+	return CDR_OK;
+}
+
 template <typename T>
 int residual_3d(const T *so, const T *x, const T *b, T *r, Dims3 F, double *norm_out, double *partial, cudaStream_t st,
                 int ns)
 {
+	if (ns == 14 && staged_ok<T>(F, so, x, b, r)) return residual_staged<T, T>(so, x, b, r, F, norm_out, partial, st);
 	const long ntiles = (long)ceil_div(F.nx, TX) * ceil_div(F.ny, TY) * F.nz;
 	const int nb = ntiles < 2048 ? (int)ntiles : 2048;
 	if (norm_out) {
@@ -146,196 +633,6 @@ template int residual_3d<double>(const double *, const double *, const double *,
                                  cudaStream_t, int);
 template int residual_3d<float>(const float *, const float *, const float *, float *, Dims3, double *, double *,
                                 cudaStream_t, int);
-
-// ----------------------------------------------------------------- smoother
-// BMG3_SymStd_SETUP_recip (src/3d/ftn/BMG3_SymStd_SETUP_recip.f90:63-69)
-template <typename T>
-__global__ void k3_recip(const T *__restrict__ so, T *__restrict__ sor, Dims3 F)
-{
-	const int i = blockIdx.x * TX + threadIdx.x + 2, j = blockIdx.y * TY + threadIdx.y + 2, k = blockIdx.z + 2;
-	if (i > F.nx + 1 || j > F.ny + 1) return;
-	sor[F.at1(i, j, k)] = T(1) / SO(i, j, k, KP);
-}
-
-// Two colours of BMG3_SymStd_relax_GS (src/3d/ftn/BMG3_SymStd_relax_GS.f90:94-136)
-// in one pass: the rows (j, k) of one parity pair, first the points of one
-// x-parity, then the others.  A row's second colour depends on the first only
-// inside the row, and rows of one parity pair do not touch each other, so a
-// block that owns whole rows needs no other block: four launches per sweep.
-// Bound by DRAM: a thread takes the points a = 2t, b = 2t + 1 (0-based) and
-// loads every coefficient of both at once, so a row's operator lines are read
-// once with all of their bytes used.  One colour per launch reads every second
-// point of a row, and each line twice.  The second point's terms that the first
-// colour does not change wait as products in registers (24 of 26), so its sum
-// keeps the reference's order and bits.  Rows longer than 2 W points run in
-// segments from the side whose first colour the second one reads.
-// SECOND_A: b first, then a (the sweep UP, colours 1..8); else a, then b (DOWN).
-template <typename T, bool VEC, bool SECOND_A>
-__global__ void __launch_bounds__(256) k3_gs_rows(const T *__restrict__ so, T *__restrict__ q,
-                                                  const T *__restrict__ qf, const T *__restrict__ sor, Dims3 F, int pj,
-                                                  int pk, int nrj, int nrows, int W)
-{
-	using V2 = typename Vec2<T>::type;
-	__shared__ T sh[256];   // first-colour values of the segment
-	__shared__ T edge[256]; // per row: the first-colour value the next segment reads
-	const int r = threadIdx.x / W, t0 = threadIdx.x - r * W;
-	const int row = blockIdx.x * (blockDim.x / W) + r;
-	const int nT = F.nx / 2 + 1, nseg = (nT + W - 1) / W;
-	const int rk = row / nrj, j = 1 + pj + 2 * (row - rk * nrj), k = 1 + pk + 2 * rk;
-	const size_t ps = F.plane(), sl = F.slice();
-	const int p = F.pitch;
-	const size_t base = ((size_t)k * (F.ny + 2) + j) * p;
-	for (int s = 0; s < nseg; ++s) {
-		const int t = (SECOND_A ? s : nseg - 1 - s) * W + t0;
-		const bool live = row < nrows && t < nT;
-		const bool va = live && t >= 1, vb = live && 2 * t + 1 <= F.nx;
-		// terms of the second point (index 0 and 4: its row neighbours), the first point's sum
-		T pr[26], c0 = T(0), c4 = T(0), first = T(0), second = T(0), far = T(0), ds = T(0);
-		if (live) {
-			const size_t o = base + 2 * t;
-			auto pair = [&](const T *x, T &a, T &b) {
-				if constexpr (VEC) {
-					const V2 v = *reinterpret_cast<const V2 *>(x);
-					a = v.x;
-					b = v.y;
-				} else {
-					a = x[0];
-					b = x[1];
-				}
-			};
-			// q of a row: left neighbour of a, a, b, right neighbour of b
-			auto row4 = [&](const T *x, T(&v)[4]) {
-				v[0] = t >= 1 ? x[-1] : T(0);
-				pair(x, v[1], v[2]);
-				v[3] = vb ? x[2] : T(0);
-			};
-			T X[4], ca, cb, acc1, f_a, f_b;
-			const T *S = so + o;
-			auto P = [&](int plane) { return S + (size_t)(plane - 1) * ps; };
-			// one term: coefficient of a and of b, iterates of a and of b
-			auto term = [&](int m, T wa, T xa, T wb, T xb) {
-				if (SECOND_A) {
-					acc1 = acc1 + wb * xb;
-					pr[m] = wa * xa;
-				} else {
-					acc1 = acc1 + wa * xa;
-					pr[m] = wb * xb;
-				}
-			};
-			// coefficient planes at the point, and at its right neighbour
-			auto own = [&](int m, const T *c, int x) {
-				pair(c, ca, cb);
-				term(m, ca, X[1 + x], cb, X[2 + x]);
-			};
-			auto right = [&](int m, const T *c, int x) {
-				ca = c[1];
-				cb = vb ? c[2] : T(0);
-				term(m, ca, X[1 + x], cb, X[2 + x]);
-			};
-			pair(qf + o, f_a, f_b);
-			acc1 = SECOND_A ? f_b : f_a;
-			const T f2 = SECOND_A ? f_a : f_b;
-			const T *qo = q + o;
-			T Y[4];
-			row4(qo, Y);
-			T wa, wb, wr;
-			pair(P(KPW), wa, wb);
-			wr = vb ? P(KPW)[2] : T(0);
-			if (SECOND_A) {  // b: left a (old), right a' (old); a waits for both new b
-				acc1 = acc1 + wb * Y[1];
-				c0 = wa;
-				c4 = wb;
-			} else {  // a: left b (old), right b (old); b waits for both new a
-				acc1 = acc1 + wa * Y[0];
-				c0 = wb;
-				c4 = wr;
-			}
-			row4(qo + p, X);
-			own(1, P(KPNW) + p, -1);
-			own(2, P(KPS) + p, 0);
-			right(3, P(KPSW) + p, 1);
-			if (SECOND_A) acc1 = acc1 + wr * Y[3];
-			else acc1 = acc1 + wb * Y[2];
-			row4(qo - p, X);
-			right(5, P(KPNW), 1);
-			own(6, P(KPS), 0);
-			own(7, P(KPSW), -1);
-			row4(qo - sl, X);
-			own(8, P(KB), 0);
-			own(9, P(KBW), -1);
-			T Z[4];
-#pragma unroll
-			for (int m = 0; m < 4; ++m) Z[m] = X[m];
-			row4(qo + p - sl, X);
-			own(10, P(KBNW) + p, -1);
-			own(11, P(KBN) + p, 0);
-			right(12, P(KBNE) + p, 1);
-#pragma unroll
-			for (int m = 0; m < 4; ++m) X[m] = Z[m];
-			right(13, P(KBE), 1);
-			row4(qo - p - sl, X);
-			right(14, P(KBSE), 1);
-			own(15, P(KBS), 0);
-			own(16, P(KBSW), -1);
-			row4(qo + sl, X);
-			own(17, P(KB) + sl, 0);
-			own(18, P(KBE) + sl, -1);
-#pragma unroll
-			for (int m = 0; m < 4; ++m) Z[m] = X[m];
-			row4(qo + p + sl, X);
-			own(19, P(KBSE) + p + sl, -1);
-			own(20, P(KBS) + p + sl, 0);
-			right(21, P(KBSW) + p + sl, 1);
-#pragma unroll
-			for (int m = 0; m < 4; ++m) X[m] = Z[m];
-			right(22, P(KBW) + sl, 1);
-			row4(qo - p + sl, X);
-			right(23, P(KBNW) + sl, 1);
-			own(24, P(KBN) + sl, 0);
-			own(25, P(KBNE) + sl, -1);
-			T sa, sb;
-			pair(sor + o, sa, sb);
-			// a point outside the interior keeps its value
-			if (SECOND_A) first = vb ? acc1 * sb : Y[2];
-			else first = va ? acc1 * sa : Y[1];
-			second = f2;
-			ds = SECOND_A ? sa : sb;
-			far = SECOND_A ? T(0) : Y[3];
-		}
-		sh[threadIdx.x] = first;
-		__syncthreads();  // the segment's row is read, its first colour formed
-		if (live) {
-			T nl, nr;  // new row neighbours of the second point
-			if (SECOND_A) {
-				nl = t0 > 0 ? sh[threadIdx.x - 1] : edge[r];
-				nr = first;
-			} else {
-				nl = first;
-				nr = t + 1 >= nT ? far : t0 + 1 < W ? sh[threadIdx.x + 1] : edge[r];
-			}
-			second = second + c0 * nl;
-			second = second + pr[1] + pr[2] + pr[3] + c4 * nr;
-#pragma unroll
-			for (int m = 5; m < 26; ++m) second = second + pr[m];
-			second = second * ds;
-			T *qo = q + base + 2 * t;
-			const T na = SECOND_A ? second : first, nb = SECOND_A ? first : second;
-			if (VEC && va && vb) {
-				V2 v;
-				v.x = na;
-				v.y = nb;
-				*reinterpret_cast<V2 *>(qo) = v;
-			} else {
-				if (va) qo[0] = na;
-				if (vb) qo[1] = nb;
-			}
-		}
-		if (nseg > 1) {
-			__syncthreads();  // edge and sh are read
-			if (t0 == (SECOND_A ? W - 1 : 0)) edge[r] = first;
-		}
-	}
-}
 
 // One colour of the seven-point branch of BMG3_SymStd_relax_GS
 // (BMG3_SymStd_relax_GS.f90:141-180): colour pts (0 or 1) holds the points
@@ -363,15 +660,27 @@ int relax_point_3d(const T *so, T *x, const T *b, const T *sor, Dims3 F, int upd
 		return CDR_OK;
 	}
 	// colours 1..8 (UP) or 8..1 (DOWN) are the parities (i, j, k), i fastest: pairs
-	// of colours share the rows of one (j, k) parity.  W pairs of points per row and
+	// of colours share the rows of one (j, k) parity.  Staged rows where they fit
+	// (see staged_ok); else W pairs of points per row and
 	// segment, as many rows to a block of 256 threads as fit; two-element accesses
 	// where rows start aligned.
+	const bool staged = staged_ok<T>(F, so, x, b, sor);
+	const size_t smem = staged_smem<T>(F);
+	if (staged)
+		CDR_TRY(staged_opt_in(updown == CDR_UP ? (const void *)k3_gs_staged<T, true>
+		                                       : (const void *)k3_gs_staged<T, false>, smem));
 	const bool vec = F.pitch % 2 == 0 && aligned_to(2 * sizeof(T), so, x, b, sor);
 	const int W = F.nx / 2 + 1 < 256 ? F.nx / 2 + 1 : 256, R = 256 / W;
 	for (int c = 0; c < 4; ++c) {
 		const int bits = updown == CDR_UP ? c : 3 - c, pj = bits & 1, pk = bits >> 1;
 		const int nrj = (F.ny - pj + 1) / 2, nrows = nrj * ((F.nz - pk + 1) / 2);
 		if (nrows == 0) continue;
+		if (staged) {
+			if (updown == CDR_UP) k3_gs_staged<T, true><<<nrows, staged_block(F), smem, st>>>(so, x, b, sor, F, pj, pk, nrj);
+			else k3_gs_staged<T, false><<<nrows, staged_block(F), smem, st>>>(so, x, b, sor, F, pj, pk, nrj);
+			CDR_LAUNCH_CHECK();
+			continue;
+		}
 		const int grd = ceil_div(nrows, R), blk = R * W;
 		if (updown == CDR_UP) {
 			if (vec) k3_gs_rows<T, true, true><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
@@ -1179,9 +1488,28 @@ __global__ void __launch_bounds__(TX *TY) k3_ir_residual(const double *__restric
 	if (threadIdx.x == 0 && threadIdx.y == 0) partial[blockIdx.x] = s;
 }
 
+// x_out = x_in + e32 on the interior
+__global__ void __launch_bounds__(256) k3_ir_add(const double *__restrict__ x, const float *__restrict__ e,
+                                                 double *__restrict__ xo, Dims3 F)
+{
+	const int i = blockIdx.x * 64 + threadIdx.x + 1, j = blockIdx.y * 4 + threadIdx.y + 1, k = blockIdx.z + 1;
+	if (i > F.nx || j > F.ny) return;
+	const size_t o = ((size_t)k * (F.ny + 2) + j) * F.pitch + i;
+	xo[o] = x[o] + (double)e[o];
+}
+
+// 27-point levels whose rows can be staged form x_out first and then its
+// residual: forming x_in + e for each of the 27 neighbours cost 81 loads and 27
+// conversions a point (255^3: 1081 us at DRAM 32 %); the extra read of x_out is 8
+// of about 156 bytes.
 int ir_residual_3d(const double *so, const double *x, const float *e, const double *b, double *xo, float *r32,
                    Dims3 d, Dims3 d32, double *norm_out, double *partial, int apply, cudaStream_t st, int ns)
 {
+	if (ns == 14 && apply && d32.pitch == d.pitch && staged_ok<double>(d, so, x, b, (const double *)xo, r32)) {
+		k3_ir_add<<<dim3(ceil_div(d.nx, 64), ceil_div(d.ny, 4), d.nz), dim3(64, 4), 0, st>>>(x, e, xo, d);
+		CDR_LAUNCH_CHECK();
+		return residual_staged<double, float>(so, xo, b, r32, d, norm_out, partial, st);
+	}
 	const long ntiles = (long)ceil_div(d.nx, TX) * ceil_div(d.ny, TY) * d.nz;
 	const int nb = ntiles < 2048 ? (int)ntiles : 2048;
 	if (ns == 4) k3_ir_residual<4><<<nb, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply);

@@ -446,3 +446,34 @@ def test_gs3_rows_edges(lib, oracle, nx, ny, nz, extra):
     assert np.array_equal(unpad(d64[1], nx), xr)
     # 2 sweeps of 27-term sums: 2 * 30 roundings of 2^-24 on values of the size of x
     assert np.abs(unpad(d32[1], nx) - xr).max() <= 60 * 2.0 ** -24 * max(np.abs(xr).max(), np.abs(x).max()) * 4
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(1, 2, 2), (2, 3, 1), (61, 2, 3), (62, 3, 2), (63, 4, 2), (331, 2, 2), (368, 2, 2),
+                                      (712, 2, 2), (1100, 2, 2)])
+def test_staged_rows3_edges(lib, oracle, nx, ny, nz):
+    """Residual (and its norm) and sweep of aligned levels around the limits of the staged rows
+    (whole warps of points, the shared-memory limit in FP64 and FP32) against the oracle's bits."""
+    so, x, b = make_op3(nx, ny, nz), grid3(nx, ny, nz, 3), grid3(nx, ny, nz, 4)
+    p = -(-(nx + 2) // 4) * 4
+    dso, dx, db, dr = padded(so, p), padded(x, p), padded(b, p), padded(np.zeros_like(x), p)
+    nrm, scratch = padded(np.zeros((1, 1)), 1), padded(np.zeros((1, 2048)), 2048)
+    _lib.check(lib.cdr_gpu_residual_3d_f64(ptr(dso), 14, ptr(dx), ptr(db), ptr(dr), nx, ny, nz, p, ptr(nrm),
+                                           ptr(scratch), stream()))
+    ref = oracle.residual3(so, x, b)
+    assert np.array_equal(unpad(dr, nx), ref)
+    assert abs(host(nrm)[0, 0] - oracle.l2norm3(ref)) <= 1e-13 * oracle.l2norm3(ref)
+    t = __import__("torch")
+    d32 = [a.to(t.float32) for a in (dso, dx, db)]
+    r32 = t.zeros_like(d32[1])
+    _lib.check(lib.cdr_gpu_residual_3d_f32(ptr(d32[0]), 14, ptr(d32[1]), ptr(d32[2]), ptr(r32), nx, ny, nz, p, None,
+                                           None, stream()))
+    # 28 products and sums of terms of size |a||x|, each rounded to 2^-24, and the inputs' rounding
+    scale = np.abs(so).max() * np.abs(x).max() + np.abs(b).max()
+    assert np.abs(unpad(r32, nx) - ref).max() <= 28 * 32 * 2.0 ** -24 * scale
+    sor = oracle.setup_recip3(so)
+    dsor = padded(sor, p)
+    for updown in (_lib.UP, _lib.DOWN):
+        oracle.relax_gs3(so, x, b, sor, updown)
+        _lib.check(lib.cdr_gpu_relax_point_3d_f64(ptr(dso), 14, ptr(dx), ptr(db), ptr(dsor), nx, ny, nz, p, updown,
+                                                  stream()))
+    assert np.array_equal(unpad(dx, nx), x)
