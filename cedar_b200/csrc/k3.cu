@@ -85,9 +85,10 @@ struct Load3 {
 // --------------------------------------------------------------- residual
 // BMG3_SymStd_residual (src/3d/ftn/BMG3_SymStd_residual.f90:67-121); grid-stride
 // over 32x8 tiles of every k-slice, FP64 partial sums of r^2 per block.
-template <typename T, bool NORM, int NS>
+// TO: type of the stored residual.
+template <typename T, bool NORM, int NS, typename TO = T>
 __global__ void __launch_bounds__(TX *TY) k3_residual(const T *__restrict__ so, const T *__restrict__ q,
-                                                      const T *__restrict__ qf, T *__restrict__ res, Dims3 F,
+                                                      const T *__restrict__ qf, TO *__restrict__ res, Dims3 F,
                                                       double *__restrict__ partial)
 {
 	__shared__ double sh[TX * TY / 32];
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(TX *TY) k3_residual(const T *__restrict__ so, 
 		const int i = (rem % tx) * TX + threadIdx.x + 2, j = (rem / tx) * TY + threadIdx.y + 2, k = kk + 2;
 		if (i <= F.nx + 1 && j <= F.ny + 1) {
 			const T r = nbs<NS, T>(so, Load3<T>{q, F}, QF(i, j, k), F, i, j, k) - SO(i, j, k, KP) * Q(i, j, k);
-			res[F.at1(i, j, k)] = r;
+			res[F.at1(i, j, k)] = (TO)r;
 			if (NORM) acc += (double)r * (double)r;
 		}
 	}
@@ -522,10 +523,10 @@ __device__ __forceinline__ void residual_pair(const T *rows, int rl, int t, bool
 }
 
 // k3_residual with the rows staged: a block walks rows (NORM: at most 2048
-// blocks, one partial sum each).  TO: type of the stored residual.
-template <typename T, typename TO, bool NORM>
-__global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)
-    k3_residual_staged(const T *__restrict__ so, const T *__restrict__ q, const T *__restrict__ qf, TO *__restrict__ res,
+// blocks, one partial sum each).
+template <typename T, bool NORM>
+__global__ void __launch_bounds__(512, 2)
+    k3_residual_staged(const T *__restrict__ so, const T *__restrict__ q, const T *__restrict__ qf, T *__restrict__ res,
                        Dims3 F, double *__restrict__ partial)
 {
 	extern __shared__ __align__(16) unsigned char k3_raw[];
@@ -542,7 +543,7 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)
 		if (live) {
 			T ra, rb;
 			residual_pair<T>(rows, rl, t, vb, ra, rb);
-			gs_pair_store<TO, true>(res + base + 2 * t, (TO)ra, (TO)rb, va, vb);
+			gs_pair_store<T, true>(res + base + 2 * t, ra, rb, va, vb);
 			if (NORM) {
 				if (va) acc += (double)ra * (double)ra;
 				if (vb) acc += (double)rb * (double)rb;
@@ -588,32 +589,27 @@ static int staged_opt_in(const void *fn, size_t smem)
 	return CDR_OK;
 }
 
-// the staged residual of a 27-point level; norm_out as in residual_3d
-template <typename T, typename TO>
-static int residual_staged(const T *so, const T *x, const T *b, TO *r, Dims3 F, double *norm_out, double *partial,
-                           cudaStream_t st)
-{
-	const size_t smem = staged_smem<T>(F);
-	const int nrows = F.ny * F.nz, blk = staged_block(F);
-	if (norm_out) {
-		const int nb = nrows < 2048 ? nrows : 2048;
-		CDR_TRY(staged_opt_in((const void *)k3_residual_staged<T, TO, true>, smem));
-		k3_residual_staged<T, TO, true><<<nb, blk, smem, st>>>(so, x, b, r, F, partial);
-		CDR_LAUNCH_CHECK();
-		k3_norm_finish<<<1, 1024, 0, st>>>(partial, nb, norm_out);
-	} else {
-		CDR_TRY(staged_opt_in((const void *)k3_residual_staged<T, TO, false>, smem));
-		k3_residual_staged<T, TO, false><<<nrows, blk, smem, st>>>(so, x, b, r, F, nullptr);
-	}
-	CDR_LAUNCH_CHECK();
-	return CDR_OK;
-}
-
 template <typename T>
 int residual_3d(const T *so, const T *x, const T *b, T *r, Dims3 F, double *norm_out, double *partial, cudaStream_t st,
                 int ns)
 {
-	if (ns == 14 && staged_ok<T>(F, so, x, b, r)) return residual_staged<T, T>(so, x, b, r, F, norm_out, partial, st);
+	// FP32 27-point rows staged (255^3: 390 -> 239 us); in FP64 a staged row takes
+	// 74 KB there and the point kernel is the faster one (863 against about 530 us)
+	if constexpr (sizeof(T) == 4)
+		if (ns == 14 && staged_ok<T>(F, so, x, b, r)) {
+			const size_t smem = staged_smem<T>(F);
+			const int nrows = F.ny * F.nz, blk = staged_block(F), nb = norm_out && nrows > 2048 ? 2048 : nrows;
+			CDR_TRY(staged_opt_in(norm_out ? (const void *)k3_residual_staged<T, true>
+			                               : (const void *)k3_residual_staged<T, false>, smem));
+			if (norm_out) k3_residual_staged<T, true><<<nb, blk, smem, st>>>(so, x, b, r, F, partial);
+			else k3_residual_staged<T, false><<<nb, blk, smem, st>>>(so, x, b, r, F, nullptr);
+			CDR_LAUNCH_CHECK();
+			if (norm_out) {
+				k3_norm_finish<<<1, 1024, 0, st>>>(partial, nb, norm_out);
+				CDR_LAUNCH_CHECK();
+			}
+			return CDR_OK;
+		}
 	const long ntiles = (long)ceil_div(F.nx, TX) * ceil_div(F.ny, TY) * F.nz;
 	const int nb = ntiles < 2048 ? (int)ntiles : 2048;
 	if (norm_out) {
@@ -1448,7 +1444,8 @@ template int solve_cg_3d<float>(const double *, float *, const float *, Dims3, c
 // Outer refinement step of the mixed-precision 3D solve (as the 2D one):
 //   x_out = x_in + e32, r64 = b - A x_out, r32 = (float) r64, ||r64||^2 per
 //   block.  Each thread forms x_in + e32 over its 27-point neighbourhood on the
-//   fly; x_in and x_out are different buffers.  apply = 0 skips e.
+//   fly; x_in and x_out are different buffers.  apply = 0 skips e (x_out is then
+//   not needed and may be left unwritten).
 struct LoadIR3 {
 	const double *__restrict__ x;
 	const float *__restrict__ e;
@@ -1498,20 +1495,26 @@ __global__ void __launch_bounds__(256) k3_ir_add(const double *__restrict__ x, c
 	xo[o] = x[o] + (double)e[o];
 }
 
-// 27-point levels whose rows can be staged form x_out first and then its
-// residual: forming x_in + e for each of the 27 neighbours cost 81 loads and 27
-// conversions a point (255^3: 1081 us at DRAM 32 %); the extra read of x_out is 8
-// of about 156 bytes.
+// 27-point levels form x_out first and then its residual: forming x_in + e for
+// each of the 27 neighbours cost 81 loads and 27 conversions a point (255^3:
+// 1058 us at 32 % of the DRAM rate); the extra read of x_out is 8 of about 156
+// bytes.
 int ir_residual_3d(const double *so, const double *x, const float *e, const double *b, double *xo, float *r32,
                    Dims3 d, Dims3 d32, double *norm_out, double *partial, int apply, cudaStream_t st, int ns)
 {
-	if (ns == 14 && apply && d32.pitch == d.pitch && staged_ok<double>(d, so, x, b, (const double *)xo, r32)) {
-		k3_ir_add<<<dim3(ceil_div(d.nx, 64), ceil_div(d.ny, 4), d.nz), dim3(64, 4), 0, st>>>(x, e, xo, d);
-		CDR_LAUNCH_CHECK();
-		return residual_staged<double, float>(so, xo, b, r32, d, norm_out, partial, st);
-	}
 	const long ntiles = (long)ceil_div(d.nx, TX) * ceil_div(d.ny, TY) * d.nz;
 	const int nb = ntiles < 2048 ? (int)ntiles : 2048;
+	if (ns == 14 && d32.pitch == d.pitch) {
+		if (apply) {
+			k3_ir_add<<<dim3(ceil_div(d.nx, 64), ceil_div(d.ny, 4), d.nz), dim3(64, 4), 0, st>>>(x, e, xo, d);
+			CDR_LAUNCH_CHECK();
+		}
+		k3_residual<double, true, 14, float><<<nb, dim3(TX, TY), 0, st>>>(so, apply ? xo : x, b, r32, d, partial);
+		CDR_LAUNCH_CHECK();
+		k3_norm_finish<<<1, 1024, 0, st>>>(partial, nb, norm_out);
+		CDR_LAUNCH_CHECK();
+		return CDR_OK;
+	}
 	if (ns == 4) k3_ir_residual<4><<<nb, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply);
 	else k3_ir_residual<14><<<nb, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply);
 	CDR_LAUNCH_CHECK();
