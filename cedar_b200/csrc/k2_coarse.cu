@@ -25,7 +25,9 @@
 
 namespace cdrgpu {
 
-constexpr int CC_THREADS = 1024;
+// 512 threads: a colour of 32-point lines needs 16 warps, a barrier of 32 warps costs
+// more than the second round of the point steps, and two CTAs share an SM in a batch
+constexpr int CC_THREADS = 512;
 constexpr int CC_WARPS = CC_THREADS / 32;
 
 // f(i, j) for i in [i0, i1], j in [j0, j1]: rows over the warps, positions over the lanes
@@ -47,124 +49,151 @@ __host__ __device__ inline int cc_sory_planes(int relax)
 	return relax == CDR_RELAX_LINE_Y || relax == CDR_RELAX_LINE_XY ? 2 : 0;
 }
 
-// Elements of level l's shared copy (rows of nx+2): operator, factors, b, x, r
-// (the coarsest keeps b and x only) and the interpolation weights of every
-// level but the first.
+// Shared-memory offsets (elements) of a level's arrays, -1 where it has none;
+// rows of nx+2 elements, y-line factors transposed with rows of ny+2.
+struct CcOffsets {
+	int so, sor, sory, ci, x, b, r;
+};
+// One plane to stage: global source of problem 0, elements between problems,
+// pitches, rows; pairs: rows move as 8-byte FP32 pairs.
+struct CcPlane {
+	const void *src;
+	long long pstride;
+	int spitch, dst, dpitch;
+	short rowlen, rows;
+	int pairs;
+};
+constexpr int kMaxCcPlanes = 18 * kMaxCoarseLevels;
+// What a launch needs beside the levels, laid out on the host: the levels' x, r
+// and restricted b first (zeroed as one range), then the staged planes, the line
+// right-hand sides, and the coarsest solve's vector and factor in FP64.
 template <typename T>
-__host__ __device__ inline size_t cc_elems(const CoarseCycle<T> &cc, int l)
+struct CcPlan {
+	CoarseCycle<T> cc;
+	CcOffsets off[kMaxCoarseLevels];
+	int nzero = 0, lines = 0, dbl_byte = 0, nplanes = 0;
+	size_t bytes = 0;
+	CcPlane plane[kMaxCcPlanes];
+};
+
+template <typename T>
+static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 {
-	const CoarseLevel<T> &L = cc.lv[l];
-	const size_t pl = (size_t)(L.nx + 2) * (L.ny + 2);
-	size_t planes = l == cc.nl - 1 ? 2 : L.ns + cc_sor_planes(cc.relax) + cc_sory_planes(cc.relax) + 3;
-	if (l > 0) planes += 8;
-	return planes * pl;
+	CcPlan<T> P;
+	P.cc = cc;
+	size_t at = 0, ln = 0;
+	auto take = [&](size_t n) {
+		const size_t o = at;
+		at += n;
+		return (int)o;
+	};
+	for (int l = 0; l < cc.nl; ++l) {
+		const CoarseLevel<T> &L = cc.lv[l];
+		const size_t pl = (size_t)(L.nx + 2) * (L.ny + 2);
+		const bool last = l == cc.nl - 1;
+		P.off[l] = CcOffsets{-1, -1, -1, -1, -1, -1, -1};
+		P.off[l].x = take(pl);
+		if (!last) P.off[l].r = take(pl);
+		if (l > 0) P.off[l].b = take(pl);
+	}
+	P.nzero = (int)at;
+	for (int l = 0; l < cc.nl; ++l) {
+		const CoarseLevel<T> &L = cc.lv[l];
+		const int ii = L.nx + 2, jj = L.ny + 2;
+		const size_t pl = (size_t)ii * jj, gpl = (size_t)L.pitch * jj;
+		const bool last = l == cc.nl - 1;
+		// planes of one array: rowlen x rows elements each, back to back in shared memory
+		auto stage = [&](const T *src, int spitch, size_t splane, int rowlen, int rows, int planes) {
+			const int o = take((size_t)rowlen * rows * planes);
+			for (int q = 0; q < planes && P.nplanes < kMaxCcPlanes; ++q) {
+				CcPlane &c = P.plane[P.nplanes++];
+				c.src = src + q * splane;
+				c.pstride = (long long)splane * planes;
+				c.spitch = spitch;
+				c.dst = o + q * rowlen * rows;
+				c.dpitch = rowlen;
+				c.rowlen = (short)rowlen;
+				c.rows = (short)rows;
+				c.pairs = sizeof(T) == 4 && rowlen % 2 == 0 && spitch % 2 == 0 && c.dst % 2 == 0 &&
+				          c.pstride % 2 == 0 && (uintptr_t)c.src % 8 == 0;
+			}
+			return o;
+		};
+		if (!last) {
+			P.off[l].so = stage(L.so, L.pitch, gpl, ii, jj, L.ns);
+			// point relaxation keeps one plane of the two allocated
+			const int np = cc_sor_planes(cc.relax);
+			if (np) {
+				P.off[l].sor = stage(L.sor, L.pitch, gpl, ii, jj, np);
+				for (int q = 0; q < np; ++q) P.plane[P.nplanes - 1 - q].pstride = 2 * (long long)gpl;
+			}
+			if (cc_sory_planes(cc.relax)) P.off[l].sory = stage(L.sory, L.tpitch, (size_t)L.tpitch * ii, jj, ii, 2);
+			const size_t a = (size_t)((L.ny + 1) / 2) * L.nx, b = (size_t)((L.nx + 1) / 2) * L.ny;
+			ln = std::max(ln, std::max(a, b));
+		}
+		if (l > 0) P.off[l].ci = stage(L.ci, L.pitch, gpl, ii, jj, 8);
+		if (l == 0) P.off[l].b = stage(L.b, L.pitch, gpl, ii, jj, 1);
+		(void)pl;
+	}
+	P.lines = take(ln);
+	P.dbl_byte = (int)((at * sizeof(T) + 7) / 8 * 8);
+	const CoarseLevel<T> &Cg = cc.lv[cc.nl - 1];
+	const size_t n = (size_t)Cg.nx * Cg.ny;
+	P.bytes = P.dbl_byte + (n + (size_t)(Cg.nx + 2) * n) * sizeof(double);
+	return P;
 }
 
-// Global arrays of problem blockIdx.x of a batch: every array of every level
-// moves by that problem's offset (problems back to back, problem step bstep).
+// Shared copy of level l
 template <typename T>
-__device__ CoarseLevel<T> cc_global(const CoarseCycle<T> &cc, int l)
+__device__ CoarseLevel<T> cc_view(const CcPlan<T> &P, int l, T *base)
 {
-	CoarseLevel<T> L = cc.lv[l];
-	const size_t p = (size_t)blockIdx.x * cc.bstep, pl = (size_t)L.pitch * (L.ny + 2);
-	L.so += p * L.ns * pl;
-	L.x += p * pl;
-	L.b += p * pl;
-	L.r += p * pl;
-	if (L.sor) L.sor += p * 2 * pl;
-	if (L.sory) L.sory += p * 2 * (size_t)L.tpitch * (L.nx + 2);
-	if (L.ci) L.ci += p * 8 * pl;
-	return L;
-}
-
-// Shared copy of level l (compact rows: pitch nx+2, y-line factors tpitch ny+2)
-template <typename T>
-__device__ CoarseLevel<T> cc_view(const CoarseCycle<T> &cc, int l, T *base)
-{
-	size_t off = 0;
-	for (int m = 0; m < l; ++m) off += cc_elems(cc, m);
-	const CoarseLevel<T> &G = cc.lv[l];
-	CoarseLevel<T> S = G;
-	S.pitch = G.nx + 2;
-	S.tpitch = G.ny + 2;
-	const size_t pl = (size_t)(G.nx + 2) * (G.ny + 2);
-	T *p = base + off;
-	if (l < cc.nl - 1) {
-		S.so = p;
-		p += G.ns * pl;
-		const int ns1 = cc_sor_planes(cc.relax), ns2 = cc_sory_planes(cc.relax);
-		S.sor = ns1 ? p : nullptr;
-		p += ns1 * pl;
-		S.sory = ns2 ? p : nullptr;
-		p += ns2 * pl;
-	} else {
-		S.so = S.sor = S.sory = nullptr;
-	}
-	S.b = p;
-	p += pl;
-	S.x = p;
-	p += pl;
-	if (l < cc.nl - 1) {
-		S.r = p;
-		p += pl;
-	} else {
-		S.r = nullptr;
-	}
-	S.ci = l > 0 ? p : nullptr;
+	const CcOffsets &o = P.off[l];
+	CoarseLevel<T> S;
+	S.nx = P.cc.lv[l].nx;
+	S.ny = P.cc.lv[l].ny;
+	S.ns = P.cc.lv[l].ns;
+	S.pitch = S.nx + 2;
+	S.tpitch = S.ny + 2;
+	S.so = base + o.so;
+	S.sor = base + o.sor;
+	S.sory = base + o.sory;
+	S.ci = base + o.ci;
+	S.x = base + o.x;
+	S.b = base + o.b;
+	S.r = base + o.r;
 	return S;
 }
 
-// copy nplanes planes of `rows` rows of rowlen elements between pitches
+// Staging by asynchronous copies (cp.async), every one in flight at once: a warp
+// takes a plane and walks its rows, lanes along the row.  One loop over the
+// host's plane table, so that its code is fetched once (a separate copy per
+// array cost a microsecond of instruction fetch each).
+template <int N>
+__device__ __forceinline__ void cp_async(unsigned dst, const void *src)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(dst), "l"(src), "n"(N) : "memory");
+}
+
 template <typename T>
-__device__ void cc_copy(const T *__restrict__ src, int sp, size_t splane, T *__restrict__ dst, int dp, size_t dplane,
-                        int rowlen, int rows, int nplanes)
+__device__ __forceinline__ void cc_stage(const CcPlan<T> &P, T *base)
 {
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	for (int row = warp; row < rows * nplanes; row += CC_WARPS) {
-		const int q = row / rows, j = row - q * rows;
-		const T *s = src + (size_t)q * splane + (size_t)j * sp;
-		T *d = dst + (size_t)q * dplane + (size_t)j * dp;
-		for (int i = lane; i < rowlen; i += 32) d[i] = s[i];
+	const long long prob = (long long)blockIdx.x * P.cc.bstep;
+	const unsigned sbase = (unsigned)__cvta_generic_to_shared(base);
+	for (int q = warp; q < P.nplanes; q += CC_WARPS) {
+		const CcPlane &c = P.plane[q];
+		const T *src = static_cast<const T *>(c.src) + prob * c.pstride;
+		unsigned dst = sbase + (unsigned)c.dst * (unsigned)sizeof(T);
+		const int rowlen = c.rowlen, rows = c.rows, spitch = c.spitch;
+		const unsigned drow = (unsigned)(c.dpitch * (int)sizeof(T));
+		if (sizeof(T) == 4 && c.pairs) {
+			for (int j = 0; j < rows; ++j, src += spitch, dst += drow)
+				for (int i = lane; i < rowlen / 2; i += 32) cp_async<8>(dst + 8 * i, src + 2 * i);
+		} else {
+			for (int j = 0; j < rows; ++j, src += spitch, dst += drow)
+				for (int i = lane; i < rowlen; i += 32) cp_async<sizeof(T)>(dst + (unsigned)sizeof(T) * i, src + i);
+		}
 	}
-}
-
-// The same copy from global into shared memory by asynchronous copies
-// (cp.async, one element each, consecutive threads on consecutive elements of
-// the flattened planes and rows): every load of the staging is in flight at
-// once instead of one row per warp at a time; cc_stage_wait completes them.
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T *dst_smem, const T *src)
-{
-	const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-	if constexpr (sizeof(T) == 8)
-		asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-	else
-		asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-
-template <typename T>
-__device__ void cc_stage(const T *__restrict__ src, int sp, size_t splane, T *__restrict__ dst, int dp,
-                         size_t dplane, int rowlen, int rows, int nplanes)
-{
-	const int per = rowlen * rows, total = per * nplanes;
-	// quotients by FP64 reciprocals: (e + 1/2) / d lies at least 1/(2d) from an
-	// integer, far beyond the product's rounding error, so the truncation is exact
-	const double ip = 1.0 / per, ir = 1.0 / rowlen;
-	for (int e = threadIdx.x; e < total; e += CC_THREADS) {
-		const int q = (int)((e + 0.5) * ip), rem = e - q * per, j = (int)((rem + 0.5) * ir), i = rem - j * rowlen;
-		cp_async_elem(dst + (size_t)q * dplane + (size_t)j * dp + i, src + (size_t)q * splane + (size_t)j * sp + i);
-	}
-}
-
-__device__ __forceinline__ void cc_stage_wait()
-{
-	asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
-template <typename T>
-__device__ void cc_fill(T *p, size_t n)
-{
-	for (size_t e = threadIdx.x; e < n; e += CC_THREADS) p[e] = T(0);
 }
 
 // r = b - A x on the level (all interior points)
@@ -308,9 +337,44 @@ __device__ void cc_lines(const CoarseLevel<T> &L, int updown, T *sm)
 				__syncwarp();
 			}
 		} else {
+			const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+			if (n <= 32) {
+				// one position per lane, the line in registers from its right-hand side to
+				// its solution: the chunk form below with chunks of one position (its bits)
+				for (int g = warp; g < ml; g += CC_WARPS) {
+					const int lc = first + 2 * g, m = lane;
+					const bool in = m < n;
+					const T *dd = fac + (DIR == CDR_DIR_X ? (size_t)lc * L.pitch : (size_t)lc * L.tpitch);
+					const T *ee = dd + eplane;
+					const T e0 = in && m > 0 ? ee[m + 1] : T(0), e1 = in && m < n - 1 ? ee[m + 2] : T(0);
+					const T dv = in ? dd[m + 1] : T(0);
+					const size_t k = xat(lc, in ? m : 0);
+					T r = line_rhs<T, NS, DIR>(L.so, ps, L.x, L.b, k, L.pitch);
+					T A = in ? -e0 : T(1), B = in ? r : T(0);
+#pragma unroll
+					for (int off = 1; off < 32; off <<= 1) {
+						const T a2 = __shfl_up_sync(0xffffffffu, A, off), b2 = __shfl_up_sync(0xffffffffu, B, off);
+						if (lane >= off) { B = madd(A, b2, B); A = A * a2; }
+					}
+					T y = __shfl_up_sync(0xffffffffu, B, 1);
+					y = m == 0 ? r : madd(-y, e0, r);
+					r = pivot_div(y, dv);
+					A = in ? -e1 : T(1);
+					B = in ? r : T(0);
+#pragma unroll
+					for (int off = 1; off < 32; off <<= 1) {
+						const T a2 = __shfl_down_sync(0xffffffffu, A, off), b2 = __shfl_down_sync(0xffffffffu, B, off);
+						if (lane + off < 32) { B = madd(A, b2, B); A = A * a2; }
+					}
+					T xv = __shfl_down_sync(0xffffffffu, B, 1);
+					xv = m == n - 1 ? r : madd(-xv, e1, r);
+					if (in) L.x[k] = xv;
+				}
+				__syncthreads();
+				continue;
+			}
 			// FP32: one warp per line, each lane a chunk of consecutive positions;
 			// both substitutions as affine-map scans over the lanes (shuffles)
-			const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 			const int cs = (n + 31) / 32;  // chunk length
 			for (int g = warp; g < ml; g += CC_THREADS / 32) {
 				const int lc = first + 2 * g;
@@ -383,9 +447,12 @@ __device__ void cc_smooth(const CoarseCycle<T> &cc, const CoarseLevel<T> &L, int
 	}
 }
 
-// BMG2_SymStd_SOLVE_cg with DPBTRS('U') on the coarsest level: the right-hand
-// side in shared memory (xs) and the factor after it (staged with the levels),
-// the substitutions by one thread (k_cg_solve's operations)
+// BMG2_SymStd_SOLVE_cg with DPBTRS('U') on the coarsest level by one warp: the
+// right-hand side in shared memory (xs), the factor after it (staged with the
+// levels).  Both sweeps run by columns: once an unknown is final, lane m
+// subtracts its term from the m-th unknown of the band ahead, so every unknown
+// receives its terms in DTBSV's order (the same bits) and a step of the chain
+// is one quotient and one update.  Pivot and coefficients load a step ahead.
 template <typename T>
 __device__ void cc_cg(const CoarseLevel<T> &L, double *xs)
 {
@@ -393,75 +460,38 @@ __device__ void cc_cg(const CoarseLevel<T> &L, double *xs)
 	const double *abs = xs + n;
 	cc_rows(1, L.nx, 1, L.ny, [&](int i, int j) { xs[(j - 1) * L.nx + i - 1] = (double)L.b[(size_t)j * L.pitch + i]; });
 	__syncthreads();
-	if (threadIdx.x == 0) {
-		constexpr int KW = 6;
-		if (kd < KW) {
-			// the same operations in the same order, the band's last KW entries of
-			// xs in registers (w[t] = xs[j - KW + t]) and each row's multipliers
-			// loaded ahead of the recurrence
-			double w[KW];
-#pragma unroll
-			for (int t = 0; t < KW; ++t) w[t] = 0.0;
-			for (int j = 0; j < n; ++j) {
-				const double *arow = abs + (size_t)j * ldab + kd - j;  // arow[i]: row j, column i
-				double a[KW];
-#pragma unroll
-				for (int t = 0; t < KW; ++t) {
-					const int i = j - KW + t;
-					a[t] = i >= 0 && i >= j - kd ? arow[i] : 0.0;
-				}
-				double temp = xs[j];
-#pragma unroll
-				for (int t = 0; t < KW; ++t) {
-					const int i = j - KW + t;
-					if (i >= 0 && i >= j - kd) temp = temp - a[t] * w[t];
-				}
-				const double v = temp / abs[(size_t)j * ldab + kd];
-				xs[j] = v;
-#pragma unroll
-				for (int t = 0; t < KW - 1; ++t) w[t] = w[t + 1];
-				w[KW - 1] = v;
-			}
-			// backward: cur = xs[j] with the updates of the rows below applied,
-			// w[t] = xs[j - KW + t] pending
-#pragma unroll
-			for (int t = 0; t < KW; ++t) {
-				const int i = n - 1 - KW + t;
-				w[t] = i >= 0 ? xs[i] : 0.0;
-			}
-			double cur = xs[n - 1];
-			for (int j = n - 1; j >= 0; --j) {
-				if (cur != 0.0) {
-					cur = cur / abs[(size_t)j * ldab + kd];
-					const double temp = cur;
-					const double *arow = abs + (size_t)j * ldab + kd - j;
-#pragma unroll
-					for (int t = KW - 1; t >= 0; --t) {
-						const int i = j - KW + t;
-						if (i >= 0 && i >= j - kd) w[t] = w[t] - temp * arow[i];
+	if (threadIdx.x < 32) {
+		const int lane = threadIdx.x;
+		for (int leg = 0; leg < 2; ++leg) {  // one copy of the step for both sweeps
+			const int dir = leg == 0 ? 1 : -1, end = leg == 0 ? n : -1;
+			// U(r, c), r <= c: the coefficient between unknowns i and i + dir (1 + m)
+			auto coef = [&](int i, int m) -> double {
+				const int o = i + dir * (1 + m);
+				if (m >= kd || i < 0 || i >= n || o < 0 || o >= n) return 0.0;
+				const int c = leg == 0 ? o : i, r = leg == 0 ? i : o;
+				return abs[(size_t)c * ldab + kd + r - c];
+			};
+			auto pivot = [&](int i) { return i >= 0 && i < n ? abs[(size_t)i * ldab + kd] : 1.0; };
+			int i = leg == 0 ? 0 : n - 1;
+			double d = pivot(i), a = coef(i, lane);
+			for (; i != end; i += dir) {
+				const double dn = pivot(i + dir), an = coef(i + dir, lane);
+				double v = xs[i];
+				__syncwarp();  // every lane has read the unknown
+				const bool go = leg == 0 || v != 0.0;
+				if (go) {
+					v = v / d;
+					if (lane == 0) xs[i] = v;
+					const int o = i + dir * (1 + lane);
+					if (lane < kd && o >= 0 && o < n) xs[o] = xs[o] - a * v;
+					for (int m = lane + 32; m < kd; m += 32) {
+						const int om = i + dir * (1 + m);
+						if (om >= 0 && om < n) xs[om] = xs[om] - coef(i, m) * v;
 					}
 				}
-				xs[j] = cur;
-				cur = w[KW - 1];
-#pragma unroll
-				for (int t = KW - 1; t >= 1; --t) w[t] = w[t - 1];
-				const int i = j - 1 - KW;  // no row at or below j updates it
-				w[0] = i >= 0 ? xs[i] : 0.0;
-			}
-		} else {
-			for (int j = 0; j < n; ++j) {
-				double temp = xs[j];
-				const int i0 = j - kd > 0 ? j - kd : 0;
-				for (int i = i0; i < j; ++i) temp = temp - abs[(size_t)j * ldab + kd + i - j] * xs[i];
-				xs[j] = temp / abs[(size_t)j * ldab + kd];
-			}
-			for (int j = n - 1; j >= 0; --j) {
-				if (xs[j] != 0.0) {
-					xs[j] = xs[j] / abs[(size_t)j * ldab + kd];
-					const double temp = xs[j];
-					const int i1 = j - kd > 0 ? j - kd : 0;
-					for (int i = j - 1; i >= i1; --i) xs[i] = xs[i] - temp * abs[(size_t)j * ldab + kd + i - j];
-				}
+				d = dn;
+				a = an;
+				__syncwarp();
 			}
 		}
 	}
@@ -469,63 +499,28 @@ __device__ void cc_cg(const CoarseLevel<T> &L, double *xs)
 	cc_rows(1, L.nx, 1, L.ny, [&](int i, int j) { L.x[(size_t)j * L.pitch + i] = (T)xs[(j - 1) * L.nx + i - 1]; });
 }
 
-// Shared-memory map: the levels' copies (cc_view), the line right-hand sides,
-// then (8-byte aligned) the coarsest solve's vector and factor in FP64.
 template <typename T>
-__host__ __device__ inline void cc_layout(const CoarseCycle<T> &cc, size_t *levels, size_t *lines, size_t *dbl)
-{
-	size_t lv = 0, ln = 0;
-	for (int l = 0; l < cc.nl; ++l) {
-		lv += cc_elems(cc, l);
-		if (l + 1 < cc.nl) {
-			const CoarseLevel<T> &L = cc.lv[l];
-			const size_t a = (size_t)((L.ny + 1) / 2) * L.nx, b = (size_t)((L.nx + 1) / 2) * L.ny;
-			ln = ln > a ? ln : a;
-			ln = ln > b ? ln : b;
-		}
-	}
-	const CoarseLevel<T> &Cg = cc.lv[cc.nl - 1];
-	const size_t n = (size_t)Cg.nx * Cg.ny;
-	*levels = lv;
-	*lines = ln;
-	*dbl = n + (size_t)(Cg.nx + 2) * n;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(CC_THREADS) k_coarse_cycle(CoarseCycle<T> cc)
+__global__ void __launch_bounds__(CC_THREADS, sizeof(T) == 4 ? 2 : 1) k_coarse_cycle(const __grid_constant__ CcPlan<T> P)
 {
 	extern __shared__ __align__(16) unsigned char cc_smem[];
+	const CoarseCycle<T> &cc = P.cc;
 	T *base = reinterpret_cast<T *>(cc_smem);
-	size_t nlv, nln, ndbl;
-	cc_layout(cc, &nlv, &nln, &ndbl);
-	T *sm = base + nlv;  // line right-hand sides
-	double *xs = reinterpret_cast<double *>(cc_smem + ((nlv + nln) * sizeof(T) + 7) / 8 * 8);
+	T *sm = base + P.lines;  // line right-hand sides
+	double *xs = reinterpret_cast<double *>(cc_smem + P.dbl_byte);
 	const int nl = cc.nl;
-	// stage: operators, factors and weights of every level; b of the first level;
-	// x, r and the other b zero (ghost rings included)
-	for (int l = 0; l < nl; ++l) {
-		const CoarseLevel<T> G = cc_global(cc, l), S = cc_view(cc, l, base);
-		const size_t gpl = (size_t)G.pitch * (G.ny + 2), spl = (size_t)S.pitch * (S.ny + 2);
-		const int ii = G.nx + 2, jj = G.ny + 2;
-		if (l < nl - 1) {
-			cc_stage<T>(G.so, G.pitch, gpl, const_cast<T *>(S.so), S.pitch, spl, ii, jj, G.ns);
-			if (S.sor) cc_stage<T>(G.sor, G.pitch, gpl, const_cast<T *>(S.sor), S.pitch, spl, ii, jj, cc_sor_planes(cc.relax));
-			if (S.sory)  // transposed: nx+2 rows of ny+2 elements
-				cc_stage<T>(G.sory, G.tpitch, (size_t)G.tpitch * ii, const_cast<T *>(S.sory), S.tpitch,
-				            (size_t)S.tpitch * ii, jj, ii, 2);
-			cc_fill(S.r, spl);
-		}
-		if (l > 0) cc_stage<T>(G.ci, G.pitch, gpl, const_cast<T *>(S.ci), S.pitch, spl, ii, jj, 8);
-		if (l == 0) cc_stage<T>(G.b, G.pitch, gpl, S.b, S.pitch, spl, ii, jj, 1);
-		else cc_fill(S.b, spl);
-		cc_fill(S.x, spl);
-	}
-	{  // the coarsest level's band factor, after its right-hand side xs
+	// stage: operators, factors and weights of every level, b of the first level,
+	// and after the coarsest right-hand side xs its band factor; x, r and the other
+	// b zero (ghost rings included)
+	cc_stage<T>(P, base);
+	{
 		const CoarseLevel<T> &Cg = cc.lv[nl - 1];
 		const int n = Cg.nx * Cg.ny, nab = (Cg.nx + 2) * n;
-		cc_stage<double>(cc.abd + (size_t)blockIdx.x * cc.bstep * nab, 0, 0, xs + n, 0, 0, nab, 1, 1);
+		const double *src = cc.abd + (size_t)blockIdx.x * cc.bstep * nab;
+		const unsigned dst = (unsigned)__cvta_generic_to_shared(xs + n);
+		for (int e = threadIdx.x; e < nab; e += CC_THREADS) cp_async<8>(dst + 8u * e, src + e);
 	}
-	cc_stage_wait();
+	for (int e = threadIdx.x; e < P.nzero; e += CC_THREADS) base[e] = T(0);
+	asm volatile("cp.async.wait_all;\n" ::: "memory");
 	__syncthreads();
 	// The cycle as one sequence of steps (down: smooth, residual, restriction,
 	// and the coarsest solve after the last; up: interpolation, smooth), so that
@@ -533,13 +528,13 @@ __global__ void __launch_bounds__(CC_THREADS) k_coarse_cycle(CoarseCycle<T> cc)
 	// region from instruction memory costs several microseconds, and separate
 	// copies for the two legs paid it twice.
 	if (nl == 1) {
-		cc_cg<T>(cc_view(cc, 0, base), xs);
+		cc_cg<T>(cc_view(P, 0, base), xs);
 		__syncthreads();
 	}
 	for (int step = 0; step < 2 * (nl - 1); ++step) {
 		const bool down = step < nl - 1;
 		const int l = down ? step : 2 * (nl - 1) - 1 - step;
-		const CoarseLevel<T> F = cc_view(cc, l, base), C = cc_view(cc, l + 1, base);
+		const CoarseLevel<T> F = cc_view(P, l, base), C = cc_view(P, l + 1, base);
 		if (!down) {
 			cc_interp<T>(F, C);
 			__syncthreads();
@@ -551,11 +546,10 @@ __global__ void __launch_bounds__(CC_THREADS) k_coarse_cycle(CoarseCycle<T> cc)
 			if (F.ns == 5) cc_residual<T, 5>(F);
 			else cc_residual<T, 3>(F);
 			__syncthreads();
-			cc_restrict<T>(F, C);
-			cc_fill(C.x, (size_t)C.pitch * (C.ny + 2));
+			cc_restrict<T>(F, C);  // the coarse iterate is still zero
 			__syncthreads();
 			if (l == nl - 2) {
-				cc_cg<T>(cc_view(cc, nl - 1, base), xs);
+				cc_cg<T>(cc_view(P, nl - 1, base), xs);
 				__syncthreads();
 			}
 		} else {
@@ -563,24 +557,18 @@ __global__ void __launch_bounds__(CC_THREADS) k_coarse_cycle(CoarseCycle<T> cc)
 		}
 	}
 	{
-		const CoarseLevel<T> G = cc_global(cc, 0), S = cc_view(cc, 0, base);
-		cc_copy<T>(S.x, S.pitch, 0, G.x, G.pitch, 0, G.nx + 2, G.ny + 2, 1);
+		const CoarseLevel<T> S = cc_view(P, 0, base);
+		const int gp = cc.lv[0].pitch;
+		T *x = cc.lv[0].x + (size_t)blockIdx.x * cc.bstep * gp * (S.ny + 2);
+		cc_rows(0, S.nx + 1, 0, S.ny + 1, [&](int i, int j) { x[(size_t)j * gp + i] = S.x[(size_t)j * S.pitch + i]; });
 	}
-}
-
-template <typename T>
-size_t coarse_cycle_smem(const CoarseCycle<T> &cc)
-{
-	size_t nlv, nln, ndbl;
-	cc_layout(cc, &nlv, &nln, &ndbl);
-	return ((nlv + nln) * sizeof(T) + 7) / 8 * 8 + ndbl * sizeof(double);
 }
 
 // Shared memory a fused coarse cycle from level descriptor lv[0..nl) needs
 template <typename T>
 size_t coarse_cycle_bytes(const CoarseCycle<T> &cc)
 {
-	return coarse_cycle_smem(cc);
+	return cc_plan(cc).bytes;
 }
 template size_t coarse_cycle_bytes<double>(const CoarseCycle<double> &);
 template size_t coarse_cycle_bytes<float>(const CoarseCycle<float> &);
@@ -592,12 +580,13 @@ int coarse_cycle(const CoarseCycle<T> &cc, int nproblems, cudaStream_t st)
 		set_error(CDR_ERR_DIM, "fused coarse cycle over %d levels", cc.nl);
 		return CDR_ERR_DIM;
 	}
-	const size_t smem = coarse_cycle_smem(cc);
+	const CcPlan<T> plan = cc_plan(cc);
+	const size_t smem = plan.bytes;
 	if (smem > kCoarseSmemMax) {
 		set_error(CDR_ERR_DIM, "fused coarse cycle needs %zu bytes of shared memory", smem);
 		return CDR_ERR_DIM;
 	}
-	k_coarse_cycle<T><<<nproblems, CC_THREADS, smem, st>>>(cc);
+	k_coarse_cycle<T><<<nproblems, CC_THREADS, smem, st>>>(plan);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

@@ -182,6 +182,33 @@ def test_fused_coarse_cycle_fp32():
     assert abs(its[0] - its[1]) <= 1
 
 
+@pytest.mark.parametrize("nx,ny", [(61, 63), (63, 64), (65, 66), (94, 51), (127, 30)])
+@pytest.mark.parametrize("levels", [-1, 2])
+def test_fused_coarse_cycle_line_edges(nx, ny, levels):
+    """Fused levels whose lines end around a warp's 32 positions, and coarsest levels whose band is
+    wider than a warp (two levels): FP64 bits of the separate kernels, FP32 to the tolerance in as
+    many cycles."""
+    from cedar_b200 import gallery as G
+    from cedar_b200.config import Config
+    from cedar_b200.solver import Solver2D
+    rng = np.random.default_rng(nx + ny)
+    k = np.exp(rng.standard_normal((ny + 1, nx + 1)))
+    so = G.fe_hetero(k, k)
+    b = np.zeros((ny + 2, nx + 2))
+    b[1:-1, 1:-1] = rng.uniform(0, 1, size=(ny, nx))
+    out = {}
+    for fuse in (64, 0):
+        for prec in ("fp64", "fp32-ir"):
+            s = Solver2D(so, Config({"solver": {"relaxation": "line-xy", "max-iter": 30, "tol": 1e-9,
+                                                "num-levels": levels},
+                                     "gpu": {"precision": prec, "line-solve": "sequential", "fuse-coarse": fuse}}))
+            out[fuse, prec] = s.solve(b), s.history.copy()
+    assert np.array_equal(out[64, "fp64"][0], out[0, "fp64"][0])
+    assert np.array_equal(out[64, "fp64"][1], out[0, "fp64"][1])
+    assert out[64, "fp32-ir"][1][-1] < 1e-9
+    assert abs(len(out[64, "fp32-ir"][1]) - len(out[0, "fp32-ir"][1])) <= 1
+
+
 @pytest.mark.parametrize("relax,ns", [("line-xy", 5), ("point", 3)])
 def test_fcycle_fp64_matches_oracle(oracle, relax, ns):
     """solver.cycle.type = "f" (cycle::fcycle): with the sequential line
