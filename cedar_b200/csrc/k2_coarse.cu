@@ -251,6 +251,65 @@ __device__ void cc_gs(const CoarseLevel<T> &L, int updown)
 	}
 }
 
+// FP32 solve of a line of n <= 32 CS points by one warp, CS consecutive positions
+// per lane in registers from their right-hand sides to their solution: the
+// chunk form of cc_lines (affine maps of the chunks scanned over the lanes) with
+// its operations and bits.  dd / ee: factors of position p (from 1) at dd[p], ee[p].
+template <typename T, int CS, typename RHS, typename PUT>
+__device__ __forceinline__ void cc_line(const T *dd, const T *ee, int n, RHS rhs, PUT put)
+{
+	const int lane = threadIdx.x & 31, lo = lane * CS;
+	T r[CS], e[CS + 1], dv[CS];  // e[c]: multiplier of position lo + c, e[CS] of the one after the chunk
+#pragma unroll
+	for (int c = 0; c <= CS; ++c) e[c] = lo + c > 0 && lo + c < n ? ee[lo + c + 1] : T(0);
+#pragma unroll
+	for (int c = 0; c < CS; ++c) {
+		dv[c] = lo + c < n ? dd[lo + c + 1] : T(0);
+		r[c] = lo + c < n ? rhs(lo + c) : T(0);
+	}
+	T A = T(1), B = T(0);
+#pragma unroll
+	for (int c = 0; c < CS; ++c)
+		if (lo + c < n) {
+			B = madd(-e[c], B, r[c]);
+			A = -e[c] * A;
+		}
+#pragma unroll
+	for (int off = 1; off < 32; off <<= 1) {
+		const T a2 = __shfl_up_sync(0xffffffffu, A, off), b2 = __shfl_up_sync(0xffffffffu, B, off);
+		if (lane >= off) { B = madd(A, b2, B); A = A * a2; }
+	}
+	T v = __shfl_up_sync(0xffffffffu, B, 1);
+	if (lane == 0) v = T(0);
+#pragma unroll
+	for (int c = 0; c < CS; ++c)
+		if (lo + c < n) {
+			v = lo + c == 0 ? r[c] : madd(-v, e[c], r[c]);
+			r[c] = pivot_div(v, dv[c]);
+		}
+	A = T(1);
+	B = T(0);
+#pragma unroll
+	for (int c = CS - 1; c >= 0; --c)
+		if (lo + c < n) {
+			B = madd(-e[c + 1], B, r[c]);
+			A = -e[c + 1] * A;
+		}
+#pragma unroll
+	for (int off = 1; off < 32; off <<= 1) {
+		const T a2 = __shfl_down_sync(0xffffffffu, A, off), b2 = __shfl_down_sync(0xffffffffu, B, off);
+		if (lane + off < 32) { B = madd(A, b2, B); A = A * a2; }
+	}
+	v = __shfl_down_sync(0xffffffffu, B, 1);
+	if (lane == 31) v = T(0);
+#pragma unroll
+	for (int c = CS - 1; c >= 0; --c)
+		if (lo + c < n) {
+			v = lo + c == n - 1 ? r[c] : madd(-v, e[c + 1], r[c]);
+			put(lo + c, v);
+		}
+}
+
 // One zebra line sweep (both colours, relax_lines_2d's order).  Each colour:
 // each line's warp forms its right-hand sides into sm (the other warps solve
 // lines of the same colour, which this line does not read), then the
@@ -338,37 +397,14 @@ __device__ void cc_lines(const CoarseLevel<T> &L, int updown, T *sm)
 			}
 		} else {
 			const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-			if (n <= 32) {
-				// one position per lane, the line in registers from its right-hand side to
-				// its solution: the chunk form below with chunks of one position (its bits)
+			if (n <= 64) {
 				for (int g = warp; g < ml; g += CC_WARPS) {
-					const int lc = first + 2 * g, m = lane;
-					const bool in = m < n;
+					const int lc = first + 2 * g;
 					const T *dd = fac + (DIR == CDR_DIR_X ? (size_t)lc * L.pitch : (size_t)lc * L.tpitch);
-					const T *ee = dd + eplane;
-					const T e0 = in && m > 0 ? ee[m + 1] : T(0), e1 = in && m < n - 1 ? ee[m + 2] : T(0);
-					const T dv = in ? dd[m + 1] : T(0);
-					const size_t k = xat(lc, in ? m : 0);
-					T r = line_rhs<T, NS, DIR>(L.so, ps, L.x, L.b, k, L.pitch);
-					T A = in ? -e0 : T(1), B = in ? r : T(0);
-#pragma unroll
-					for (int off = 1; off < 32; off <<= 1) {
-						const T a2 = __shfl_up_sync(0xffffffffu, A, off), b2 = __shfl_up_sync(0xffffffffu, B, off);
-						if (lane >= off) { B = madd(A, b2, B); A = A * a2; }
-					}
-					T y = __shfl_up_sync(0xffffffffu, B, 1);
-					y = m == 0 ? r : madd(-y, e0, r);
-					r = pivot_div(y, dv);
-					A = in ? -e1 : T(1);
-					B = in ? r : T(0);
-#pragma unroll
-					for (int off = 1; off < 32; off <<= 1) {
-						const T a2 = __shfl_down_sync(0xffffffffu, A, off), b2 = __shfl_down_sync(0xffffffffu, B, off);
-						if (lane + off < 32) { B = madd(A, b2, B); A = A * a2; }
-					}
-					T xv = __shfl_down_sync(0xffffffffu, B, 1);
-					xv = m == n - 1 ? r : madd(-xv, e1, r);
-					if (in) L.x[k] = xv;
+					auto rhs = [&](int m) { return line_rhs<T, NS, DIR>(L.so, ps, L.x, L.b, xat(lc, m), L.pitch); };
+					auto put = [&](int m, T v) { L.x[xat(lc, m)] = v; };
+					if (n <= 32) cc_line<T, 1>(dd, dd + eplane, n, rhs, put);
+					else cc_line<T, 2>(dd, dd + eplane, n, rhs, put);
 				}
 				__syncthreads();
 				continue;
@@ -447,12 +483,9 @@ __device__ void cc_smooth(const CoarseCycle<T> &cc, const CoarseLevel<T> &L, int
 	}
 }
 
-// BMG2_SymStd_SOLVE_cg with DPBTRS('U') on the coarsest level by one warp: the
-// right-hand side in shared memory (xs), the factor after it (staged with the
-// levels).  Both sweeps run by columns: once an unknown is final, lane m
-// subtracts its term from the m-th unknown of the band ahead, so every unknown
-// receives its terms in DTBSV's order (the same bits) and a step of the chain
-// is one quotient and one update.  Pivot and coefficients load a step ahead.
+// BMG2_SymStd_SOLVE_cg with DPBTRS('U') on the coarsest level by one warp
+// (band_solve_warp): the right-hand side in shared memory (xs), the factor after
+// it (staged with the levels).
 template <typename T>
 __device__ void cc_cg(const CoarseLevel<T> &L, double *xs)
 {
@@ -460,41 +493,7 @@ __device__ void cc_cg(const CoarseLevel<T> &L, double *xs)
 	const double *abs = xs + n;
 	cc_rows(1, L.nx, 1, L.ny, [&](int i, int j) { xs[(j - 1) * L.nx + i - 1] = (double)L.b[(size_t)j * L.pitch + i]; });
 	__syncthreads();
-	if (threadIdx.x < 32) {
-		const int lane = threadIdx.x;
-		for (int leg = 0; leg < 2; ++leg) {  // one copy of the step for both sweeps
-			const int dir = leg == 0 ? 1 : -1, end = leg == 0 ? n : -1;
-			// U(r, c), r <= c: the coefficient between unknowns i and i + dir (1 + m)
-			auto coef = [&](int i, int m) -> double {
-				const int o = i + dir * (1 + m);
-				if (m >= kd || i < 0 || i >= n || o < 0 || o >= n) return 0.0;
-				const int c = leg == 0 ? o : i, r = leg == 0 ? i : o;
-				return abs[(size_t)c * ldab + kd + r - c];
-			};
-			auto pivot = [&](int i) { return i >= 0 && i < n ? abs[(size_t)i * ldab + kd] : 1.0; };
-			int i = leg == 0 ? 0 : n - 1;
-			double d = pivot(i), a = coef(i, lane);
-			for (; i != end; i += dir) {
-				const double dn = pivot(i + dir), an = coef(i + dir, lane);
-				double v = xs[i];
-				__syncwarp();  // every lane has read the unknown
-				const bool go = leg == 0 || v != 0.0;
-				if (go) {
-					v = v / d;
-					if (lane == 0) xs[i] = v;
-					const int o = i + dir * (1 + lane);
-					if (lane < kd && o >= 0 && o < n) xs[o] = xs[o] - a * v;
-					for (int m = lane + 32; m < kd; m += 32) {
-						const int om = i + dir * (1 + m);
-						if (om >= 0 && om < n) xs[om] = xs[om] - coef(i, m) * v;
-					}
-				}
-				d = dn;
-				a = an;
-				__syncwarp();
-			}
-		}
-	}
+	if (threadIdx.x < 32) band_solve_warp(abs, ldab, n, xs);
 	__syncthreads();
 	cc_rows(1, L.nx, 1, L.ny, [&](int i, int j) { L.x[(size_t)j * L.pitch + i] = (T)xs[(j - 1) * L.nx + i - 1]; });
 }

@@ -169,6 +169,48 @@ __device__ __forceinline__ T pivot_div(T y, T dstored)
 	return sizeof(T) == 4 ? y * dstored : y / dstored;
 }
 
+// DPBTRS('U') for one right-hand side xs (shared memory, n unknowns) by one warp,
+// factor ab(ldab, n), ldab - 1 entries above the diagonal.  Both sweeps run by
+// columns: once an unknown is final, lane m subtracts its term from the m-th
+// unknown of the band ahead, so every unknown receives its terms in DTBSV's
+// order (the same bits) and a step of the chain is one quotient and one update.
+// Pivot and coefficients load a step ahead.
+__device__ __forceinline__ void band_solve_warp(const double *ab, int ldab, int n, double *xs)
+{
+	const int lane = threadIdx.x & 31, kd = ldab - 1;
+	for (int leg = 0; leg < 2; ++leg) {  // one copy of the step for both sweeps
+		const int dir = leg == 0 ? 1 : -1, end = leg == 0 ? n : -1;
+		// U(r, c), r <= c: the coefficient between unknowns i and i + dir (1 + m)
+		auto coef = [&](int i, int m) -> double {
+			const int o = i + dir * (1 + m);
+			if (m >= kd || i < 0 || i >= n || o < 0 || o >= n) return 0.0;
+			const int c = leg == 0 ? o : i, r = leg == 0 ? i : o;
+			return ab[(size_t)c * ldab + kd + r - c];
+		};
+		auto pivot = [&](int i) { return i >= 0 && i < n ? ab[(size_t)i * ldab + kd] : 1.0; };
+		int i = leg == 0 ? 0 : n - 1;
+		double d = pivot(i), a = coef(i, lane);
+		for (; i != end; i += dir) {
+			const double dn = pivot(i + dir), an = coef(i + dir, lane);
+			double v = xs[i];
+			__syncwarp();  // every lane has read the unknown
+			if (leg == 0 || v != 0.0) {
+				v = v / d;
+				if (lane == 0) xs[i] = v;
+				const int o = i + dir * (1 + lane);
+				if (lane < kd && o >= 0 && o < n) xs[o] = xs[o] - a * v;
+				for (int m = lane + 32; m < kd; m += 32) {
+					const int om = i + dir * (1 + m);
+					if (om >= 0 && om < n) xs[om] = xs[om] - coef(i, m) * v;
+				}
+			}
+			d = dn;
+			a = an;
+			__syncwarp();
+		}
+	}
+}
+
 template <int NW>
 __device__ __forceinline__ double block_sum(double v, double *sh)
 {

@@ -939,31 +939,14 @@ template <typename T>
 __global__ void k_cg_solve(const double *__restrict__ ab, T *__restrict__ q, const T *__restrict__ qf, Dims2 d)
 {
 	extern __shared__ double xs[];
-	if (threadIdx.x != 0 || blockIdx.x != 0) return;
-	const int ldab = d.nx + 2, kd = d.nx + 1, n = d.nx * d.ny;
+	const int ldab = d.nx + 2, n = d.nx * d.ny, lane = threadIdx.x;
 	ab += d.bofs((size_t)ldab * n);
 	q += d.bofs(d.plane());
 	qf += d.bofs(d.plane());
-	int kk = 0;
-	for (int j = 1; j <= d.ny; ++j)
-		for (int i = 1; i <= d.nx; ++i) xs[kk++] = (double)qf[d.at(i, j)];
-	for (int j = 0; j < n; ++j) {
-		double temp = xs[j];
-		int i0 = j - kd > 0 ? j - kd : 0;
-		for (int i = i0; i < j; ++i) temp = temp - ab[(size_t)j * ldab + kd + i - j] * xs[i];
-		xs[j] = temp / ab[(size_t)j * ldab + kd];
-	}
-	for (int j = n - 1; j >= 0; --j) {
-		if (xs[j] != 0.0) {
-			xs[j] = xs[j] / ab[(size_t)j * ldab + kd];
-			double temp = xs[j];
-			int i1 = j - kd > 0 ? j - kd : 0;
-			for (int i = j - 1; i >= i1; --i) xs[i] = xs[i] - temp * ab[(size_t)j * ldab + kd + i - j];
-		}
-	}
-	kk = 0;
-	for (int j = 1; j <= d.ny; ++j)
-		for (int i = 1; i <= d.nx; ++i) q[d.at(i, j)] = (T)xs[kk++];
+	for (int m = lane; m < n; m += 32) xs[m] = (double)qf[d.at(m % d.nx + 1, m / d.nx + 1)];
+	__syncwarp();
+	band_solve_warp(ab, ldab, n, xs);
+	for (int m = lane; m < n; m += 32) q[d.at(m % d.nx + 1, m / d.nx + 1)] = (T)xs[m];
 }
 
 int setup_cg_2d(const double *so, int nstencil, Dims2 d, double *abd, int *info, cudaStream_t st)

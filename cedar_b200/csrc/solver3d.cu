@@ -311,7 +311,10 @@ static int create3(cdr_gpu_solver3 *h, const double *so_src, int src_pitch, cuda
 			s2.maxiter = 1;
 			s2.precision = s.precision;
 			s2.line_flags = s.line_flags;
-			s2.fuse_coarse = s.fuse_coarse;  // the planes' coarse levels fused as the caller asks
+			// the planes' coarse levels fused as the caller asks; FP32 planes from twice
+			// that edge where shared memory holds the level (one CTA per plane, tens of
+			// planes: 15 launches of a level of about 5 us each become one CTA's steps)
+			s2.fuse_coarse = h->mixed() && s.fuse_coarse < 1 << 20 ? 2 * s.fuse_coarse : s.fuse_coarse;
 			const int np = dir == 0 ? L.nz : dir == 1 ? L.ny : L.nx;
 			const int n1 = dir == 2 ? L.ny : L.nx, n2 = dir == 0 ? L.ny : L.nz;
 			L.pl[dir].reset(new Batch2());
