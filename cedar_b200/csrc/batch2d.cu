@@ -356,6 +356,7 @@ namespace {
 __global__ void k_masked_copy(const double *__restrict__ src, double *__restrict__ dst, size_t per,
                               const int *__restrict__ flag)
 {
+	await_previous();
 	if (!flag[blockIdx.z]) return;
 	const size_t o = (size_t)blockIdx.z * per;
 	for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < per; e += (size_t)gridDim.x * blockDim.x)
@@ -575,7 +576,7 @@ int cdr_gpu_batch2d_solve_device(cdr_gpu_batch2d *h, const double *b_dev, double
 			CDR_TRY(h->run_cycle(0));
 			CDR_TRY(residual_2d<double>(F.so, F.ns, F.x, F.b, F.r, d, h->norm, h->partial, st));
 			// keep the iterate of every problem still iterating
-			k_masked_copy<<<cgrid, 256, 0, st>>>(F.x, h->x64[0], pl, h->active);
+			launch(k_masked_copy, cgrid, 256, 0, st, F.x, h->x64[0], pl, h->active);
 			CDR_LAUNCH_CHECK();
 		}
 		CDR_CUDA_TRY(cudaEventRecord(h->ev[it + 1], st));

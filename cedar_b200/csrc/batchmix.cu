@@ -72,6 +72,7 @@ struct Cls {
 
 __global__ void k_zero_f32(float *__restrict__ p, size_t n)
 {
+	await_previous();
 	for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
 		p[e] = 0.f;
 }
@@ -582,7 +583,7 @@ int cdr_gpu_batchmix_solve_device(cdr_gpu_batchmix *h, const double *const *b_de
 			if (C.size[0] < h->smoothed_sizes()) continue;  // the cycle's first sweep treats it as zero
 			B2Level &F = C.B->lv[0];
 			const size_t n = F.plane() * C.nb;
-			k_zero_f32<<<(unsigned)std::min<size_t>((n + 255) / 256, 148 * 16), 256, 0, st>>>(F.x32, n);
+			launch(k_zero_f32, (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16), 256, 0, st, F.x32, n);
 			CDR_LAUNCH_CHECK();
 		}
 		CDR_TRY(h->run_cycle());

@@ -46,6 +46,71 @@ void count_launches(long long n);
 // cdr_gpu_last_error() reports its text.
 void set_error(int code, const char *fmt, ...);
 
+// Kernel launch.  Where it pays, the grid depends programmatically on the kernel
+// before it in the stream: it becomes resident while that one drains, which hides
+// the launch and the first instruction fetch of the many short kernels of a cycle.
+// Every kernel launched here begins with await_previous(): it touches no memory
+// before the kernels ahead of it have completed.
+// The rule counts SMs' worth of blocks (threads or shared memory, whichever fills
+// an SM first).  Blocks that become resident early settle on the SMs that are
+// free first, so a grid that does not fill the chip piles up on a few SMs when a
+// large kernel is draining (2047^2: an FCG iteration 718 -> 750 us), and so do
+// blocks of more than an eighth of an SM (all grids early: 881 us).  Early
+// therefore: grids of small blocks, up to about a wave, that either fill most of the
+// chip or follow a kernel that left half of it free; a few large blocks always.
+struct LaunchSize {
+	double sms, block;  // SMs' worth of the grid; part of an SM one block takes
+	double blocks;
+};
+inline LaunchSize launch_size(dim3 grid, dim3 block, size_t smem)
+{
+	LaunchSize z;
+	z.blocks = (double)grid.x * grid.y * grid.z;
+	const double th = (double)(block.x * block.y * block.z) / 2048.0, sm = (double)smem / (228.0 * 1024.0);
+	z.block = th > sm ? th : sm;
+	z.sms = z.blocks * z.block;
+	return z;
+}
+inline bool launch_early(const LaunchSize &z, double before)
+{
+	if (z.blocks <= 16.0) return true;
+	return z.block <= 0.126 && z.sms <= 185.0 && (z.sms >= 60.0 || before <= 74.0);
+}
+// SMs' worth of this thread's last launch (only weighs the choice above)
+inline double &launch_before()
+{
+	static thread_local double sms = 0.0;
+	return sms;
+}
+
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[0].val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = block;
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = st;
+	cfg.attrs = attr;
+	const LaunchSize z = launch_size(grid, block, smem);
+	cfg.numAttrs = launch_early(z, launch_before()) ? 1 : 0;
+	launch_before() = z.sms;
+	(void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // CDR_LAUNCH_CHECK reads the error
+}
+
+#ifdef __CUDACC__
+// First statement of every kernel started by launch(): waits for the kernels
+// ahead to complete, then lets the next one become resident (its own wait
+// keeps it from running; one grid ahead at a time).
+__device__ __forceinline__ void await_previous()
+{
+	asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 #define CDR_CUDA_TRY(expr)                                                          \
 	do {                                                                            \
 		cudaError_t _e = (expr);                                                    \

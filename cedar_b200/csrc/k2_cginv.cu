@@ -34,6 +34,7 @@ constexpr int CGI_RING = 128;  // ring slots per column (>= kd + 2)
 __global__ void __launch_bounds__(32) k_cg_inverse(const double *__restrict__ ab, int n, int kd, int ldab,
                                                    double *__restrict__ ainv)
 {
+	await_previous();
 	__shared__ double ring[CGI_RING][32];
 	__shared__ double ucol[2][CGI_RING];
 	const int lane = threadIdx.x, c0 = blockIdx.x * 32, c = c0 + lane;
@@ -90,6 +91,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_cg_inv_apply(const T *__restrict__ ainv, T *__restrict__ q,
                                                       const T *__restrict__ qf, Dims2 d)
 {
+	await_previous();
 	extern __shared__ __align__(16) unsigned char cgi_raw[];
 	T *bs = reinterpret_cast<T *>(cgi_raw);
 	constexpr int V = 16 / sizeof(T);
@@ -150,6 +152,7 @@ template <typename T>
 __global__ void __launch_bounds__(IA_BLOCK) k_cg_inv_apply_bulk(const T *__restrict__ ainv, T *__restrict__ q,
                                                                 const T *__restrict__ qf, Dims2 d)
 {
+	await_previous();
 	extern __shared__ __align__(128) unsigned char ia_raw[];
 	__shared__ double red[IA_BLOCK / 32];
 	constexpr int V = 16 / sizeof(T);
@@ -263,7 +266,7 @@ int cg_inverse_2d(const double *abd, Dims2 d, double *ainv, cudaStream_t st)
 		set_error(CDR_ERR_DIM, "coarsest grid %dx%d too wide for the inverse (bandwidth %d)", d.nx, d.ny, kd);
 		return CDR_ERR_DIM;
 	}
-	k_cg_inverse<<<ceil_div(n, 32), 32, 0, st>>>(abd, n, kd, ldab, ainv);
+	launch(k_cg_inverse, ceil_div(n, 32), 32, 0, st, abd, n, kd, ldab, ainv);
 	CDR_LAUNCH_CHECK();
 	// the streamed product's shared-memory opt-in (setup time, before any capture)
 	const size_t big = 226 * 1024;
@@ -291,12 +294,12 @@ int solve_cg_inv_2d(const T *ainv, T *x, const T *b, Dims2 d, cudaStream_t st)
 		}();
 		const int per_sm = (int)((228 * 1024) / (smb + 1024));
 		const int g = slots * (per_sm > 0 ? per_sm : 1);
-		k_cg_inv_apply_bulk<T><<<n < g ? n : g, IA_BLOCK, smb, st>>>(ainv, x, b, d);
+		launch(k_cg_inv_apply_bulk<T>, n < g ? n : g, IA_BLOCK, smb, st, ainv, x, b, d);
 		CDR_LAUNCH_CHECK();
 		return CDR_OK;
 	}
 	const int rows_per_cta = 256 / 32, grid = ceil_div(n, rows_per_cta) < 148 * 4 ? ceil_div(n, rows_per_cta) : 148 * 4;
-	k_cg_inv_apply<T><<<grid, 256, sm, st>>>(ainv, x, b, d);
+	launch(k_cg_inv_apply<T>, grid, 256, sm, st, ainv, x, b, d);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

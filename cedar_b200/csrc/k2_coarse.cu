@@ -501,6 +501,7 @@ __device__ void cc_cg(const CoarseLevel<T> &L, double *xs)
 template <typename T>
 __global__ void __launch_bounds__(CC_THREADS, sizeof(T) == 4 ? 2 : 1) k_coarse_cycle(const __grid_constant__ CcPlan<T> P)
 {
+	await_previous();
 	extern __shared__ __align__(16) unsigned char cc_smem[];
 	const CoarseCycle<T> &cc = P.cc;
 	T *base = reinterpret_cast<T *>(cc_smem);
@@ -585,7 +586,7 @@ int coarse_cycle(const CoarseCycle<T> &cc, int nproblems, cudaStream_t st)
 		set_error(CDR_ERR_DIM, "fused coarse cycle needs %zu bytes of shared memory", smem);
 		return CDR_ERR_DIM;
 	}
-	k_coarse_cycle<T><<<nproblems, CC_THREADS, smem, st>>>(plan);
+	launch(k_coarse_cycle<T>, nproblems, CC_THREADS, smem, st, plan);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

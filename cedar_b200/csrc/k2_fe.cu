@@ -37,6 +37,7 @@ struct CellK {
 
 __global__ void k_fe_assemble(CellK K, double *__restrict__ so, Dims2 d)
 {
+	await_previous();
 	const int i = blockIdx.x * TX + threadIdx.x + 1, j = blockIdx.y * TY + threadIdx.y + 1;
 	if (i > d.nx || j > d.ny) return;
 	const size_t ps = d.plane(), k = d.at(i, j);
@@ -73,6 +74,7 @@ __global__ void k_fe_assemble(CellK K, double *__restrict__ so, Dims2 d)
 __global__ void k_fe_grad(const double *__restrict__ u, const double *__restrict__ lam, Dims2 d,
                           double *__restrict__ gkx, double *__restrict__ gky, int cp)
 {
+	await_previous();
 	const int ci = blockIdx.x * TX + threadIdx.x, cj = blockIdx.y * TY + threadIdx.y;
 	if (ci > d.nx || cj > d.ny) return;
 	double ul[4], ll[4];
@@ -112,7 +114,7 @@ int cdr_gpu_fe_assemble_2d_f64(const double *kx, const double *ky, int cell_pitc
 	}
 	const Dims2 d{nx, ny, pitch};
 	CDR_CUDA_TRY(cudaMemsetAsync(so, 0, sizeof(double) * d.plane() * 5, stream));
-	k_fe_assemble<<<dim3(ceil_div(nx, TX), ceil_div(ny, TY)), dim3(TX, TY), 0, stream>>>(CellK{kx, ky, cell_pitch}, so,
+	launch(k_fe_assemble, dim3(ceil_div(nx, TX), ceil_div(ny, TY)), dim3(TX, TY), 0, stream, CellK{kx, ky, cell_pitch}, so,
 	                                                                                     d);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -127,7 +129,7 @@ int cdr_gpu_fe_grad_2d_f64(const double *u, const double *lam, int nx, int ny, i
 		return CDR_ERR_DIM;
 	}
 	const Dims2 d{nx, ny, pitch};
-	k_fe_grad<<<dim3(ceil_div(nx + 1, TX), ceil_div(ny + 1, TY)), dim3(TX, TY), 0, stream>>>(u, lam, d, gkx, gky,
+	launch(k_fe_grad, dim3(ceil_div(nx + 1, TX), ceil_div(ny + 1, TY)), dim3(TX, TY), 0, stream, u, lam, d, gkx, gky,
 	                                                                                        cell_pitch);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -166,6 +168,7 @@ __constant__ signed char c_planes3[14][2][3] = {
 __global__ void k_fe_assemble3(const double *__restrict__ kc, int cp, int cs, double *__restrict__ so, int nx, int ny,
                                int nz, int pitch)
 {
+	await_previous();
 	const int i = blockIdx.x * TX + threadIdx.x + 1, j = blockIdx.y * TY + threadIdx.y + 1, k = blockIdx.z + 1;
 	if (i > nx || j > ny) return;
 	const double h = 1.0 / (nx + 1);
@@ -202,7 +205,7 @@ extern "C" int cdr_gpu_fe_assemble_3d_f64(const double *k, int cell_pitch, int c
 	}
 	const size_t plane = (size_t)pitch * (ny + 2) * (nz + 2);
 	CDR_CUDA_TRY(cudaMemsetAsync(so, 0, sizeof(double) * plane * 14, stream));
-	k_fe_assemble3<<<dim3(ceil_div(nx, TX), ceil_div(ny, TY), nz), dim3(TX, TY), 0, stream>>>(k, cell_pitch, cell_slice,
+	launch(k_fe_assemble3, dim3(ceil_div(nx, TX), ceil_div(ny, TY), nz), dim3(TX, TY), 0, stream, k, cell_pitch, cell_slice,
 	                                                                                         so, nx, ny, nz, pitch);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;

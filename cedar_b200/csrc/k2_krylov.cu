@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(TX *TY) k_fcg_beta(const TZ *__restrict__ z, c
                                                      const double *__restrict__ q, Dims2 d,
                                                      double *__restrict__ partial, FcgScalars *S)
 {
+	await_previous();
 	double acc[1] = {0.0};
 	if (!S->first) {
 		int i, j;
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(TX *TY) k_fcg_dir(const double *__restrict__ s
                                                     double *__restrict__ q, const double *__restrict__ r, Dims2 d,
                                                     double *__restrict__ partial, FcgScalars *S)
 {
+	await_previous();
 	const size_t ps = d.plane();
 	const int pitch = d.pitch;
 	const bool odd = S->iter & 1;
@@ -192,6 +194,7 @@ __global__ void __launch_bounds__(TX *TY) k_fcg_update(const double *__restrict_
                                                        TZ *__restrict__ z, Dims2 d, double *__restrict__ partial,
                                                        FcgScalars *S)
 {
+	await_previous();
 	const size_t ps = d.plane();
 	const int pitch = d.pitch;
 	const bool odd = S->iter & 1;
@@ -239,6 +242,7 @@ __global__ void __launch_bounds__(TX *TY) k_fcg_update_rec(double *__restrict__ 
                                                            TZ *__restrict__ z, Dims2 d, double *__restrict__ partial,
                                                            FcgScalars *S)
 {
+	await_previous();
 	const int pitch = d.pitch;
 	const bool odd = S->iter & 1;
 	const double *__restrict__ pnew = odd ? p0 : p1;
@@ -271,6 +275,7 @@ template <typename TZ>
 __global__ void __launch_bounds__(TX *TY) k_fcg_load(const double *__restrict__ r, TZ *__restrict__ rin,
                                                      TZ *__restrict__ z, Dims2 d, FcgScalars *S, int restart)
 {
+	await_previous();
 	const int i = blockIdx.x * TX + threadIdx.x, j = blockIdx.y * TY + threadIdx.y;
 	if (i > d.nx + 1 || j > d.ny + 1) return;
 	const size_t k = d.at(i, j);
@@ -288,7 +293,7 @@ __global__ void __launch_bounds__(TX *TY) k_fcg_load(const double *__restrict__ 
 template <typename TZ>
 int fcg_load(const double *r, TZ *rin, TZ *z, Dims2 d, FcgScalars *S, cudaStream_t st, bool restart)
 {
-	k_fcg_load<TZ><<<dim3(ceil_div(d.nx + 2, TX), ceil_div(d.ny + 2, TY)), dim3(TX, TY), 0, st>>>(r, rin, z, d, S,
+	launch(k_fcg_load<TZ>, dim3(ceil_div(d.nx + 2, TX), ceil_div(d.ny + 2, TY)), dim3(TX, TY), 0, st, r, rin, z, d, S,
 	                                                                                         restart ? 1 : 0);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -305,20 +310,20 @@ int fcg_step(const double *so, int ns, const TZ *z, const float *zf, TR *rin, TR
 {
 	const dim3 nb(ceil_div(d.nx, TX), ceil_div(d.ny, TY * FR)), blk(TX, TY);
 	if (zf) {
-		k_fcg_beta<TZ, true><<<nb, blk, 0, st>>>(z, zf, q, d, partial, S);
+		launch(k_fcg_beta<TZ, true>, nb, blk, 0, st, z, zf, q, d, partial, S);
 		CDR_LAUNCH_CHECK();
-		if (ns == 5) k_fcg_dir<TZ, 5, true><<<nb, blk, 0, st>>>(so, z, zf, p0, p1, q, r, d, partial, S);
-		else k_fcg_dir<TZ, 3, true><<<nb, blk, 0, st>>>(so, z, zf, p0, p1, q, r, d, partial, S);
+		if (ns == 5) launch(k_fcg_dir<TZ, 5, true>, nb, blk, 0, st, so, z, zf, p0, p1, q, r, d, partial, S);
+		else launch(k_fcg_dir<TZ, 3, true>, nb, blk, 0, st, so, z, zf, p0, p1, q, r, d, partial, S);
 	} else {
-		k_fcg_beta<TZ, false><<<nb, blk, 0, st>>>(z, nullptr, q, d, partial, S);
+		launch(k_fcg_beta<TZ, false>, nb, blk, 0, st, z, nullptr, q, d, partial, S);
 		CDR_LAUNCH_CHECK();
-		if (ns == 5) k_fcg_dir<TZ, 5, false><<<nb, blk, 0, st>>>(so, z, nullptr, p0, p1, q, r, d, partial, S);
-		else k_fcg_dir<TZ, 3, false><<<nb, blk, 0, st>>>(so, z, nullptr, p0, p1, q, r, d, partial, S);
+		if (ns == 5) launch(k_fcg_dir<TZ, 5, false>, nb, blk, 0, st, so, z, nullptr, p0, p1, q, r, d, partial, S);
+		else launch(k_fcg_dir<TZ, 3, false>, nb, blk, 0, st, so, z, nullptr, p0, p1, q, r, d, partial, S);
 	}
 	CDR_LAUNCH_CHECK();
-	if (!formed) k_fcg_update_rec<TR><<<nb, blk, 0, st>>>(x0, x1, r, p0, p1, q, rin, zz, d, partial, S);
-	else if (ns == 5) k_fcg_update<TR, 5><<<nb, blk, 0, st>>>(so, x0, x1, b, r, p0, p1, rin, zz, d, partial, S);
-	else k_fcg_update<TR, 3><<<nb, blk, 0, st>>>(so, x0, x1, b, r, p0, p1, rin, zz, d, partial, S);
+	if (!formed) launch(k_fcg_update_rec<TR>, nb, blk, 0, st, x0, x1, r, p0, p1, q, rin, zz, d, partial, S);
+	else if (ns == 5) launch(k_fcg_update<TR, 5>, nb, blk, 0, st, so, x0, x1, b, r, p0, p1, rin, zz, d, partial, S);
+	else launch(k_fcg_update<TR, 3>, nb, blk, 0, st, so, x0, x1, b, r, p0, p1, rin, zz, d, partial, S);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

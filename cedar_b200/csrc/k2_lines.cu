@@ -141,6 +141,7 @@ template <bool W64, bool W32>
 __global__ void __launch_bounds__(32) k_lines_setup(const double *__restrict__ so, int ns, LineFactors f, Dims2 d,
                                                     int tpitch, int dir0, bool vecx, bool vecy, int *__restrict__ info)
 {
+	await_previous();
 	if (dir0 + (int)blockIdx.y == CDR_DIR_X)
 		line_factors<W64, W32, CDR_DIR_X>(so, ns, f.x, f.x32, d, tpitch, vecx, info);
 	else
@@ -160,9 +161,9 @@ int setup_lines_2d(const double *so, int nstencil, const LineFactors &f, Dims2 d
 	const int nl = !y ? d.ny : !x ? d.nx : d.nx > d.ny ? d.nx : d.ny;
 	const dim3 grd(ceil_div(nl, 32), x && y ? 2 : 1, d.nb);
 	const int dir0 = x ? CDR_DIR_X : CDR_DIR_Y;
-	if (w64 && w32) k_lines_setup<true, true><<<grd, 32, 0, st>>>(so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
-	else if (w64) k_lines_setup<true, false><<<grd, 32, 0, st>>>(so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
-	else k_lines_setup<false, true><<<grd, 32, 0, st>>>(so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
+	if (w64 && w32) launch(k_lines_setup<true, true>, grd, 32, 0, st, so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
+	else if (w64) launch(k_lines_setup<true, false>, grd, 32, 0, st, so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
+	else launch(k_lines_setup<false, true>, grd, 32, 0, st, so, nstencil, f, d, tpitch, dir0, vecx, vecy, info);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -195,6 +196,7 @@ template <typename T, int NS, int DIR, bool EXACT>
 __global__ void __launch_bounds__(LT) k_lines(const T *__restrict__ so, T *__restrict__ q, const T *__restrict__ qf,
                                               const T *__restrict__ sor, Dims2 d, int tpitch, int first, int G)
 {
+	await_previous();
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	T *sA = reinterpret_cast<T *>(smem_raw);
 	T *sB = sA + LT;
@@ -311,6 +313,7 @@ __global__ void __launch_bounds__(XL ? FAST_BLOCK_X : (LB ? LB : yblock_max<T>()
     k_lines_fast(const T *__restrict__ so, T *__restrict__ q, const T *__restrict__ qf, const T *__restrict__ sor,
                  Dims2 d, int tpitch, int first, int tpl_log2, int G, const T *__restrict__ yc)
 {
+	await_previous();
 	// group totals of the scans: lines * groups = blockDim / SG at most
 	__shared__ T sA[FAST_BLOCK_Y / SG], sB[FAST_BLOCK_Y / SG];
 	const int TPL = 1 << tpl_log2;
@@ -364,6 +367,7 @@ __global__ void __launch_bounds__(LB ? LB : yblock_max<T>(), LB ? 2 : 1)
                   Dims2 d, int tpitch, int c2, int tpl_log2, int G, unsigned *__restrict__ sync, int nvb,
                   const T *__restrict__ yc)
 {
+	await_previous();
 	__shared__ T sA[FAST_BLOCK_Y / SG], sB[FAST_BLOCK_Y / SG];
 	__shared__ int s_vb, s_ok;
 	const int TPL = 1 << tpl_log2;
@@ -476,6 +480,7 @@ __global__ void __launch_bounds__(XS_BLOCK, 2) k_lines_xstream(const T *__restri
                                                                const T *__restrict__ qf, const T *__restrict__ sor,
                                                                Dims2 d, int first, int nlines)
 {
+	await_previous();
 	extern __shared__ __align__(128) unsigned char xs_raw[];
 	__shared__ T sA[XS_BLOCK / SG], sB[XS_BLOCK / SG];  // group totals of the scans
 	constexpr int R = xs_rows<NS>();
@@ -796,10 +801,9 @@ static int launch_fast(const T *so, T *x, const T *b, const T *sor, Dims2 d, int
 		// packed couplings (zero-start sweeps read no couplings)
 		if (pack && !zero) {
 			if (ysmall && block <= YSMALL_BLOCK)
-				k_lines_fast<T, NS, DIR, K, ysmall ? YSMALL_BLOCK : 0, false, true><<<grd, block, 0, st>>>(
-				    so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
+				launch(k_lines_fast<T, NS, DIR, K, ysmall ? YSMALL_BLOCK : 0, false, true>, grd, block, 0, st, so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
 			else
-				k_lines_fast<T, NS, DIR, K, 0, false, true><<<grd, block, 0, st>>>(so, x, b, sor, d, tpitch, first,
+				launch(k_lines_fast<T, NS, DIR, K, 0, false, true>, grd, block, 0, st, so, x, b, sor, d, tpitch, first,
 				                                                                    tpl_log2, G, yc);
 			CDR_LAUNCH_CHECK();
 			return CDR_OK;
@@ -808,13 +812,13 @@ static int launch_fast(const T *so, T *x, const T *b, const T *sor, Dims2 d, int
 	if (ysmall && block <= YSMALL_BLOCK) {
 		constexpr int LB = ysmall ? YSMALL_BLOCK : 0;
 		if (zero)
-			k_lines_fast<T, NS, DIR, K, LB, true><<<grd, block, 0, st>>>(so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
+			launch(k_lines_fast<T, NS, DIR, K, LB, true>, grd, block, 0, st, so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
 		else
-			k_lines_fast<T, NS, DIR, K, LB><<<grd, block, 0, st>>>(so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
+			launch(k_lines_fast<T, NS, DIR, K, LB>, grd, block, 0, st, so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
 	} else if (zero) {
-		k_lines_fast<T, NS, DIR, K, 0, true><<<grd, block, 0, st>>>(so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
+		launch(k_lines_fast<T, NS, DIR, K, 0, true>, grd, block, 0, st, so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
 	} else {
-		k_lines_fast<T, NS, DIR, K><<<grd, block, 0, st>>>(so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
+		launch(k_lines_fast<T, NS, DIR, K>, grd, block, 0, st, so, x, b, sor, d, tpitch, first, tpl_log2, G, yc);
 	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -863,7 +867,7 @@ static int launch_xstream(const float *so, float *x, const float *b, const float
 		return CDR_ERR_CUDA;
 	}
 	const int grid = nlines < cap ? nlines : cap;
-	k_lines_xstream<float, NS, 8><<<grid, tpl, smem, st>>>(so, x, b, sor, d, first, nlines);
+	launch(k_lines_xstream<float, NS, 8>, grid, tpl, smem, st, so, x, b, sor, d, first, nlines);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -888,22 +892,22 @@ static int launch_ypair(const T *so, T *x, const T *b, const T *sor, Dims2 d, in
 	// zero start and packed couplings: the first colour reads b only, the second the packed couplings
 	if (small) {
 		if (zero && pack)
-			k_ylines_pair<T, NS, K, LB, true, true><<<nvb, block, 0, st>>>(so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
+			launch(k_ylines_pair<T, NS, K, LB, true, true>, nvb, block, 0, st, so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
 		else if (zero)
-			k_ylines_pair<T, NS, K, LB, true><<<nvb, block, 0, st>>>(so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
+			launch(k_ylines_pair<T, NS, K, LB, true>, nvb, block, 0, st, so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
 		else if (pack)
-			k_ylines_pair<T, NS, K, LB, false, true><<<nvb, block, 0, st>>>(so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
+			launch(k_ylines_pair<T, NS, K, LB, false, true>, nvb, block, 0, st, so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
 		else
-			k_ylines_pair<T, NS, K, LB><<<nvb, block, 0, st>>>(so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
+			launch(k_ylines_pair<T, NS, K, LB>, nvb, block, 0, st, so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
 	} else {
 		if (zero && pack)
-			k_ylines_pair<T, NS, K, 0, true, true><<<nvb, block, 0, st>>>(so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
+			launch(k_ylines_pair<T, NS, K, 0, true, true>, nvb, block, 0, st, so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
 		else if (zero)
-			k_ylines_pair<T, NS, K, 0, true><<<nvb, block, 0, st>>>(so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
+			launch(k_ylines_pair<T, NS, K, 0, true>, nvb, block, 0, st, so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
 		else if (pack)
-			k_ylines_pair<T, NS, K, 0, false, true><<<nvb, block, 0, st>>>(so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
+			launch(k_ylines_pair<T, NS, K, 0, false, true>, nvb, block, 0, st, so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
 		else
-			k_ylines_pair<T, NS, K><<<nvb, block, 0, st>>>(so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
+			launch(k_ylines_pair<T, NS, K>, nvb, block, 0, st, so, x, b, sor, d, tpitch, c2, tpl_log2, G, sync, nvb, yc);
 	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -960,8 +964,8 @@ static int launch_lines(const T *so, T *x, const T *b, const T *sor, Dims2 d, in
 	}
 	CDR_TRY(lines_prepare());
 	const dim3 grd(ceil_div(nlines, G), 1, d.nb);
-	if (exact) k_lines<T, NS, DIR, true><<<grd, LT, smem, st>>>(so, x, b, sor, d, tpitch, first, G);
-	else k_lines<T, NS, DIR, false><<<grd, LT, smem, st>>>(so, x, b, sor, d, tpitch, first, G);
+	if (exact) launch(k_lines<T, NS, DIR, true>, grd, LT, smem, st, so, x, b, sor, d, tpitch, first, G);
+	else launch(k_lines<T, NS, DIR, false>, grd, LT, smem, st, so, x, b, sor, d, tpitch, first, G);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -1177,6 +1181,7 @@ template int relax_lines_2d<float>(const float *, int, float *, const float *, c
 template <typename T, int NS>
 __global__ void k_pack_ylines(const T *__restrict__ so, T *__restrict__ yc, Dims2 d, int tpitch)
 {
+	await_previous();
 	const int j = blockIdx.x * blockDim.x + threadIdx.x + 1, i = blockIdx.y + 1;
 	if (j > d.ny || i > d.nx) return;
 	const size_t ps = d.plane(), fps = (size_t)tpitch * (d.nx + 2);
@@ -1204,8 +1209,8 @@ int pack_ylines_2d(const T *so, int nstencil, T *yc, Dims2 d, int tpitch, cudaSt
 		return CDR_ERR_DIM;
 	}
 	const dim3 g(ceil_div(d.ny, 256), d.nx, d.nb);
-	if (nstencil == 5) k_pack_ylines<T, 5><<<g, 256, 0, st>>>(so, yc, d, tpitch);
-	else k_pack_ylines<T, 3><<<g, 256, 0, st>>>(so, yc, d, tpitch);
+	if (nstencil == 5) launch(k_pack_ylines<T, 5>, g, 256, 0, st, so, yc, d, tpitch);
+	else launch(k_pack_ylines<T, 3>, g, 256, 0, st, so, yc, d, tpitch);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

@@ -31,6 +31,7 @@ namespace cdrgpu {
 template <typename T>
 __global__ void k_ghost(T *__restrict__ q, Dims2 d, int planes, int xmode, int ymode, int jpar)
 {
+	await_previous();
 	const int nxg = d.nx + 2, nrow = 2 * nxg;
 	int t = blockIdx.x * blockDim.x + threadIdx.x, i, j;
 	if (t < nrow) {
@@ -63,7 +64,7 @@ int ghost_copy_2d(T *q, Dims2 d, int planes, int xmode, int ymode, int jpar, cud
 		return CDR_ERR_ARG;
 	}
 	const int n = 2 * (d.nx + 2) + 2 * d.ny;
-	k_ghost<T><<<ceil_div(n, 256), 256, 0, st>>>(q, d, planes, xmode, ymode, jpar);
+	launch(k_ghost<T>, ceil_div(n, 256), 256, 0, st, q, d, planes, xmode, ymode, jpar);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -195,6 +196,7 @@ __device__ void oi_yedge(const OISten<NS> &SO, double *ci, size_t cps, const Dim
 template <int NS>
 __global__ void k_oi_per_edges(const double *__restrict__ so, double *__restrict__ ci, Dims2 f, Dims2 c, PerOI g)
 {
+	await_previous();
 	const int IC = blockIdx.x * TX + threadIdx.x + 1, JC = blockIdx.y * TY + threadIdx.y + 1;
 	if (IC > g.IIC || JC > g.JJC) return;
 	const OISten<NS> SO{so, f.plane(), f.pitch};
@@ -219,6 +221,7 @@ __global__ void k_oi_per_edges(const double *__restrict__ so, double *__restrict
 template <int NS>
 __global__ void k_oi_per_corners(const double *__restrict__ so, double *__restrict__ ci, Dims2 f, Dims2 c, PerOI g)
 {
+	await_previous();
 	const int IC = blockIdx.x * TX + threadIdx.x + g.IBEGC, JC = blockIdx.y * TY + threadIdx.y + g.JBEGC;
 	if (IC > g.IENDC || JC > g.JENDC) return;
 	const OISten<NS> SO{so, f.plane(), f.pitch};
@@ -276,13 +279,13 @@ int setup_interp_per_2d(const double *so, int nstencil, double *ci, Dims2 f, Dim
 	dim3 g1(ceil_div(g.IIC, TX), ceil_div(g.JJC, TY));
 	dim3 g2(ceil_div(g.IENDC - g.IBEGC + 1, TX), ceil_div(g.JENDC - g.JBEGC + 1, TY));
 	if (nstencil == 5) {
-		k_oi_per_edges<5><<<g1, blk, 0, st>>>(so, ci, f, c, g);
+		launch(k_oi_per_edges<5>, g1, blk, 0, st, so, ci, f, c, g);
 		CDR_LAUNCH_CHECK();
-		k_oi_per_corners<5><<<g2, blk, 0, st>>>(so, ci, f, c, g);
+		launch(k_oi_per_corners<5>, g2, blk, 0, st, so, ci, f, c, g);
 	} else {
-		k_oi_per_edges<3><<<g1, blk, 0, st>>>(so, ci, f, c, g);
+		launch(k_oi_per_edges<3>, g1, blk, 0, st, so, ci, f, c, g);
 		CDR_LAUNCH_CHECK();
-		k_oi_per_corners<3><<<g2, blk, 0, st>>>(so, ci, f, c, g);
+		launch(k_oi_per_corners<3>, g2, blk, 0, st, so, ci, f, c, g);
 	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -294,6 +297,7 @@ int setup_interp_per_2d(const double *so, int nstencil, double *ci, Dims2 f, Dim
 // assembly of BMG2_SymStd_SETUP_cg_LU's periodic branches, one thread.
 __global__ void k_cg_per_assemble(const double *__restrict__ so, int ns, Dims2 d, double *__restrict__ abd, int per)
 {
+	await_previous();
 	if (threadIdx.x != 0 || blockIdx.x != 0) return;
 	const int II = d.nx + 2, JJ = d.ny + 2, I1 = II - 1, J1 = JJ - 1, I2 = I1 - 1, N = I2 * (J1 - 1);
 	const bool perx = per & 1, pery = (per >> 1) & 1, nine = ns == 5;
@@ -351,6 +355,7 @@ __global__ void k_cg_per_assemble(const double *__restrict__ so, int ns, Dims2 d
 // Every entry sees the serial routine's operations in its order.
 __global__ void __launch_bounds__(1024) k_cg_per_factor(double *__restrict__ a, int n, int *info)
 {
+	await_previous();
 	__shared__ double rcp_s;
 	__shared__ int stop_s;
 	const int tid = threadIdx.x, nt = blockDim.x;
@@ -388,9 +393,9 @@ int setup_cg_per_2d(const double *so, int nstencil, Dims2 d, double *abd, int *i
 {
 	const size_t n = (size_t)d.nx * d.ny;
 	CDR_CUDA_TRY(cudaMemsetAsync(abd, 0, sizeof(double) * n * n, st));
-	k_cg_per_assemble<<<1, 1, 0, st>>>(so, nstencil, d, abd, per);
+	launch(k_cg_per_assemble, 1, 1, 0, st, so, nstencil, d, abd, per);
 	CDR_LAUNCH_CHECK();
-	k_cg_per_factor<<<1, 1024, 0, st>>>(abd, (int)n, info);
+	launch(k_cg_per_factor, 1, 1024, 0, st, abd, (int)n, info);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -404,6 +409,7 @@ int setup_cg_per_2d(const double *so, int nstencil, Dims2 d, double *abd, int *i
 __global__ void __launch_bounds__(1024) k_cg_per_solve(const double *__restrict__ a, double *__restrict__ q,
                                                        const double *__restrict__ qf, Dims2 d, int per)
 {
+	await_previous();
 	extern __shared__ double bb[];
 	__shared__ double shift_s;
 	__shared__ int nz_s;
@@ -468,7 +474,7 @@ int solve_cg_per_2d(const double *abd, double *x, const double *b, Dims2 d, int 
 		set_error(CDR_ERR_DIM, "coarsest grid %dx%d too large for the dense periodic solve", d.nx, d.ny);
 		return CDR_ERR_DIM;
 	}
-	k_cg_per_solve<<<1, 1024, sm, st>>>(abd, x, b, d, per);
+	launch(k_cg_per_solve, 1, 1024, sm, st, abd, x, b, d, per);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(TX *TY) k_residual(const T *__restrict__ so, c
                                                      const T *__restrict__ qf, T *__restrict__ res, Dims2 d,
                                                      double *__restrict__ partial)
 {
+	await_previous();
 	__shared__ double sh[TX * TY / 32];
 	const int tiles_x = (d.nx + TX - 1) / TX;
 	const int ntiles = tiles_x * ((d.ny + TY - 1) / TY);
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(TX *TY) k_residual_v(const T *__restrict__ so,
                                                        const T *__restrict__ qf, T *__restrict__ res, Dims2 d,
                                                        double *__restrict__ partial)
 {
+	await_previous();
 	constexpr int V = 16 / sizeof(T);
 	using VT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
 	__shared__ double sh[TX * TY / 32];
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(TX *TY) k_residual_v(const T *__restrict__ so,
 // one block per problem: out[b] = sqrt(sum of partial[b*n .. b*n+n))
 __global__ void __launch_bounds__(1024) k_norm_finish(const double *__restrict__ partial, int n, double *out)
 {
+	await_previous();
 	__shared__ double sh[32];
 	partial += (size_t)blockIdx.x * n;
 	out += blockIdx.x;
@@ -192,26 +195,26 @@ int residual_2d(const T *so, int nstencil, const T *x, const T *b, T *r, Dims2 d
 		if (norm_out) {
 			int nb = norm_blocks(d);
 			nb = nb < tx * ty ? nb : tx * ty;
-			if (nstencil == 5) k_residual_v<T, 5, true><<<dim3(nb, 1, d.nb), blk, 0, st>>>(so, x, b, r, d, partial);
-			else k_residual_v<T, 3, true><<<dim3(nb, 1, d.nb), blk, 0, st>>>(so, x, b, r, d, partial);
+			if (nstencil == 5) launch(k_residual_v<T, 5, true>, dim3(nb, 1, d.nb), blk, 0, st, so, x, b, r, d, partial);
+			else launch(k_residual_v<T, 3, true>, dim3(nb, 1, d.nb), blk, 0, st, so, x, b, r, d, partial);
 			CDR_LAUNCH_CHECK();
-			k_norm_finish<<<d.nb, 1024, 0, st>>>(partial, nb, norm_out);
+			launch(k_norm_finish, d.nb, 1024, 0, st, partial, nb, norm_out);
 		} else {
-			if (nstencil == 5) k_residual_v<T, 5, false><<<dim3(tx, ty, d.nb), blk, 0, st>>>(so, x, b, r, d, nullptr);
-			else k_residual_v<T, 3, false><<<dim3(tx, ty, d.nb), blk, 0, st>>>(so, x, b, r, d, nullptr);
+			if (nstencil == 5) launch(k_residual_v<T, 5, false>, dim3(tx, ty, d.nb), blk, 0, st, so, x, b, r, d, nullptr);
+			else launch(k_residual_v<T, 3, false>, dim3(tx, ty, d.nb), blk, 0, st, so, x, b, r, d, nullptr);
 		}
 		CDR_LAUNCH_CHECK();
 		return CDR_OK;
 	}
 	if (norm_out) {
 		int nb = norm_blocks(d);
-		if (nstencil == 5) k_residual<T, 5, true><<<dim3(nb, 1, d.nb), blk, 0, st>>>(so, x, b, r, d, partial);
-		else k_residual<T, 3, true><<<dim3(nb, 1, d.nb), blk, 0, st>>>(so, x, b, r, d, partial);
+		if (nstencil == 5) launch(k_residual<T, 5, true>, dim3(nb, 1, d.nb), blk, 0, st, so, x, b, r, d, partial);
+		else launch(k_residual<T, 3, true>, dim3(nb, 1, d.nb), blk, 0, st, so, x, b, r, d, partial);
 		CDR_LAUNCH_CHECK();
-		k_norm_finish<<<d.nb, 1024, 0, st>>>(partial, nb, norm_out);
+		launch(k_norm_finish, d.nb, 1024, 0, st, partial, nb, norm_out);
 	} else {
-		if (nstencil == 5) k_residual<T, 5, false><<<dim3(ntiles, 1, d.nb), blk, 0, st>>>(so, x, b, r, d, nullptr);
-		else k_residual<T, 3, false><<<dim3(ntiles, 1, d.nb), blk, 0, st>>>(so, x, b, r, d, nullptr);
+		if (nstencil == 5) launch(k_residual<T, 5, false>, dim3(ntiles, 1, d.nb), blk, 0, st, so, x, b, r, d, nullptr);
+		else launch(k_residual<T, 3, false>, dim3(ntiles, 1, d.nb), blk, 0, st, so, x, b, r, d, nullptr);
 	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -227,6 +230,7 @@ template int residual_2d<float>(const float *, int, const float *, const float *
 template <typename T>
 __global__ void k_recip(const T *__restrict__ so, int ns, T *__restrict__ sor, Dims2 d)
 {
+	await_previous();
 	so += d.bofs(ns * d.plane());
 	sor += d.bofs(2 * d.plane());
 	int i = blockIdx.x * TX + threadIdx.x + 1, j = blockIdx.y * TY + threadIdx.y + 1;
@@ -236,7 +240,7 @@ __global__ void k_recip(const T *__restrict__ so, int ns, T *__restrict__ sor, D
 template <typename T>
 int setup_recip_2d(const T *so, T *sor, Dims2 d, cudaStream_t st, int ns)
 {
-	k_recip<T><<<dim3(ceil_div(d.nx, TX), ceil_div(d.ny, TY), d.nb), dim3(TX, TY), 0, st>>>(so, ns, sor, d);
+	launch(k_recip<T>, dim3(ceil_div(d.nx, TX), ceil_div(d.ny, TY), d.nb), dim3(TX, TY), 0, st, so, ns, sor, d);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -252,6 +256,7 @@ __global__ void __launch_bounds__(TX *TY) k_gs_colour(const T *__restrict__ so, 
                                                       const T *__restrict__ qf, const T *__restrict__ sor,
                                                       Dims2 d, int pi, int pj)
 {
+	await_previous();
 	const size_t ps = d.plane();
 	const int pitch = d.pitch;
 	so += d.bofs(NS * ps);
@@ -290,7 +295,7 @@ int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Di
 		dim3 grd(ceil_div((d.nx + 1) / 2, TX), ceil_div((d.ny + 1) / 2, TY), d.nb);
 		for (int c = 0; c < 4; ++c) {
 			int o = updown == CDR_DOWN ? c : 3 - c;
-			k_gs_colour<T, 5><<<grd, blk, 0, st>>>(so, x, b, sor, d, order[o][1], order[o][0]);
+			launch(k_gs_colour<T, 5>, grd, blk, 0, st, so, x, b, sor, d, order[o][1], order[o][0]);
 			CDR_LAUNCH_CHECK();
 			if (perx) CDR_TRY(ghost_copy_2d<T>(x, d, 1, 1, 0, order[o][0], st));
 		}
@@ -300,7 +305,7 @@ int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Di
 		dim3 grd(ceil_div((d.nx + 1) / 2, TX), ceil_div(d.ny, TY), d.nb);
 		for (int c = 0; c < 2; ++c) {
 			int par = updown == CDR_DOWN ? c : 1 - c;
-			k_gs_colour<T, 3><<<grd, blk, 0, st>>>(so, x, b, sor, d, par, 0);
+			launch(k_gs_colour<T, 3>, grd, blk, 0, st, so, x, b, sor, d, par, 0);
 			CDR_LAUNCH_CHECK();
 			if (perx) CDR_TRY(ghost_copy_2d<T>(x, d, 1, 1, 0, -1, st));
 		}
@@ -320,6 +325,7 @@ template <typename T, typename TC = T>
 __global__ void __launch_bounds__(TX *TY) k_restrict(const TC *__restrict__ ci, const T *__restrict__ q,
                                                      TC *__restrict__ qc, Dims2 f, Dims2 c)
 {
+	await_previous();
 	int ic = blockIdx.x * TX + threadIdx.x + 1, jc = blockIdx.y * TY + threadIdx.y + 1;
 	if (ic > c.nx || jc > c.ny) return;
 	const size_t cps = c.plane();
@@ -332,7 +338,7 @@ __global__ void __launch_bounds__(TX *TY) k_restrict(const TC *__restrict__ ci, 
 template <typename T>
 int restrict_2d(const T *ci, const T *rf, T *bc, Dims2 f, Dims2 c, cudaStream_t st)
 {
-	k_restrict<T><<<dim3(ceil_div(c.nx, TX), ceil_div(c.ny, TY), c.nb), dim3(TX, TY), 0, st>>>(ci, rf, bc, f, c);
+	launch(k_restrict<T>, dim3(ceil_div(c.nx, TX), ceil_div(c.ny, TY), c.nb), dim3(TX, TY), 0, st, ci, rf, bc, f, c);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -341,7 +347,7 @@ template int restrict_2d<float>(const float *, const float *, float *, Dims2, Di
 
 int restrict_2d_mixed(const double *ci, const float *rf, double *bc, Dims2 f, Dims2 c, cudaStream_t st)
 {
-	k_restrict<float, double><<<dim3(ceil_div(c.nx, TX), ceil_div(c.ny, TY), c.nb), dim3(TX, TY), 0, st>>>(ci, rf, bc,
+	launch(k_restrict<float, double>, dim3(ceil_div(c.nx, TX), ceil_div(c.ny, TY), c.nb), dim3(TX, TY), 0, st, ci, rf, bc,
 	                                                                                                     f, c);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -357,6 +363,7 @@ __global__ void __launch_bounds__(TX *TY) k_interp_add(const TC *__restrict__ ci
                                                        const T *__restrict__ res, const T *__restrict__ soc,
                                                        T *__restrict__ q, Dims2 f, Dims2 c, int nsf)
 {
+	await_previous();
 	int ic = blockIdx.x * TX + threadIdx.x + 1, jc = blockIdx.y * TY + threadIdx.y + 1;
 	if (ic > f.nx / 2 + 1 || jc > f.ny / 2 + 1) return;
 	const size_t cps = c.plane();
@@ -372,8 +379,7 @@ template <typename T>
 int interp_add_2d(const T *ci, const T *xc, const T *rf, const T *sof, T *xf, Dims2 f, Dims2 c, cudaStream_t st,
                   int nsf)
 {
-	k_interp_add<T><<<dim3(ceil_div(f.nx / 2 + 1, TX), ceil_div(f.ny / 2 + 1, TY), f.nb), dim3(TX, TY), 0, st>>>(
-	    ci, xc, rf, sof, xf, f, c, nsf);
+	launch(k_interp_add<T>, dim3(ceil_div(f.nx / 2 + 1, TX), ceil_div(f.ny / 2 + 1, TY), f.nb), dim3(TX, TY), 0, st, ci, xc, rf, sof, xf, f, c, nsf);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -385,8 +391,8 @@ template int interp_add_2d<float>(const float *, const float *, const float *, c
 int interp_add_2d_mixed(const double *ci, const double *xc, const float *rf, const float *sof, float *xf, Dims2 f,
                         Dims2 c, cudaStream_t st, int nsf)
 {
-	k_interp_add<float, double><<<dim3(ceil_div(f.nx / 2 + 1, TX), ceil_div(f.ny / 2 + 1, TY), f.nb), dim3(TX, TY), 0,
-	                              st>>>(ci, xc, rf, sof, xf, f, c, nsf);
+	launch(k_interp_add<float, double>, dim3(ceil_div(f.nx / 2 + 1, TX), ceil_div(f.ny / 2 + 1, TY), f.nb), dim3(TX, TY), 0,
+	                              st, ci, xc, rf, sof, xf, f, c, nsf);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -401,6 +407,7 @@ __global__ void __launch_bounds__(TX *TY) k_interp_add_wide(const float *__restr
                                                             const float *__restrict__ qin, double *__restrict__ qout,
                                                             Dims2 f, Dims2 c, int nsf)
 {
+	await_previous();
 	const int ic = blockIdx.x * TX + threadIdx.x + 1, jc = blockIdx.y * TY + threadIdx.y + 1;
 	if (ic > f.nx / 2 + 1 || jc > f.ny / 2 + 1) return;
 	const size_t cps = c.plane();
@@ -452,6 +459,7 @@ __global__ void __launch_bounds__(256) k_interp_add_wide_rows(const float *__res
                                                              const float *__restrict__ qin,
                                                              double *__restrict__ qout, Dims2 f, Dims2 c)
 {
+	await_previous();
 	const int ic = blockIdx.x * blockDim.x + threadIdx.x + 1, jf = blockIdx.y + 1;
 	if (ic > f.nx / 2 + 1) return;
 	const size_t cps = c.plane();
@@ -496,6 +504,7 @@ __global__ void __launch_bounds__(256) k_interp_add_wide_rows(const float *__res
 // rounded once.
 __global__ void k_rowsum_excess(const double *__restrict__ so, int ns, float *__restrict__ dg, Dims2 d)
 {
+	await_previous();
 	const size_t ps = d.plane();
 	const int P = d.pitch;
 	const int i = blockIdx.x * TX + threadIdx.x + 1, j = blockIdx.y * TY + threadIdx.y + 1;
@@ -512,7 +521,7 @@ __global__ void k_rowsum_excess(const double *__restrict__ so, int ns, float *__
 
 int rowsum_excess_2d(const double *so, int ns, float *dg, Dims2 d, cudaStream_t st)
 {
-	k_rowsum_excess<<<dim3(ceil_div(d.nx, TX), ceil_div(d.ny, TY)), dim3(TX, TY), 0, st>>>(so, ns, dg, d);
+	launch(k_rowsum_excess, dim3(ceil_div(d.nx, TX), ceil_div(d.ny, TY)), dim3(TX, TY), 0, st, so, ns, dg, d);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -531,6 +540,7 @@ __global__ void __launch_bounds__(TX *TY) k_residual_wide(const float *__restric
                                                           const double *__restrict__ q, const float *__restrict__ qf,
                                                           float *__restrict__ res, float *__restrict__ zero, Dims2 d)
 {
+	await_previous();
 	constexpr int V = 4;
 	const size_t ps = d.plane();
 	const int P = d.pitch;
@@ -609,8 +619,8 @@ int residual_2d_wide(const float *so, const float *dg, int ns, const double *x, 
 		return CDR_ERR_ARG;
 	}
 	const dim3 g(ceil_div(d.nx + 1, TX * 4), ceil_div(d.ny, TY)), blk(TX, TY);
-	if (ns == 5) k_residual_wide<5><<<g, blk, 0, st>>>(so, dg, x, b, r, zero, d);
-	else k_residual_wide<3><<<g, blk, 0, st>>>(so, dg, x, b, r, zero, d);
+	if (ns == 5) launch(k_residual_wide<5>, g, blk, 0, st, so, dg, x, b, r, zero, d);
+	else launch(k_residual_wide<3>, g, blk, 0, st, so, dg, x, b, r, zero, d);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -621,11 +631,10 @@ int interp_add_2d_wide(const float *ci, const float *xc, const float *rf, const 
 	// rows of 16-byte alignment, a single problem: the row kernel; otherwise by
 	// 2 x 2 blocks of fine points
 	if (f.nb == 1 && f.pitch % 4 == 0 && ((uintptr_t)xin | (uintptr_t)xout) % 16 == 0) {
-		k_interp_add_wide_rows<<<dim3(ceil_div(f.nx / 2 + 1, 256), 2 * (f.ny / 2) + 1), 256, 0, st>>>(
-		    ci, xc, rf, sof, xin, xout, f, c);
+		launch(k_interp_add_wide_rows, dim3(ceil_div(f.nx / 2 + 1, 256), 2 * (f.ny / 2) + 1), 256, 0, st, ci, xc, rf, sof, xin, xout, f, c);
 	} else {
-		k_interp_add_wide<<<dim3(ceil_div(f.nx / 2 + 1, TX), ceil_div(f.ny / 2 + 1, TY), f.nb), dim3(TX, TY), 0,
-		                    st>>>(ci, xc, rf, sof, xin, xout, f, c, nsf);
+		launch(k_interp_add_wide, dim3(ceil_div(f.nx / 2 + 1, TX), ceil_div(f.ny / 2 + 1, TY), f.nb), dim3(TX, TY), 0,
+		                    st, ci, xc, rf, sof, xin, xout, f, c, nsf);
 	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -639,6 +648,7 @@ int interp_add_2d_wide(const float *ci, const float *xc, const float *rf, const 
 template <int NS>
 __global__ void k_oi_edges(const double *__restrict__ so, double *__restrict__ ci, Dims2 f, Dims2 c)
 {
+	await_previous();
 	int ic = blockIdx.x * TX + threadIdx.x + 1, jc = blockIdx.y * TY + threadIdx.y + 1;
 	const size_t ps = f.plane(), cps = c.plane();
 	const int fp = f.pitch;
@@ -689,6 +699,7 @@ __global__ void k_oi_edges(const double *__restrict__ so, double *__restrict__ c
 template <int NS>
 __global__ void k_oi_corners(const double *__restrict__ so, double *__restrict__ ci, Dims2 f, Dims2 c)
 {
+	await_previous();
 	int ic = blockIdx.x * TX + threadIdx.x + 2, jc = blockIdx.y * TY + threadIdx.y + 2;
 	if (ic > f.nx / 2 + 1 || jc > f.ny / 2 + 1) return;
 	const size_t ps = f.plane(), cps = c.plane();
@@ -734,13 +745,13 @@ int setup_interp_2d(const double *so, int nstencil, double *ci, Dims2 f, Dims2 c
 	dim3 g1(ceil_div(c.nx + 1, TX), ceil_div(c.ny + 1, TY), c.nb);
 	dim3 g2(ceil_div(f.nx / 2, TX), ceil_div(f.ny / 2, TY), c.nb);
 	if (nstencil == 5) {
-		k_oi_edges<5><<<g1, blk, 0, st>>>(so, ci, f, c);
+		launch(k_oi_edges<5>, g1, blk, 0, st, so, ci, f, c);
 		CDR_LAUNCH_CHECK();
-		k_oi_corners<5><<<g2, blk, 0, st>>>(so, ci, f, c);
+		launch(k_oi_corners<5>, g2, blk, 0, st, so, ci, f, c);
 	} else {
-		k_oi_edges<3><<<g1, blk, 0, st>>>(so, ci, f, c);
+		launch(k_oi_edges<3>, g1, blk, 0, st, so, ci, f, c);
 		CDR_LAUNCH_CHECK();
-		k_oi_corners<3><<<g2, blk, 0, st>>>(so, ci, f, c);
+		launch(k_oi_corners<3>, g2, blk, 0, st, so, ci, f, c);
 	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -758,6 +769,7 @@ template <int NS>
 __global__ void k_galerkin(const double *__restrict__ so, const double *__restrict__ ci, double *__restrict__ soc,
                            Dims2 f, Dims2 c)
 {
+	await_previous();
 	const int ic = blockIdx.x * TX + threadIdx.x + 1, jc = blockIdx.y * TY + threadIdx.y + 1;
 	if (ic > c.nx || jc > c.ny) return;
 	const size_t ps = f.plane(), cps = c.plane();
@@ -861,8 +873,8 @@ int galerkin_2d(const double *so, int nstencil, const double *ci, double *soc, D
 {
 	CDR_CUDA_TRY(cudaMemsetAsync(soc, 0, sizeof(double) * c.plane() * 5 * c.nb, st));
 	dim3 g(ceil_div(c.nx, TX), ceil_div(c.ny, TY), c.nb);
-	if (nstencil == 5) k_galerkin<5><<<g, dim3(TX, TY), 0, st>>>(so, ci, soc, f, c);
-	else k_galerkin<3><<<g, dim3(TX, TY), 0, st>>>(so, ci, soc, f, c);
+	if (nstencil == 5) launch(k_galerkin<5>, g, dim3(TX, TY), 0, st, so, ci, soc, f, c);
+	else launch(k_galerkin<3>, g, dim3(TX, TY), 0, st, so, ci, soc, f, c);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -874,6 +886,7 @@ int galerkin_2d(const double *so, int nstencil, const double *ci, double *soc, D
 __global__ void __launch_bounds__(1024) k_cg_factor(const double *__restrict__ so, int ns, Dims2 d,
                                                     double *__restrict__ ab, int *info)
 {
+	await_previous();
 	__shared__ double rcp_s;
 	__shared__ int stop_s;
 	const int tid = threadIdx.x, nt = blockDim.x;
@@ -938,6 +951,7 @@ __global__ void __launch_bounds__(1024) k_cg_factor(const double *__restrict__ s
 template <typename T>
 __global__ void k_cg_solve(const double *__restrict__ ab, T *__restrict__ q, const T *__restrict__ qf, Dims2 d)
 {
+	await_previous();
 	extern __shared__ double xs[];
 	const int ldab = d.nx + 2, n = d.nx * d.ny, lane = threadIdx.x;
 	ab += d.bofs((size_t)ldab * n);
@@ -951,7 +965,7 @@ __global__ void k_cg_solve(const double *__restrict__ ab, T *__restrict__ q, con
 
 int setup_cg_2d(const double *so, int nstencil, Dims2 d, double *abd, int *info, cudaStream_t st)
 {
-	k_cg_factor<<<dim3(1, 1, d.nb), 1024, 0, st>>>(so, nstencil, d, abd, info);
+	launch(k_cg_factor, dim3(1, 1, d.nb), 1024, 0, st, so, nstencil, d, abd, info);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -964,7 +978,7 @@ int solve_cg_2d(const double *abd, T *x, const T *b, Dims2 d, cudaStream_t st)
 		set_error(CDR_ERR_DIM, "coarsest grid %dx%d too large for the direct solve", d.nx, d.ny);
 		return CDR_ERR_DIM;
 	}
-	k_cg_solve<T><<<dim3(1, 1, d.nb), 32, sm, st>>>(abd, x, b, d);
+	launch(k_cg_solve<T>, dim3(1, 1, d.nb), 32, sm, st, abd, x, b, d);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -975,6 +989,7 @@ template int solve_cg_2d<float>(const double *, float *, const float *, Dims2, c
 template <typename TO, typename TI>
 __global__ void k_convert(const TI *__restrict__ in, TO *__restrict__ out, size_t n)
 {
+	await_previous();
 	for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
 		out[e] = (TO)in[e];
 }
@@ -984,7 +999,7 @@ int convert_f64_f32(const double *in, float *out, size_t n, cudaStream_t st)
 	int nb = (int)((n + 255) / 256);
 	if (nb > 148 * 16) nb = 148 * 16;
 	if (nb < 1) nb = 1;
-	k_convert<float, double><<<nb, 256, 0, st>>>(in, out, n);
+	launch(k_convert<float, double>, nb, 256, 0, st, in, out, n);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -1003,6 +1018,7 @@ __global__ void __launch_bounds__(TX *TY) k_ir_residual(const double *__restrict
                                                         Dims2 d32, double *__restrict__ partial, int apply,
                                                         const int *__restrict__ active)
 {
+	await_previous();
 	__shared__ double sh[TX * TY / 32];
 	const int tiles_x = (d.nx + TX - 1) / TX;
 	const int ntiles = tiles_x * ((d.ny + TY - 1) / TY);
@@ -1060,6 +1076,7 @@ __global__ void __launch_bounds__(TX *TY) k_ir_residual_v(const double *__restri
                                                           Dims2 d32, double *__restrict__ partial, int apply,
                                                           const int *__restrict__ active)
 {
+	await_previous();
 	__shared__ double sh[TX * TY / 32];
 	const int tiles_x = (d.nx + 2 * TX) / (2 * TX);  // pairs (0,1), (2,3), ... up to nx
 	const int ntiles = tiles_x * ((d.ny + TY - 1) / TY);
@@ -1145,15 +1162,15 @@ int ir_residual_2d(const double *so, int nstencil, const double *x, const float 
 	                 ((uintptr_t)so | (uintptr_t)x | (uintptr_t)b | (uintptr_t)xo) % 16 == 0 &&
 	                 ((uintptr_t)e | (uintptr_t)r32) % 8 == 0;
 	if (vec && nstencil == 5)
-		k_ir_residual_v<5><<<grd, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply, active);
+		launch(k_ir_residual_v<5>, grd, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, d32, partial, apply, active);
 	else if (vec)
-		k_ir_residual_v<3><<<grd, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply, active);
+		launch(k_ir_residual_v<3>, grd, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, d32, partial, apply, active);
 	else if (nstencil == 5)
-		k_ir_residual<5><<<grd, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply, active);
+		launch(k_ir_residual<5>, grd, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, d32, partial, apply, active);
 	else
-		k_ir_residual<3><<<grd, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply, active);
+		launch(k_ir_residual<3>, grd, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, d32, partial, apply, active);
 	CDR_LAUNCH_CHECK();
-	k_norm_finish<<<d.nb, 1024, 0, st>>>(partial, nb, norm_out);
+	launch(k_norm_finish, d.nb, 1024, 0, st, partial, nb, norm_out);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(TX *TY) k3_residual(const T *__restrict__ so, 
                                                       const T *__restrict__ qf, TO *__restrict__ res, Dims3 F,
                                                       double *__restrict__ partial)
 {
+	await_previous();
 	__shared__ double sh[TX * TY / 32];
 	const int tx = (F.nx + TX - 1) / TX, ty = (F.ny + TY - 1) / TY;
 	const long ntiles = (long)tx * ty * F.nz;
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(TX *TY) k3_residual(const T *__restrict__ so, 
 
 __global__ void __launch_bounds__(1024) k3_norm_finish(const double *__restrict__ partial, int n, double *out)
 {
+	await_previous();
 	__shared__ double sh[32];
 	double v = 0;
 	for (int i = threadIdx.x; i < n; i += blockDim.x) v += partial[i];
@@ -131,6 +133,7 @@ __global__ void __launch_bounds__(1024) k3_norm_finish(const double *__restrict_
 template <typename T>
 __global__ void k3_recip(const T *__restrict__ so, T *__restrict__ sor, Dims3 F)
 {
+	await_previous();
 	const int i = blockIdx.x * TX + threadIdx.x + 2, j = blockIdx.y * TY + threadIdx.y + 2, k = blockIdx.z + 2;
 	if (i > F.nx + 1 || j > F.ny + 1) return;
 	sor[F.at1(i, j, k)] = T(1) / SO(i, j, k, KP);
@@ -297,6 +300,7 @@ __global__ void __launch_bounds__(256) k3_gs_rows(const T *__restrict__ so, T *_
                                                   const T *__restrict__ qf, const T *__restrict__ sor, Dims3 F, int pj,
                                                   int pk, int nrj, int nrows, int W)
 {
+	await_previous();
 	__shared__ T sh[256];    // first-colour values of the segment
 	__shared__ T edge[256];  // per row: the first-colour value the next segment reads
 	const int r = threadIdx.x / W, t0 = threadIdx.x - r * W;
@@ -415,6 +419,7 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)
     k3_gs_staged(const T *__restrict__ so, T *__restrict__ q, const T *__restrict__ qf, const T *__restrict__ sor,
                  Dims3 F, int pj, int pk, int nrj)
 {
+	await_previous();
 	extern __shared__ __align__(16) unsigned char k3_raw[];
 	T *rows = reinterpret_cast<T *>(k3_raw);
 	const int nch = staged_chunks<T>(F), rl = nch * (16 / (int)sizeof(T)), t = threadIdx.x;
@@ -529,6 +534,7 @@ __global__ void __launch_bounds__(512, 2)
     k3_residual_staged(const T *__restrict__ so, const T *__restrict__ q, const T *__restrict__ qf, T *__restrict__ res,
                        Dims3 F, double *__restrict__ partial)
 {
+	await_previous();
 	extern __shared__ __align__(16) unsigned char k3_raw[];
 	__shared__ double sh[16];
 	T *rows = reinterpret_cast<T *>(k3_raw);
@@ -601,11 +607,11 @@ int residual_3d(const T *so, const T *x, const T *b, T *r, Dims3 F, double *norm
 			const int nrows = F.ny * F.nz, blk = staged_block(F), nb = norm_out && nrows > 2048 ? 2048 : nrows;
 			CDR_TRY(staged_opt_in(norm_out ? (const void *)k3_residual_staged<T, true>
 			                               : (const void *)k3_residual_staged<T, false>, smem));
-			if (norm_out) k3_residual_staged<T, true><<<nb, blk, smem, st>>>(so, x, b, r, F, partial);
-			else k3_residual_staged<T, false><<<nb, blk, smem, st>>>(so, x, b, r, F, nullptr);
+			if (norm_out) launch(k3_residual_staged<T, true>, nb, blk, smem, st, so, x, b, r, F, partial);
+			else launch(k3_residual_staged<T, false>, nb, blk, smem, st, so, x, b, r, F, nullptr);
 			CDR_LAUNCH_CHECK();
 			if (norm_out) {
-				k3_norm_finish<<<1, 1024, 0, st>>>(partial, nb, norm_out);
+				launch(k3_norm_finish, 1, 1024, 0, st, partial, nb, norm_out);
 				CDR_LAUNCH_CHECK();
 			}
 			return CDR_OK;
@@ -613,14 +619,14 @@ int residual_3d(const T *so, const T *x, const T *b, T *r, Dims3 F, double *norm
 	const long ntiles = (long)ceil_div(F.nx, TX) * ceil_div(F.ny, TY) * F.nz;
 	const int nb = ntiles < 2048 ? (int)ntiles : 2048;
 	if (norm_out) {
-		if (ns == 4) k3_residual<T, true, 4><<<nb, dim3(TX, TY), 0, st>>>(so, x, b, r, F, partial);
-		else k3_residual<T, true, 14><<<nb, dim3(TX, TY), 0, st>>>(so, x, b, r, F, partial);
+		if (ns == 4) launch(k3_residual<T, true, 4>, nb, dim3(TX, TY), 0, st, so, x, b, r, F, partial);
+		else launch(k3_residual<T, true, 14>, nb, dim3(TX, TY), 0, st, so, x, b, r, F, partial);
 		CDR_LAUNCH_CHECK();
-		k3_norm_finish<<<1, 1024, 0, st>>>(partial, nb, norm_out);
+		launch(k3_norm_finish, 1, 1024, 0, st, partial, nb, norm_out);
 	} else {
 		const int nb2 = ntiles < 148 * 64 ? (int)ntiles : 148 * 64;
-		if (ns == 4) k3_residual<T, false, 4><<<nb2, dim3(TX, TY), 0, st>>>(so, x, b, r, F, nullptr);
-		else k3_residual<T, false, 14><<<nb2, dim3(TX, TY), 0, st>>>(so, x, b, r, F, nullptr);
+		if (ns == 4) launch(k3_residual<T, false, 4>, nb2, dim3(TX, TY), 0, st, so, x, b, r, F, nullptr);
+		else launch(k3_residual<T, false, 14>, nb2, dim3(TX, TY), 0, st, so, x, b, r, F, nullptr);
 	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -638,6 +644,7 @@ __global__ void __launch_bounds__(TX *TY) k3_gs7_colour(const T *__restrict__ so
                                                         const T *__restrict__ qf, const T *__restrict__ sor, Dims3 F,
                                                         int pts)
 {
+	await_previous();
 	const int j = 2 + blockIdx.y * TY + threadIdx.y, k = 2 + blockIdx.z;
 	const int i = 2 + ((j + k + pts) & 1) + 2 * (blockIdx.x * TX + threadIdx.x);
 	if (i > F.nx + 1 || j > F.ny + 1) return;
@@ -650,7 +657,7 @@ int relax_point_3d(const T *so, T *x, const T *b, const T *sor, Dims3 F, int upd
 	if (ns == 4) {  // UP (and the non-symmetric sweep): colour 0 then 1; DOWN: 1 then 0
 		const dim3 blk(TX, TY), grd(ceil_div((F.nx + 1) / 2, TX), ceil_div(F.ny, TY), F.nz);
 		for (int c = 0; c < 2; ++c) {
-			k3_gs7_colour<T><<<grd, blk, 0, st>>>(so, x, b, sor, F, updown == CDR_DOWN ? 1 - c : c);
+			launch(k3_gs7_colour<T>, grd, blk, 0, st, so, x, b, sor, F, updown == CDR_DOWN ? 1 - c : c);
 			CDR_LAUNCH_CHECK();
 		}
 		return CDR_OK;
@@ -672,18 +679,18 @@ int relax_point_3d(const T *so, T *x, const T *b, const T *sor, Dims3 F, int upd
 		const int nrj = (F.ny - pj + 1) / 2, nrows = nrj * ((F.nz - pk + 1) / 2);
 		if (nrows == 0) continue;
 		if (staged) {
-			if (updown == CDR_UP) k3_gs_staged<T, true><<<nrows, staged_block(F), smem, st>>>(so, x, b, sor, F, pj, pk, nrj);
-			else k3_gs_staged<T, false><<<nrows, staged_block(F), smem, st>>>(so, x, b, sor, F, pj, pk, nrj);
+			if (updown == CDR_UP) launch(k3_gs_staged<T, true>, nrows, staged_block(F), smem, st, so, x, b, sor, F, pj, pk, nrj);
+			else launch(k3_gs_staged<T, false>, nrows, staged_block(F), smem, st, so, x, b, sor, F, pj, pk, nrj);
 			CDR_LAUNCH_CHECK();
 			continue;
 		}
 		const int grd = ceil_div(nrows, R), blk = R * W;
 		if (updown == CDR_UP) {
-			if (vec) k3_gs_rows<T, true, true><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
-			else k3_gs_rows<T, false, true><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			if (vec) launch(k3_gs_rows<T, true, true>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			else launch(k3_gs_rows<T, false, true>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
 		} else {
-			if (vec) k3_gs_rows<T, true, false><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
-			else k3_gs_rows<T, false, false><<<grd, blk, 0, st>>>(so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			if (vec) launch(k3_gs_rows<T, true, false>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			else launch(k3_gs_rows<T, false, false>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
 		}
 		CDR_LAUNCH_CHECK();
 	}
@@ -696,7 +703,7 @@ template int relax_point_3d<float>(const float *, float *, const float *, const 
 template <typename T>
 int setup_recip_3d(const T *so, T *sor, Dims3 F, cudaStream_t st)
 {
-	k3_recip<T><<<dim3(ceil_div(F.nx, TX), ceil_div(F.ny, TY), F.nz), dim3(TX, TY), 0, st>>>(so, sor, F);
+	launch(k3_recip<T>, dim3(ceil_div(F.nx, TX), ceil_div(F.ny, TY), F.nz), dim3(TX, TY), 0, st, so, sor, F);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -708,6 +715,7 @@ template <typename T>
 __global__ void __launch_bounds__(TX *TY) k3_restrict(const T *__restrict__ ci, const T *__restrict__ q,
                                                       T *__restrict__ qc, Dims3 F, Dims3 C)
 {
+	await_previous();
 	const int ic = blockIdx.x * TX + threadIdx.x + 2, jc = blockIdx.y * TY + threadIdx.y + 2, kc = blockIdx.z + 2;
 	if (ic > C.nx + 1 || jc > C.ny + 1) return;
 	const int i = 2 * ic - 2, j = 2 * jc - 2, k = 2 * kc - 2;
@@ -737,6 +745,7 @@ __global__ void __launch_bounds__(TX *TY) k3_interp_add(const T *__restrict__ ci
                                                         const T *__restrict__ res, const T *__restrict__ so,
                                                         T *__restrict__ q, Dims3 F, Dims3 C)
 {
+	await_previous();
 	const int ic = blockIdx.x * TX + threadIdx.x + 2, jc = blockIdx.y * TY + threadIdx.y + 2, kc = blockIdx.z + 2;
 	const int iic1 = C.nx + 1, kkc1 = C.nz + 1;
 	const int iicf1 = F.nx / 2 + 2, jjcf1 = F.ny / 2 + 2, kkcf1 = F.nz / 2 + 2;
@@ -791,7 +800,7 @@ __global__ void __launch_bounds__(TX *TY) k3_interp_add(const T *__restrict__ ci
 template <typename T>
 int restrict_3d(const T *ci, const T *rf, T *bc, Dims3 F, Dims3 C, cudaStream_t st)
 {
-	k3_restrict<T><<<dim3(ceil_div(C.nx, TX), ceil_div(C.ny, TY), C.nz), dim3(TX, TY), 0, st>>>(ci, rf, bc, F, C);
+	launch(k3_restrict<T>, dim3(ceil_div(C.nx, TX), ceil_div(C.ny, TY), C.nz), dim3(TX, TY), 0, st, ci, rf, bc, F, C);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -802,7 +811,7 @@ template <typename T>
 int interp_add_3d(const T *ci, const T *xc, const T *rf, const T *sof, T *xf, Dims3 F, Dims3 C, cudaStream_t st)
 {
 	const dim3 grd(ceil_div(F.nx / 2 + 1, TX), ceil_div(F.ny / 2 + 1, TY), F.nz / 2 + 1);
-	k3_interp_add<T><<<grd, dim3(TX, TY), 0, st>>>(ci, xc, rf, sof, xf, F, C);
+	launch(k3_interp_add<T>, grd, dim3(TX, TY), 0, st, ci, xc, rf, sof, xf, F, C);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -822,6 +831,7 @@ __device__ __forceinline__ double dmin2(double a, double b) { return a < b ? a :
 __global__ void __launch_bounds__(TX *TY) k3_oi(const double *__restrict__ so, double *__restrict__ ci, Dims3 F,
                                                 Dims3 C, int phase)
 {
+	await_previous();
 	const int ic = blockIdx.x * TX + threadIdx.x + 2, jc = blockIdx.y * TY + threadIdx.y + 2, kc = blockIdx.z + 2;
 	const int iic1 = C.nx + 1, jjc1 = C.ny + 1, kkc1 = C.nz + 1;
 	const int iicf1 = F.nx / 2 + 2, jjcf1 = F.ny / 2 + 2, kkcf1 = F.nz / 2 + 2;
@@ -1014,6 +1024,7 @@ __global__ void __launch_bounds__(TX *TY) k3_oi(const double *__restrict__ so, d
 __global__ void __launch_bounds__(TX *TY) k3_oi7(const double *__restrict__ so, double *__restrict__ ci, Dims3 F,
                                                  Dims3 C, int phase)
 {
+	await_previous();
 	const int ic = blockIdx.x * TX + threadIdx.x + 2, jc = blockIdx.y * TY + threadIdx.y + 2, kc = blockIdx.z + 2;
 	const int iic1 = C.nx + 1, jjc1 = C.ny + 1, kkc1 = C.nz + 1;
 	const int iicf1 = F.nx / 2 + 2, jjcf1 = F.ny / 2 + 2, kkcf1 = F.nz / 2 + 2;
@@ -1129,8 +1140,8 @@ int setup_interp_3d(const double *so, double *ci, Dims3 F, Dims3 C, cudaStream_t
 	CDR_CUDA_TRY(cudaMemsetAsync(ci, 0, sizeof(double) * C.plane() * 26, st));
 	const dim3 grd(ceil_div(F.nx / 2 + 1, TX), ceil_div(F.ny / 2 + 1, TY), F.nz / 2 + 1);
 	for (int ph = 0; ph < 3; ++ph) {
-		if (ns == 4) k3_oi7<<<grd, dim3(TX, TY), 0, st>>>(so, ci, F, C, ph);
-		else k3_oi<<<grd, dim3(TX, TY), 0, st>>>(so, ci, F, C, ph);
+		if (ns == 4) launch(k3_oi7, grd, dim3(TX, TY), 0, st, so, ci, F, C, ph);
+		else launch(k3_oi, grd, dim3(TX, TY), 0, st, so, ci, F, C, ph);
 		CDR_LAUNCH_CHECK();
 	}
 	return CDR_OK;
@@ -1235,6 +1246,7 @@ template <int NS>
 __global__ void __launch_bounds__(TX *TY) k3_galerkin(const double *__restrict__ so, const double *__restrict__ ci,
                                                       double *__restrict__ soc, Dims3 F, Dims3 C)
 {
+	await_previous();
 	const int ic = blockIdx.x * TX + threadIdx.x + 2, jc = blockIdx.y * TY + threadIdx.y + 2;
 	const int kc = blockIdx.z / 14 + 2, pl = blockIdx.z % 14 + 1;
 	if (ic > C.nx + 1 || jc > C.ny + 1) return;
@@ -1265,8 +1277,8 @@ int galerkin_3d(const double *so, const double *ci, double *soc, Dims3 F, Dims3 
 {
 	CDR_CUDA_TRY(cudaMemsetAsync(soc, 0, sizeof(double) * C.plane() * 14, st));
 	const dim3 grd(ceil_div(C.nx, TX), ceil_div(C.ny, TY), C.nz * 14);
-	if (ns == 4) k3_galerkin<4><<<grd, dim3(TX, TY), 0, st>>>(so, ci, soc, F, C);
-	else k3_galerkin<14><<<grd, dim3(TX, TY), 0, st>>>(so, ci, soc, F, C);
+	if (ns == 4) launch(k3_galerkin<4>, grd, dim3(TX, TY), 0, st, so, ci, soc, F, C);
+	else launch(k3_galerkin<14>, grd, dim3(TX, TY), 0, st, so, ci, soc, F, C);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -1279,6 +1291,7 @@ int galerkin_3d(const double *so, const double *ci, double *soc, Dims3 F, Dims3 
 template <int NS>
 __global__ void k3_cg_factor(const double *__restrict__ so, Dims3 F, double *__restrict__ abd, int nabd1, int *info)
 {
+	await_previous();
 	auto S = [&](int ii, int jj, int kk, int p) -> double { return (NS == 4 && p > KB) ? 0.0 : SO(ii, jj, kk, p); };
 	if (threadIdx.x != 0 || blockIdx.x != 0) return;
 	const int II = F.nx + 2, JJ = F.ny + 2, KK = F.nz + 2;
@@ -1347,6 +1360,7 @@ template <typename T, bool WARP, bool STAGED>
 __global__ void __launch_bounds__(WARP ? 128 : 1024) k3_cg_solve(const double *__restrict__ ab, int ldab, T *__restrict__ q,
                                                     const T *__restrict__ qf, Dims3 F)
 {
+	await_previous();
 	extern __shared__ double xs[];
 	const int kd = ldab - 1, n = F.nx * F.ny * F.nz, tid = threadIdx.x;
 	auto at = [&](int m) -> size_t {  // unknown m, x fastest
@@ -1412,8 +1426,8 @@ __global__ void __launch_bounds__(WARP ? 128 : 1024) k3_cg_solve(const double *_
 
 int setup_cg_3d(const double *so, Dims3 F, double *abd, int *info, cudaStream_t st, int ns)
 {
-	if (ns == 4) k3_cg_factor<4><<<1, 32, 0, st>>>(so, F, abd, F.nx * (F.ny + 1) + 2, info);
-	else k3_cg_factor<14><<<1, 32, 0, st>>>(so, F, abd, F.nx * (F.ny + 1) + 2, info);
+	if (ns == 4) launch(k3_cg_factor<4>, 1, 32, 0, st, so, F, abd, F.nx * (F.ny + 1) + 2, info);
+	else launch(k3_cg_factor<14>, 1, 32, 0, st, so, F, abd, F.nx * (F.ny + 1) + 2, info);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -1429,11 +1443,11 @@ int solve_cg_3d(const double *abd, T *x, const T *b, Dims3 F, cudaStream_t st)
 	}
 	const int blk = kd <= 128 ? 128 : kd < 1024 ? (kd + 31) / 32 * 32 : 1024;
 	if (staged <= 48 * 1024) {
-		if (kd <= 32) k3_cg_solve<T, true, true><<<1, blk, staged, st>>>(abd, ldab, x, b, F);
-		else k3_cg_solve<T, false, true><<<1, blk, staged, st>>>(abd, ldab, x, b, F);
+		if (kd <= 32) launch(k3_cg_solve<T, true, true>, 1, blk, staged, st, abd, ldab, x, b, F);
+		else launch(k3_cg_solve<T, false, true>, 1, blk, staged, st, abd, ldab, x, b, F);
 	} else {
-		if (kd <= 32) k3_cg_solve<T, true, false><<<1, blk, sm, st>>>(abd, ldab, x, b, F);
-		else k3_cg_solve<T, false, false><<<1, blk, sm, st>>>(abd, ldab, x, b, F);
+		if (kd <= 32) launch(k3_cg_solve<T, true, false>, 1, blk, sm, st, abd, ldab, x, b, F);
+		else launch(k3_cg_solve<T, false, false>, 1, blk, sm, st, abd, ldab, x, b, F);
 	}
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
@@ -1464,6 +1478,7 @@ __global__ void __launch_bounds__(TX *TY) k3_ir_residual(const double *__restric
                                                          double *__restrict__ xo, float *__restrict__ r32, Dims3 F,
                                                          Dims3 E, double *__restrict__ partial, int apply)
 {
+	await_previous();
 	__shared__ double sh[TX * TY / 32];
 	const int tx = (F.nx + TX - 1) / TX, ty = (F.ny + TY - 1) / TY;
 	const long ntiles = (long)tx * ty * F.nz;
@@ -1489,6 +1504,7 @@ __global__ void __launch_bounds__(TX *TY) k3_ir_residual(const double *__restric
 __global__ void __launch_bounds__(256) k3_ir_add(const double *__restrict__ x, const float *__restrict__ e,
                                                  double *__restrict__ xo, Dims3 F)
 {
+	await_previous();
 	const int i = blockIdx.x * 64 + threadIdx.x + 1, j = blockIdx.y * 4 + threadIdx.y + 1, k = blockIdx.z + 1;
 	if (i > F.nx || j > F.ny) return;
 	const size_t o = ((size_t)k * (F.ny + 2) + j) * F.pitch + i;
@@ -1506,19 +1522,19 @@ int ir_residual_3d(const double *so, const double *x, const float *e, const doub
 	const int nb = ntiles < 2048 ? (int)ntiles : 2048;
 	if (ns == 14 && d32.pitch == d.pitch) {
 		if (apply) {
-			k3_ir_add<<<dim3(ceil_div(d.nx, 64), ceil_div(d.ny, 4), d.nz), dim3(64, 4), 0, st>>>(x, e, xo, d);
+			launch(k3_ir_add, dim3(ceil_div(d.nx, 64), ceil_div(d.ny, 4), d.nz), dim3(64, 4), 0, st, x, e, xo, d);
 			CDR_LAUNCH_CHECK();
 		}
-		k3_residual<double, true, 14, float><<<nb, dim3(TX, TY), 0, st>>>(so, apply ? xo : x, b, r32, d, partial);
+		launch(k3_residual<double, true, 14, float>, nb, dim3(TX, TY), 0, st, so, apply ? xo : x, b, r32, d, partial);
 		CDR_LAUNCH_CHECK();
-		k3_norm_finish<<<1, 1024, 0, st>>>(partial, nb, norm_out);
+		launch(k3_norm_finish, 1, 1024, 0, st, partial, nb, norm_out);
 		CDR_LAUNCH_CHECK();
 		return CDR_OK;
 	}
-	if (ns == 4) k3_ir_residual<4><<<nb, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply);
-	else k3_ir_residual<14><<<nb, dim3(TX, TY), 0, st>>>(so, x, e, b, xo, r32, d, d32, partial, apply);
+	if (ns == 4) launch(k3_ir_residual<4>, nb, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, d32, partial, apply);
+	else launch(k3_ir_residual<14>, nb, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, d32, partial, apply);
 	CDR_LAUNCH_CHECK();
-	k3_norm_finish<<<1, 1024, 0, st>>>(partial, nb, norm_out);
+	launch(k3_norm_finish, 1, 1024, 0, st, partial, nb, norm_out);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

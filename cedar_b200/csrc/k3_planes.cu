@@ -36,6 +36,7 @@ template <int NS2>
 __global__ void k3_plane_coeff(const double *__restrict__ so, Dims3 F, int dir, double *__restrict__ so2, int n1,
                                int n2, int pitch2)
 {
+	await_previous();
 	const int a = blockIdx.x * TX + threadIdx.x, b = blockIdx.y * TY + threadIdx.y, ipl = blockIdx.z + 1;
 	if (a > n1 + 1 || b > n2 + 1) return;
 	if (dir == 1 && (b < 1 || b > n2)) return;
@@ -53,6 +54,7 @@ template <typename T, bool TO_PLANE>
 __global__ void k3_plane_copy(T *__restrict__ x3, Dims3 F, int dir, int first, int step, T *__restrict__ x2, int n1,
                               int n2, int pitch2)
 {
+	await_previous();
 	const int a = blockIdx.x * TX + threadIdx.x, b = blockIdx.y * TY + threadIdx.y;
 	const int ipl = first + 1 + blockIdx.z * step;
 	if (a > n1 + 1 || b > n2 + 1) return;
@@ -72,14 +74,14 @@ int plane_copy(T *x3, Dims3 F, int dir, int first, int step, int count, T *x2, i
 {
 	if (dir == 2) {  // yz planes: through a shared-memory transpose
 		const dim3 grd(ceil_div(count, TX), ceil_div(n1 + 2, TX), n2 + 2);
-		if (to_plane) k3_plane_copy_yz<T, true><<<grd, dim3(TX, TY), 0, st>>>(x3, F, first, step, count, x2, n1, n2, pitch2);
-		else k3_plane_copy_yz<T, false><<<grd, dim3(TX, TY), 0, st>>>(x3, F, first, step, count, x2, n1, n2, pitch2);
+		if (to_plane) launch(k3_plane_copy_yz<T, true>, grd, dim3(TX, TY), 0, st, x3, F, first, step, count, x2, n1, n2, pitch2);
+		else launch(k3_plane_copy_yz<T, false>, grd, dim3(TX, TY), 0, st, x3, F, first, step, count, x2, n1, n2, pitch2);
 		CDR_LAUNCH_CHECK();
 		return CDR_OK;
 	}
 	const dim3 grd(ceil_div(n1 + 2, TX), ceil_div(n2 + 2, TY), count);
-	if (to_plane) k3_plane_copy<T, true><<<grd, dim3(TX, TY), 0, st>>>(x3, F, dir, first, step, x2, n1, n2, pitch2);
-	else k3_plane_copy<T, false><<<grd, dim3(TX, TY), 0, st>>>(x3, F, dir, first, step, x2, n1, n2, pitch2);
+	if (to_plane) launch(k3_plane_copy<T, true>, grd, dim3(TX, TY), 0, st, x3, F, dir, first, step, x2, n1, n2, pitch2);
+	else launch(k3_plane_copy<T, false>, grd, dim3(TX, TY), 0, st, x3, F, dir, first, step, x2, n1, n2, pitch2);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(TX *TY) k3_plane_rhs(const T *__restrict__ so,
                                                        const T *__restrict__ bb, Dims3 F, int dir, int first, int step,
                                                        T *__restrict__ b2, int n1, int n2, int pitch2)
 {
+	await_previous();
 	const int p = blockIdx.x * TX + threadIdx.x + 1, q = blockIdx.y * TY + threadIdx.y + 1;
 	const int ipl = first + 1 + blockIdx.z * step;
 	if (p > n1 || q > n2) return;
@@ -164,6 +167,7 @@ __global__ void __launch_bounds__(TX *TY) k3_plane_rhs_yz(const T *__restrict__ 
                                                           const T *__restrict__ bb, Dims3 F, int first, int step,
                                                           int count, T *__restrict__ b2, int n1, int n2, int pitch2)
 {
+	await_previous();
 	__shared__ T tile[TX][TX + 1];
 	const int z0 = blockIdx.x * TX, a0 = blockIdx.y * TX + 1, q = blockIdx.z + 1;
 	const size_t P = F.plane();
@@ -205,6 +209,7 @@ template <typename T, bool TO_PLANE>
 __global__ void __launch_bounds__(TX *TY) k3_plane_copy_yz(T *__restrict__ x3, Dims3 F, int first, int step,
                                                            int count, T *__restrict__ x2, int n1, int n2, int pitch2)
 {
+	await_previous();
 	__shared__ T tile[TX][TX + 1];
 	const int z0 = blockIdx.x * TX, a0 = blockIdx.y * TX, b = blockIdx.z;
 	const size_t pl2 = (size_t)pitch2 * (n2 + 2);
@@ -239,14 +244,14 @@ int plane_rhs(const T *so, const T *x, const T *b, Dims3 F, int dir, int first, 
 {
 	if (dir == 2) {
 		const dim3 grd(ceil_div(count, TX), ceil_div(n1, TX), n2);
-		if (ns == 4) k3_plane_rhs_yz<T, 4><<<grd, dim3(TX, TY), 0, st>>>(so, x, b, F, first, step, count, b2, n1, n2, pitch2);
-		else k3_plane_rhs_yz<T, 14><<<grd, dim3(TX, TY), 0, st>>>(so, x, b, F, first, step, count, b2, n1, n2, pitch2);
+		if (ns == 4) launch(k3_plane_rhs_yz<T, 4>, grd, dim3(TX, TY), 0, st, so, x, b, F, first, step, count, b2, n1, n2, pitch2);
+		else launch(k3_plane_rhs_yz<T, 14>, grd, dim3(TX, TY), 0, st, so, x, b, F, first, step, count, b2, n1, n2, pitch2);
 		CDR_LAUNCH_CHECK();
 		return CDR_OK;
 	}
 	const dim3 grd(ceil_div(n1, TX), ceil_div(n2, TY), count);
-	if (ns == 4) k3_plane_rhs<T, 4><<<grd, dim3(TX, TY), 0, st>>>(so, x, b, F, dir, first, step, b2, n1, n2, pitch2);
-	else k3_plane_rhs<T, 14><<<grd, dim3(TX, TY), 0, st>>>(so, x, b, F, dir, first, step, b2, n1, n2, pitch2);
+	if (ns == 4) launch(k3_plane_rhs<T, 4>, grd, dim3(TX, TY), 0, st, so, x, b, F, dir, first, step, b2, n1, n2, pitch2);
+	else launch(k3_plane_rhs<T, 14>, grd, dim3(TX, TY), 0, st, so, x, b, F, dir, first, step, b2, n1, n2, pitch2);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
@@ -261,8 +266,8 @@ int plane_coeff(const double *so, Dims3 F, int dir, double *so2, int n, int n1, 
 	const int ns2 = ns == 4 ? 3 : 5;
 	CDR_CUDA_TRY(cudaMemsetAsync(so2, 0, sizeof(double) * ns2 * (size_t)pitch2 * (n2 + 2) * n, st));
 	const dim3 grd(ceil_div(n1 + 2, TX), ceil_div(n2 + 2, TY), n);
-	if (ns == 4) k3_plane_coeff<3><<<grd, dim3(TX, TY), 0, st>>>(so, F, dir, so2, n1, n2, pitch2);
-	else k3_plane_coeff<5><<<grd, dim3(TX, TY), 0, st>>>(so, F, dir, so2, n1, n2, pitch2);
+	if (ns == 4) launch(k3_plane_coeff<3>, grd, dim3(TX, TY), 0, st, so, F, dir, so2, n1, n2, pitch2);
+	else launch(k3_plane_coeff<5>, grd, dim3(TX, TY), 0, st, so, F, dir, so2, n1, n2, pitch2);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }

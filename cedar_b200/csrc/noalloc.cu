@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(TX *TY) k_residual_tile_norm(const double *__r
                                                                const double *__restrict__ qf, double *__restrict__ res,
                                                                Dims2 d, double *__restrict__ partial)
 {
+	await_previous();
 	__shared__ double sh[TX * TY / 32];
 	const int tiles_x = (d.nx + TX - 1) / TX;
 	const int i = (blockIdx.x % tiles_x) * TX + threadIdx.x + 1;
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(TX *TY) k_residual_tile_norm(const double *__r
 
 __global__ void __launch_bounds__(1024) k_noalloc_norm_finish(const double *__restrict__ partial, int n, double *out)
 {
+	await_previous();
 	__shared__ double sh[32];
 	double v = 0;
 	for (int i = threadIdx.x; i < n; i += blockDim.x) v += partial[i];
@@ -128,11 +130,11 @@ extern "C" int cdr_gpu_residual_2d_f64_noalloc(const double *so, int nstencil, c
 	CDR_TRY(noalloc_scratch(&partial));
 	const Dims2 d{nx, ny, pitch};
 	if (nstencil == 5)
-		k_residual_tile_norm<5><<<(unsigned)tiles, dim3(TX, TY), 0, stream>>>(so, x, b, r, d, partial);
+		launch(k_residual_tile_norm<5>, (unsigned)tiles, dim3(TX, TY), 0, stream, so, x, b, r, d, partial);
 	else
-		k_residual_tile_norm<3><<<(unsigned)tiles, dim3(TX, TY), 0, stream>>>(so, x, b, r, d, partial);
+		launch(k_residual_tile_norm<3>, (unsigned)tiles, dim3(TX, TY), 0, stream, so, x, b, r, d, partial);
 	CDR_LAUNCH_CHECK();
-	k_noalloc_norm_finish<<<1, 1024, 0, stream>>>(partial, (int)tiles, norm_out);
+	launch(k_noalloc_norm_finish, 1, 1024, 0, stream, partial, (int)tiles, norm_out);
 	CDR_LAUNCH_CHECK();
 	return CDR_OK;
 }
