@@ -6,6 +6,11 @@ namespace cdrgpu {
 
 constexpr int TX = 32, TY = 8;  // 2D tile of the point kernels
 
+// two-element vectors of a type
+template <typename T> struct Vec2;
+template <> struct Vec2<float> { using type = float2; };
+template <> struct Vec2<double> { using type = double2; };
+
 // a*b + c: one fused multiply-add in FP32 (the preconditioner's kernels), a
 // separately rounded product and sum in FP64 (the library is built without FMA
 // contraction so that the FP64 kernels give the reference's bits; c + a*b and

@@ -276,6 +276,121 @@ __global__ void __launch_bounds__(TX *TY) k_gs_colour(const T *__restrict__ so, 
 	gs_at<T, NS>(so, ps, q, qf, sor, d.at(i, j), pitch);
 }
 
+// Two colours of the nine-point sweep (BMG2_SymStd_relax_GS.f90:93-133) in one
+// pass: the rows of one parity, first the points of one x-parity, then the
+// others.  A row's second colour depends on the first only inside the row, so a
+// block that owns whole rows needs no other block, and a sweep is two launches.
+// A thread takes the points a = 2t, b = 2t + 1 (0-based) and loads every operand
+// of both at once: a row's operator lines are read once with all of their bytes
+// used (one colour per launch uses every second element, and reads each line
+// twice).  A visit of a 1000 x 701 FP64 level (two sweeps, residual, transfers)
+// 65 -> 54 us; in segments of 512 pairs 70 us.  Rows longer than
+// 2 W points run in segments from the side whose first colour the second one
+// reads.  SECOND_A: b first, then a (DOWN); else a, then b (UP).
+template <typename T, bool VEC, bool SECOND_A>
+__global__ void __launch_bounds__(256) k_gs_rows(const T *__restrict__ so, T *__restrict__ q, const T *__restrict__ qf,
+                                                 const T *__restrict__ sor, Dims2 d, int j0, int W)
+{
+	await_previous();
+	using V2 = typename Vec2<T>::type;
+	__shared__ T sh[256];    // first-colour values of the segment
+	__shared__ T edge[256];  // per row: the first-colour value the next segment reads
+	const size_t ps = d.plane();
+	so += d.bofs(5 * ps);
+	q += d.bofs(ps);
+	qf += d.bofs(ps);
+	sor += d.bofs(2 * ps);
+	const int r = threadIdx.x / W, t0 = threadIdx.x - r * W;
+	const int j = j0 + 2 * (int)(blockIdx.x * (blockDim.x / W) + r);
+	const int nT = d.nx / 2 + 1, nseg = (nT + W - 1) / W, p = d.pitch;
+	auto pair = [&](const T *x, T(&v)[2]) {
+		if constexpr (VEC) {
+			const V2 u = *reinterpret_cast<const V2 *>(x);
+			v[0] = u.x;
+			v[1] = u.y;
+		} else {
+			v[0] = x[0];
+			v[1] = x[1];
+		}
+	};
+	for (int s = 0; s < nseg; ++s) {
+		const int t = (SECOND_A ? s : nseg - 1 - s) * W + t0;
+		const bool live = j <= d.ny && t < nT, va = live && t >= 1, vb = live && 2 * t + 1 <= d.nx;
+		const size_t k = (size_t)j * p + 2 * t;
+		T f[2], ds[2], w[3], s0[2], s1[2], sw0[2], nw0[2], nw1[2], sw1[2], Y[4], M[4], P[4];
+		T first = T(0);
+		// point e (0: a, 1: b) from its row neighbours, in gs_at's operand order
+		auto point = [&](int e, T left, T right) -> T {
+			T acc = madd(w[e], left, f[e]);
+			acc = madd(w[e + 1], right, acc);
+			acc = madd(s0[e], M[1 + e], acc);
+			acc = madd(s1[e], P[1 + e], acc);
+			acc = madd(sw0[e], M[e], acc);
+			acc = madd(nw0[e], M[2 + e], acc);
+			acc = madd(nw1[e], P[e], acc);
+			acc = madd(sw1[e], P[2 + e], acc);
+			return acc * ds[e];
+		};
+		if (live) {
+			auto row4 = [&](const T *x, T(&v)[4]) {  // left neighbour of a, a, b, right neighbour of b
+				T c[2];
+				pair(x, c);
+				v[0] = t >= 1 ? x[-1] : T(0);
+				v[1] = c[0];
+				v[2] = c[1];
+				v[3] = vb ? x[2] : T(0);
+			};
+			auto right = [&](const T *x, T(&v)[2]) {  // a plane at the right neighbours
+				v[0] = x[1];
+				v[1] = vb ? x[2] : T(0);
+			};
+			const T *cw = so + ps + k, *cs = so + 2 * ps + k, *csw = so + 3 * ps + k, *cnw = so + 4 * ps + k;
+			T c[2];
+			pair(cw, c);
+			w[0] = c[0];
+			w[1] = c[1];
+			w[2] = vb ? cw[2] : T(0);
+			pair(cs, s0);
+			pair(cs + p, s1);
+			pair(csw, sw0);
+			right(cnw, nw0);
+			pair(cnw + p, nw1);
+			right(csw + p, sw1);
+			pair(qf + k, f);
+			pair(sor + k, ds);
+			row4(q + k, Y);
+			row4(q + k - p, M);
+			row4(q + k + p, P);
+			// a point outside the interior keeps its value
+			if (SECOND_A) first = vb ? point(1, Y[1], Y[3]) : Y[2];
+			else first = va ? point(0, Y[0], Y[2]) : Y[1];
+		}
+		sh[threadIdx.x] = first;
+		__syncthreads();  // the segment's row is read, its first colour formed
+		if (live) {
+			T second;
+			if (SECOND_A) second = va ? point(0, t0 > 0 ? sh[threadIdx.x - 1] : edge[r], first) : T(0);
+			else second = vb ? point(1, first, t + 1 >= nT ? Y[3] : t0 + 1 < W ? sh[threadIdx.x + 1] : edge[r]) : T(0);
+			const T na = SECOND_A ? second : first, nb = SECOND_A ? first : second;
+			T *qo = q + k;
+			if (VEC && va && vb) {
+				V2 v;
+				v.x = na;
+				v.y = nb;
+				*reinterpret_cast<V2 *>(qo) = v;
+			} else {
+				if (va) qo[0] = na;
+				if (vb) qo[1] = nb;
+			}
+		}
+		if (nseg > 1) {
+			__syncthreads();  // edge and sh are read
+			if (t0 == (SECOND_A ? W - 1 : 0)) edge[r] = first;
+		}
+	}
+}
+
+
 // Periodic branch (BMG2_SymStd_relax_GS.f90:139-226): the reference copies a
 // row's x ghosts after the row's points of a colour and the y ghost rows after
 // the whole sweep.  Points of a colour never read another row's x ghosts that
@@ -288,7 +403,27 @@ int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Di
 {
 	dim3 blk(TX, TY);
 	const bool perx = per & 1, pery = (per >> 1) & 1;
-	if (nstencil == 5) {
+	if (nstencil == 5 && !per) {
+		// two colours per launch; W pairs of points per row and segment (equal segments
+		// of at most 256), rows to a block of 128 threads or one longer row
+		const bool vec = d.pitch % 2 == 0 &&
+		                 ((uintptr_t)so | (uintptr_t)x | (uintptr_t)b | (uintptr_t)sor) % (2 * sizeof(T)) == 0;
+		const int nT = d.nx / 2 + 1, W = ceil_div(nT, ceil_div(nT, 256)), R = W < 128 ? 128 / W : 1;
+		for (int c = 0; c < 2; ++c) {
+			// DOWN: rows of odd 0-based j first, i odd then even; UP: the reverse
+			const int j0 = (updown == CDR_DOWN) == (c == 0) ? 1 : 2;
+			if (j0 > d.ny) continue;
+			const dim3 grd(ceil_div((d.ny - j0) / 2 + 1, R), 1, d.nb);
+			if (updown == CDR_DOWN) {
+				if (vec) launch(k_gs_rows<T, true, true>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
+				else launch(k_gs_rows<T, false, true>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
+			} else {
+				if (vec) launch(k_gs_rows<T, true, false>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
+				else launch(k_gs_rows<T, false, false>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
+			}
+			CDR_LAUNCH_CHECK();
+		}
+	} else if (nstencil == 5) {
 		// DOWN: (JBEG, IBEG) = (2,2),(2,3),(3,2),(3,3) with JBEG outer; UP reversed.
 		// Fortran index 2 is 0-based 1 (odd), 3 is 0-based 2 (even).
 		const int order[4][2] = {{1, 1}, {1, 0}, {0, 1}, {0, 0}};  // (j odd?, i odd?)

@@ -64,10 +64,6 @@ __device__ __forceinline__ T nbs(const T *__restrict__ so, XQ xq, T qf, Dims3 F,
 	else return nb27<T>(so, xq, qf, F, i, j, k);
 }
 
-template <typename T> struct Vec2;
-template <> struct Vec2<float> { using type = float2; };
-template <> struct Vec2<double> { using type = double2; };
-
 // every pointer a multiple of n bytes
 template <typename... P>
 static bool aligned_to(size_t n, const P *...p)

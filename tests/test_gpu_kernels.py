@@ -580,3 +580,30 @@ def test_line_factors_chunk_edges(lib, oracle, nx, ny, extra):
             assert np.array_equal(got[inner], want)
             got[inner] = -7.0
             assert (got == -7.0).all()
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (2, 5), (3, 2), (62, 7), (127, 9), (255, 4), (509, 6), (510, 5), (511, 3),
+                                   (512, 4), (1026, 2), (2050, 4)])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_gs_rows_edges(lib, oracle, nx, ny, extra):
+    """The two-colour nine-point row sweep at the edges of its blocks and row segments (256 pairs of
+    points), with aligned and unaligned rows: FP64 bits of the oracle, FP32 within the rounding of
+    its 9-term sums."""
+    import torch
+    k = np.exp(np.random.default_rng(nx).standard_normal((ny + 1, nx + 1)))
+    so, x, b = np.ascontiguousarray(G.fe_hetero(k, k)), grid(nx, ny, 1), grid(nx, ny, 2)
+    sor = np.zeros_like(x)
+    sor[1:-1, 1:-1] = 1.0 / so[0][1:-1, 1:-1]
+    p = nx + 2 + (nx + extra) % 2
+    d64 = [padded(a, p) for a in (so, x, b, sor)]
+    d32 = [a.to(torch.float32) for a in d64]
+    both = np.zeros((2,) + x.shape)
+    both[1] = sor
+    for updown in (_lib.DOWN, _lib.UP):
+        oracle.relax_gs(so, x, b, both, updown)
+        for d, f in ((d64, lib.cdr_gpu_relax_point_2d_f64), (d32, lib.cdr_gpu_relax_point_2d_f32)):
+            _lib.check(f(ptr(d[0]), 5, ptr(d[1]), ptr(d[2]), ptr(d[3]), nx, ny, p, updown, stream()))
+    assert np.array_equal(host(d64[1])[:, :nx + 2], x)
+    # two sweeps of 9-term sums of inputs rounded to 2^-24, on values of the size of x and b / c
+    size = np.abs(x).max() + np.abs(b * sor).max()
+    assert np.abs(host(d32[1])[:, :nx + 2] - x).max() <= 2 * 4 * 10 * 2.0 ** -24 * size
