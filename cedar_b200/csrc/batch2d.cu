@@ -278,17 +278,18 @@ int Batch2::ncycle(int l, Sel sel, bool zero)
 	return CDR_OK;
 }
 
-// First level (not the fine one) of the fused coarse cycle: both edges at most
-// fuse_coarse and the level's shared-memory copy within the limit
+// First level of the fused coarse cycle (the fine one only with fuse_fine): both
+// edges at most fuse_coarse and the level's shared-memory copy within the limit
 template <typename T>
 int Batch2::pick_fused()
 {
 	if (s.fuse_coarse <= 0) return -1;
-	for (int l0 = 1; l0 + 1 < L(); ++l0) {
+	for (int l0 = fuse_fine ? 0 : 1; l0 + 1 < L(); ++l0) {
 		if (lv[l0].nx > s.fuse_coarse || lv[l0].ny > s.fuse_coarse || L() - l0 > kMaxCoarseLevels) continue;
 		CoarseCycle<T> cc;
 		cc.nl = L() - l0;
 		cc.relax = s.relaxation;
+		cc.x0 = l0 == 0;
 		for (int l = l0; l < L(); ++l) {
 			CoarseLevel<T> &c = cc.lv[l - l0];
 			c.nx = lv[l].nx;
@@ -302,7 +303,7 @@ int Batch2::pick_fused()
 
 // Levels l0..L-1 of the selected problems in one launch, one CTA per problem
 template <typename T>
-int Batch2::fused(int l0, Sel sel)
+int Batch2::fused(int l0, Sel sel, bool x0)
 {
 	CoarseCycle<T> cc;
 	cc.nl = L() - l0;
@@ -329,6 +330,7 @@ int Batch2::fused(int l0, Sel sel)
 	cc.npre = s.nrelax_pre;
 	cc.npost = s.nrelax_post;
 	cc.bstep = sel.step;
+	cc.x0 = x0;
 	return coarse_cycle<T>(cc, sel.count, st);
 }
 
@@ -341,6 +343,7 @@ int Batch2::cycle(Sel sel, bool zero)
 		const size_t f = sel.first, fp = F.plane();
 		return solve_cg_2d<T>(abd + f * abd_size(), BA<T>::x(F) + f * fp, BA<T>::b(F) + f * fp, F.dims(sel), st);
 	}
+	if (lc[sizeof(T) == 4] == 0) return fused<T>(0, sel, !zero);
 	return ncycle<T>(0, sel, zero);
 }
 template int Batch2::cycle<double>(Sel, bool);

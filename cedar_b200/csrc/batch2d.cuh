@@ -48,6 +48,9 @@ public:
 	int *info = nullptr;  // [0] line factorizations, [1] coarse Cholesky
 	int lc[2] = {-1, -1}; // first level of the fused coarse cycle, [0] FP64, [1] FP32 (-1: none)
 	cudaStream_t st = nullptr;
+	// the fused coarse cycle may start at the fine level (a whole cycle in one
+	// launch, one CTA per problem); set before init
+	bool fuse_fine = false;
 
 	Batch2() = default;
 	Batch2(const Batch2 &) = delete;
@@ -85,7 +88,7 @@ private:
 	template <typename T>
 	int ncycle(int l, Sel sel, bool zero = false);
 	template <typename T>
-	int fused(int l0, Sel sel);
+	int fused(int l0, Sel sel, bool x0 = false);  // x0: level l0's iterate is read, not zero
 	template <typename T>
 	int pick_fused();
 	template <typename T>

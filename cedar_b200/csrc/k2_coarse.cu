@@ -92,7 +92,7 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 		const size_t pl = (size_t)(L.nx + 2) * (L.ny + 2);
 		const bool last = l == cc.nl - 1;
 		P.off[l] = CcOffsets{-1, -1, -1, -1, -1, -1, -1};
-		P.off[l].x = take(pl);
+		if (l > 0 || !cc.x0) P.off[l].x = take(pl);
 		if (!last) P.off[l].r = take(pl);
 		if (l > 0) P.off[l].b = take(pl);
 	}
@@ -129,10 +129,12 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 			}
 			if (cc_sory_planes(cc.relax)) P.off[l].sory = stage(L.sory, L.tpitch, (size_t)L.tpitch * ii, jj, ii, 2);
 			const size_t a = (size_t)((L.ny + 1) / 2) * L.nx, b = (size_t)((L.nx + 1) / 2) * L.ny;
-			ln = std::max(ln, std::max(a, b));
+			// FP32 lines of up to 64 points stay in registers
+			if (sizeof(T) == 8 || L.nx > 64 || L.ny > 64) ln = std::max(ln, std::max(a, b));
 		}
 		if (l > 0) P.off[l].ci = stage(L.ci, L.pitch, gpl, ii, jj, 8);
 		if (l == 0) P.off[l].b = stage(L.b, L.pitch, gpl, ii, jj, 1);
+		if (l == 0 && cc.x0) P.off[l].x = stage(L.x, L.pitch, gpl, ii, jj, 1);
 		(void)pl;
 	}
 	P.lines = take(ln);
@@ -508,9 +510,9 @@ __global__ void __launch_bounds__(CC_THREADS, sizeof(T) == 4 ? 2 : 1) k_coarse_c
 	T *sm = base + P.lines;  // line right-hand sides
 	double *xs = reinterpret_cast<double *>(cc_smem + P.dbl_byte);
 	const int nl = cc.nl;
-	// stage: operators, factors and weights of every level, b of the first level,
-	// and after the coarsest right-hand side xs its band factor; x, r and the other
-	// b zero (ghost rings included)
+	// stage: operators, factors and weights of every level, b (and, with x0, x) of
+	// the first level, and after the coarsest right-hand side xs its band factor; the
+	// other x, r and b zero (ghost rings included)
 	cc_stage<T>(P, base);
 	{
 		const CoarseLevel<T> &Cg = cc.lv[nl - 1];

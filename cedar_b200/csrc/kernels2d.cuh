@@ -136,7 +136,7 @@ int fcg_step(const double *so, int ns, const TZ *z, const float *zf, TR *rin, TR
 constexpr size_t kNormScratchBytes = 2048 * sizeof(double);
 
 // Levels of a fused coarse cycle (k2_coarse.cu): level 0 holds the restricted
-// right-hand side and a zero iterate on entry; the last level is the coarsest
+// right-hand side and a zero iterate (or, with x0, its iterate) on entry; the last level is the coarsest
 // (banded Cholesky factor abd).  Arrays of a batch lie back to back (problem
 // blockIdx.x * bstep; the pointers are those of the first problem).
 constexpr int kMaxCoarseLevels = 12;
@@ -152,9 +152,10 @@ struct CoarseCycle {
 	int nl = 0;
 	const double *abd = nullptr;
 	int relax = CDR_RELAX_POINT, npre = 2, npost = 1, bstep = 1;
+	bool x0 = false;  // the first level's iterate is read (else it is zero on entry)
 };
 // shared memory of the fused kernel (bytes) and its limit
-constexpr size_t kCoarseSmemMax = 220 * 1024;
+constexpr size_t kCoarseSmemMax = 226 * 1024;
 template <typename T>
 size_t coarse_cycle_bytes(const CoarseCycle<T> &cc);
 template <typename T>

@@ -318,6 +318,8 @@ static int create3(cdr_gpu_solver3 *h, const double *so_src, int src_pitch, cuda
 			const int np = dir == 0 ? L.nz : dir == 1 ? L.ny : L.nx;
 			const int n1 = dir == 2 ? L.ny : L.nx, n2 = dir == 0 ? L.ny : L.nz;
 			L.pl[dir].reset(new Batch2());
+			// small planes: the whole 2D cycle in one launch
+			L.pl[dir]->fuse_fine = true;
 			CDR_TRY(L.pl[dir]->init(s2, L.ns == 4 ? 3 : 5, n1, n2, np, h->st));
 		}
 		if (h->mixed()) {

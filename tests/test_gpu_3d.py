@@ -477,3 +477,23 @@ def test_staged_rows3_edges(lib, oracle, nx, ny, nz):
         _lib.check(lib.cdr_gpu_relax_point_3d_f64(ptr(dso), 14, ptr(dx), ptr(db), ptr(dsor), nx, ny, nz, p, updown,
                                                   stream()))
     assert np.array_equal(unpad(dx, nx), x)
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(17, 9, 12), (32, 33, 31), (48, 40, 5), (64, 56, 9), (65, 33, 20)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32-ir"])
+def test_fused_planes3(lib, oracle, nx, ny, nz, precision):
+    """Plane smoothers whose 2D cycle runs in one launch from the plane's fine level (its iterate read,
+    not zero), at the sizes where that starts and stops, against the separate launches: FP64 with
+    sequential line solves bit for bit, FP32 to the tolerance in as many cycles."""
+    from cedar_b200.solver import Solver3D
+    so, b = make_op3(nx, ny, nz), grid3(nx, ny, nz, 2)
+    out = []
+    for fuse in (32, 0):
+        s = Solver3D(so, Config({"solver": {"relaxation": "plane-xyz", "max-iter": 12, "tol": 1e-9},
+                                 "gpu": {"precision": precision, "line-solve": "sequential", "fuse-coarse": fuse}}))
+        x = s.solve(b, grid3(nx, ny, nz, 7))
+        out.append((x, s.history.copy()))
+    if precision == "fp64":
+        assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    else:
+        assert out[0][1][-1] < 1e-9 and abs(len(out[0][1]) - len(out[1][1])) <= 1
