@@ -251,6 +251,9 @@ __device__ __forceinline__ void line_chunk(const T *__restrict__ so, T *__restri
 	const T *D = DIR == CDR_DIR_X ? sor + (size_t)lc * P : sor + (size_t)lc * tpitch;
 	const T *E = DIR == CDR_DIR_X ? sor + ps + (size_t)lc * P : sor + (size_t)tpitch * (d.nx + 2) + (size_t)lc * tpitch;
 
+	// long chunks read their pivots only after the forward scan: have them in L2 by then
+	if (K > 8 && has) asm volatile("prefetch.global.L2 [%0];" ::"l"(D + p0));
+
 	// 1. right-hand sides of the chunk
 	T r[K];
 #pragma unroll

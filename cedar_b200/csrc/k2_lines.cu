@@ -992,10 +992,10 @@ static int tune_dir(const T *so, T *x, const T *b, const T *sor, Dims2 d, int tp
 	const int TPL = 1 << tpl_log2_of(n, K);
 	const int caps_x[4] = {32, 64, 128, 256};
 	const int caps_y[4] = {TPL, 2 * TPL, 4 * TPL, 8 * TPL};
-	// Each candidate is timed on one sweep (both colours) after L2 has been
-	// overwritten, best of three: the sweep of a level inside a cycle finds its
-	// arrays in DRAM, and a level that fits in L2 would otherwise favour shapes
-	// that only win on L2-resident data.
+	// Each candidate is timed as a cycle runs it: captured in a graph (launches of
+	// the host would add a gap between the colours that a cycle does not have), two
+	// sweeps of both colours after L2 has been overwritten -- the first finds the
+	// level's arrays in DRAM, the second what L2 keeps of them -- best of three.
 	int dev = 0, l2 = 0;
 	CDR_CUDA_TRY(cudaGetDevice(&dev));
 	CDR_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
@@ -1009,30 +1009,38 @@ static int tune_dir(const T *so, T *x, const T *b, const T *sor, Dims2 d, int tp
 	CDR_CUDA_TRY(cudaEventCreate(&e0));
 	CDR_CUDA_TRY(cudaEventCreate(&e1));
 	int rc = CDR_OK;
+	auto sweep = [&](const LineShape &sh) -> int {
+		if (DIR == CDR_DIR_Y && ysync && d.nb == 1 && sh.pair)  // both colours in one launch
+			return sh.K == 16 ? launch_ypair<T, NS, 16>(so, x, b, sor, d, tpitch, CDR_DOWN, sh.cap, ysync, st, false, yc)
+			                  : launch_ypair<T, NS, 8>(so, x, b, sor, d, tpitch, CDR_DOWN, sh.cap, ysync, st, false, yc);
+		int r = CDR_OK;
+		for (int f = 1; f <= 2 && r == CDR_OK; ++f)
+			r = launch_lines<T, NS, DIR>(so, x, b, sor, d, tpitch, f, false, st, &sh, false, yc);
+		return r;
+	};
 	auto time_shape = [&](const LineShape &sh) -> float {
 		float ms = 1e30f;
+		cudaGraph_t g = nullptr;
+		cudaGraphExec_t ge = nullptr;
+		if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+			rc = CDR_ERR_CUDA;
+			return ms;
+		}
+		rc = sweep(sh);
+		if (rc == CDR_OK) rc = sweep(sh);
+		if (cudaStreamEndCapture(st, &g) != cudaSuccess && rc == CDR_OK) rc = CDR_ERR_CUDA;
+		if (rc == CDR_OK && cudaGraphInstantiate(&ge, g, 0) != cudaSuccess) rc = CDR_ERR_CUDA;
+		if (g) cudaGraphDestroy(g);
 		for (int rep = 0; rep < 3 && rc == CDR_OK; ++rep) {
-			if ((flush && cudaMemsetAsync(flush, rep, flush_bytes, st) != cudaSuccess) ||
-			    cudaEventRecord(e0, st) != cudaSuccess) {
-				rc = CDR_ERR_CUDA;
-				break;
-			}
-			if (DIR == CDR_DIR_Y && ysync && d.nb == 1 && sh.pair) {  // both colours in one launch
-				rc = sh.K == 16 ? launch_ypair<T, NS, 16>(so, x, b, sor, d, tpitch, CDR_DOWN, sh.cap, ysync, st, false, yc)
-				                : launch_ypair<T, NS, 8>(so, x, b, sor, d, tpitch, CDR_DOWN, sh.cap, ysync, st, false, yc);
-			} else {
-				for (int f = 1; f <= 2 && rc == CDR_OK; ++f)
-					rc = launch_lines<T, NS, DIR>(so, x, b, sor, d, tpitch, f, false, st, &sh, false, yc);
-			}
-			if (rc != CDR_OK) break;
 			float t = 0.f;
-			if (cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-			    cudaEventElapsedTime(&t, e0, e1) != cudaSuccess) {
+			if ((flush && cudaMemsetAsync(flush, rep, flush_bytes, st) != cudaSuccess) ||
+			    cudaEventRecord(e0, st) != cudaSuccess || cudaGraphLaunch(ge, st) != cudaSuccess ||
+			    cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+			    cudaEventElapsedTime(&t, e0, e1) != cudaSuccess)
 				rc = CDR_ERR_CUDA;
-				break;
-			}
 			ms = t < ms ? t : ms;
 		}
+		if (ge) cudaGraphExecDestroy(ge);
 		return ms;
 	};
 	// the default shape stands unless a candidate is at least 5 % faster (10 %
