@@ -230,13 +230,17 @@ __device__ void cc_gs(const CoarseLevel<T> &L, int updown)
 {
 	const size_t ps = (size_t)L.pitch * (L.ny + 2);
 	if (NS == 5) {
-		const int order[4][2] = {{1, 1}, {1, 0}, {0, 1}, {0, 0}};  // (j odd?, i odd?)
-		for (int c = 0; c < 4; ++c) {
-			const int o = updown == CDR_DOWN ? c : 3 - c;
-			const int i0 = order[o][1] ? 1 : 2, j0 = order[o][0] ? 1 : 2;
-			cc_rows(0, (L.nx - i0) / 2, 0, (L.ny - j0) / 2, [&](int a, int b) {
-				gs_at<T, 5>(L.so, ps, L.x, L.b, L.sor, (size_t)(j0 + 2 * b) * L.pitch + i0 + 2 * a, L.pitch);
-			});
+		// DOWN: rows of odd j (0-based), in a row odd then even i, then the rows of even
+		// j; UP: the reverse.  A row's second colour depends on its first only inside
+		// the row, so the row's warp does both: two barriers per sweep instead of four.
+		const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, first = updown == CDR_DOWN ? 1 : 2;
+		for (int h = 0; h < 2; ++h) {
+			for (int j = (h == 0 ? first : 3 - first) + 2 * warp; j <= L.ny; j += 2 * CC_WARPS)
+				for (int c = 0; c < 2; ++c) {
+					for (int i = (c == 0 ? first : 3 - first) + 2 * lane; i <= L.nx; i += 64)
+						gs_at<T, 5>(L.so, ps, L.x, L.b, L.sor, (size_t)j * L.pitch + i, L.pitch);
+					__syncwarp();
+				}
 			__syncthreads();
 		}
 	} else {

@@ -311,13 +311,18 @@ CoarseCycle<T> coarse_desc(std::vector<Level> &lv, int l0, const cdr_gpu_setting
 
 // First level (not the fine one) from which the fused coarse cycle runs: both
 // edges at most fuse_coarse and the level's shared-memory copy within the limit.
+// FP32 cycles fuse from twice that edge: their lines of up to 64 points stay in a
+// warp's registers (a colour under a microsecond), where a level's 15 launches
+// take about 5 us each; FP64 lines run DPTTS2's sequential order there and do not
+// gain.
 template <typename T>
 int pick_fused_level(std::vector<Level> &lv, const cdr_gpu_settings &s)
 {
 	const int L = (int)lv.size();
 	if (s.fuse_coarse <= 0) return -1;
+	const int edge = sizeof(T) == 4 && s.fuse_coarse < 1 << 20 ? 2 * s.fuse_coarse : s.fuse_coarse;
 	for (int l = 1; l + 1 < L; ++l) {
-		if (lv[l].nx > s.fuse_coarse || lv[l].ny > s.fuse_coarse || L - l > kMaxCoarseLevels) continue;
+		if (lv[l].nx > edge || lv[l].ny > edge || L - l > kMaxCoarseLevels) continue;
 		if (coarse_cycle_bytes(coarse_desc<T>(lv, l, s)) <= kCoarseSmemMax) return l;
 	}
 	return -1;
