@@ -1453,32 +1453,31 @@ template int solve_cg_3d<float>(const double *, float *, const float *, Dims3, c
 
 // Outer refinement step of the mixed-precision 3D solve (as the 2D one):
 //   x_out = x_in + e32, r64 = b - A x_out, r32 = (float) r64, ||r64||^2 per
-//   block.  Each thread forms x_in + e32 over its 27-point neighbourhood on the
-//   fly; x_in and x_out are different buffers.  apply = 0 skips e (x_out is then
-//   not needed and may be left unwritten).
+//   block; x_in and x_out are different buffers.  apply = 0 skips e (x_out is
+//   then not needed and may be left unwritten).
+// Seven-point levels: each thread forms x_in + e32 over its neighbours on the fly.
 struct LoadIR3 {
 	const double *__restrict__ x;
 	const float *__restrict__ e;
-	Dims3 F, E;
+	Dims3 F;
 	int apply;
 	__device__ __forceinline__ double operator()(int i, int j, int k) const
 	{
-		const double v = x[F.at1(i, j, k)];
-		return apply ? v + (double)e[E.at1(i, j, k)] : v;
+		const size_t o = F.at1(i, j, k);
+		return apply ? x[o] + (double)e[o] : x[o];
 	}
 };
 
-template <int NS>
-__global__ void __launch_bounds__(TX *TY) k3_ir_residual(const double *__restrict__ so, const double *__restrict__ x,
-                                                         const float *__restrict__ e, const double *__restrict__ b,
-                                                         double *__restrict__ xo, float *__restrict__ r32, Dims3 F,
-                                                         Dims3 E, double *__restrict__ partial, int apply)
+__global__ void __launch_bounds__(TX *TY) k3_ir_residual7(const double *__restrict__ so, const double *__restrict__ x,
+                                                          const float *__restrict__ e, const double *__restrict__ b,
+                                                          double *__restrict__ xo, float *__restrict__ r32, Dims3 F,
+                                                          double *__restrict__ partial, int apply)
 {
 	await_previous();
 	__shared__ double sh[TX * TY / 32];
 	const int tx = (F.nx + TX - 1) / TX, ty = (F.ny + TY - 1) / TY;
 	const long ntiles = (long)tx * ty * F.nz;
-	const LoadIR3 xq{x, e, F, E, apply};
+	const LoadIR3 xq{x, e, F, apply};
 	double acc = 0.0;
 	for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
 		const int kk = (int)(t / ((long)tx * ty));
@@ -1486,9 +1485,9 @@ __global__ void __launch_bounds__(TX *TY) k3_ir_residual(const double *__restric
 		const int i = (rem % tx) * TX + threadIdx.x + 2, j = (rem / tx) * TY + threadIdx.y + 2, k = kk + 2;
 		if (i <= F.nx + 1 && j <= F.ny + 1) {
 			const double xc = xq(i, j, k);
-			const double r = nbs<NS, double>(so, xq, b[F.at1(i, j, k)], F, i, j, k) - SO(i, j, k, KP) * xc;
+			const double r = nb7<double>(so, xq, b[F.at1(i, j, k)], F, i, j, k) - SO(i, j, k, KP) * xc;
 			acc += r * r;
-			r32[E.at1(i, j, k)] = (float)r;
+			r32[F.at1(i, j, k)] = (float)r;
 			xo[F.at1(i, j, k)] = xc;
 		}
 	}
@@ -1509,26 +1508,22 @@ __global__ void __launch_bounds__(256) k3_ir_add(const double *__restrict__ x, c
 
 // 27-point levels form x_out first and then its residual: forming x_in + e for
 // each of the 27 neighbours cost 81 loads and 27 conversions a point (255^3:
-// 1058 us at 32 % of the DRAM rate); the extra read of x_out is 8 of about 156
-// bytes.
+// 1058 us at 32 % of the DRAM rate, now 65 us and about 530); the extra read of
+// x_out is 8 of about 156 bytes.
 int ir_residual_3d(const double *so, const double *x, const float *e, const double *b, double *xo, float *r32,
-                   Dims3 d, Dims3 d32, double *norm_out, double *partial, int apply, cudaStream_t st, int ns)
+                   Dims3 d, double *norm_out, double *partial, int apply, cudaStream_t st, int ns)
 {
 	const long ntiles = (long)ceil_div(d.nx, TX) * ceil_div(d.ny, TY) * d.nz;
 	const int nb = ntiles < 2048 ? (int)ntiles : 2048;
-	if (ns == 14 && d32.pitch == d.pitch) {
+	if (ns == 4) {
+		launch(k3_ir_residual7, nb, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, partial, apply);
+	} else {
 		if (apply) {
 			launch(k3_ir_add, dim3(ceil_div(d.nx, 64), ceil_div(d.ny, 4), d.nz), dim3(64, 4), 0, st, x, e, xo, d);
 			CDR_LAUNCH_CHECK();
 		}
 		launch(k3_residual<double, true, 14, float>, nb, dim3(TX, TY), 0, st, so, apply ? xo : x, b, r32, d, partial);
-		CDR_LAUNCH_CHECK();
-		launch(k3_norm_finish, 1, 1024, 0, st, partial, nb, norm_out);
-		CDR_LAUNCH_CHECK();
-		return CDR_OK;
 	}
-	if (ns == 4) launch(k3_ir_residual<4>, nb, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, d32, partial, apply);
-	else launch(k3_ir_residual<14>, nb, dim3(TX, TY), 0, st, so, x, e, b, xo, r32, d, d32, partial, apply);
 	CDR_LAUNCH_CHECK();
 	launch(k3_norm_finish, 1, 1024, 0, st, partial, nb, norm_out);
 	CDR_LAUNCH_CHECK();

@@ -45,7 +45,7 @@ int setup_cg_3d(const double *so, Dims3 d, double *abd, int *info, cudaStream_t 
 template <typename T>
 int solve_cg_3d(const double *abd, T *x, const T *b, Dims3 d, cudaStream_t st);
 int ir_residual_3d(const double *so, const double *x, const float *e, const double *b, double *xo, float *r32,
-                   Dims3 d, Dims3 d32, double *norm_out, double *partial, int apply, cudaStream_t st, int ns = 14);
+                   Dims3 d, double *norm_out, double *partial, int apply, cudaStream_t st, int ns = 14);
 
 // Plane relaxation data movement (dir 0 = xy, 1 = xz, 2 = yz); plane problems
 // are (n1, n2) grids of row pitch pitch2, problem ipl-1 for plane ipl.

@@ -377,7 +377,7 @@ static int solve3_loaded(cdr_gpu_solver3 *h, int *iters, double *hist, int maxhi
 		CDR_TRY(residual_3d<double>(F.so, F.x, F.b, F.r, F.d, h->norm, h->partial, st, F.ns));
 	} else {
 		CDR_CUDA_TRY(cudaMemcpyAsync(h->x64[0], F.x, sizeof(double) * F.d.plane(), cudaMemcpyDeviceToDevice, st));
-		CDR_TRY(ir_residual_3d(F.so, h->x64[0], F.x32, F.b, h->x64[1], F.b32, F.d, F.d, h->norm, h->partial, 0, st,
+		CDR_TRY(ir_residual_3d(F.so, h->x64[0], F.x32, F.b, h->x64[1], F.b32, F.d, h->norm, h->partial, 0, st,
 		                       F.ns));
 	}
 	CDR_TRY(fetch());
@@ -389,7 +389,7 @@ static int solve3_loaded(cdr_gpu_solver3 *h, int *iters, double *hist, int maxhi
 		} else {
 			CDR_CUDA_TRY(cudaMemsetAsync(F.x32, 0, sizeof(float) * F.d.plane(), st));
 			CDR_TRY(h->run_cycle(1));
-			CDR_TRY(ir_residual_3d(F.so, h->x64[cur], F.x32, F.b, h->x64[1 - cur], F.b32, F.d, F.d, h->norm,
+			CDR_TRY(ir_residual_3d(F.so, h->x64[cur], F.x32, F.b, h->x64[1 - cur], F.b32, F.d, h->norm,
 			                       h->partial, 1, st, F.ns));
 			cur = 1 - cur;
 		}
