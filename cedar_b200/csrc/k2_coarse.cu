@@ -55,14 +55,14 @@ struct CcOffsets {
 	int so, sor, sory, ci, x, b, r;
 };
 // One plane to stage: global source of problem 0, elements between problems,
-// pitches, rows; pairs: rows move as 8-byte FP32 pairs.
+// source pitch, rows of rowlen elements (back to back in shared memory at dst);
+// pairs: rows move as 8-byte FP32 pairs.
 struct CcPlane {
 	const void *src;
-	long long pstride;
-	int spitch, dst, dpitch;
-	short rowlen, rows;
-	int pairs;
+	int pstride, spitch, dst;
+	unsigned short rowlen, rows : 15, pairs : 1;
 };
+static_assert(sizeof(CcPlane) == 24, "one plane of the kernel parameter");
 constexpr int kMaxCcPlanes = 18 * kMaxCoarseLevels;
 // What a launch needs beside the levels, laid out on the host: the levels' x, r
 // and restricted b first (zeroed as one range), then the staged planes, the line
@@ -79,6 +79,9 @@ struct CcPlan {
 template <typename T>
 static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 {
+	// a kernel parameter: within the classic 4 KB (a plane smoother's graph holds
+	// about a hundred of these launches, whose parameters every launch copies)
+	static_assert(sizeof(CcPlan<T>) <= 4096, "plan within 4 KB");
 	CcPlan<T> P;
 	P.cc = cc;
 	size_t at = 0, ln = 0;
@@ -108,12 +111,11 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 			for (int q = 0; q < planes && P.nplanes < kMaxCcPlanes; ++q) {
 				CcPlane &c = P.plane[P.nplanes++];
 				c.src = src + q * splane;
-				c.pstride = (long long)splane * planes;
+				c.pstride = (int)(splane * planes);
 				c.spitch = spitch;
 				c.dst = o + q * rowlen * rows;
-				c.dpitch = rowlen;
-				c.rowlen = (short)rowlen;
-				c.rows = (short)rows;
+				c.rowlen = (unsigned short)rowlen;
+				c.rows = (unsigned short)rows;
 				c.pairs = sizeof(T) == 4 && rowlen % 2 == 0 && spitch % 2 == 0 && c.dst % 2 == 0 &&
 				          c.pstride % 2 == 0 && (uintptr_t)c.src % 8 == 0;
 			}
@@ -125,7 +127,7 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 			const int np = cc_sor_planes(cc.relax);
 			if (np) {
 				P.off[l].sor = stage(L.sor, L.pitch, gpl, ii, jj, np);
-				for (int q = 0; q < np; ++q) P.plane[P.nplanes - 1 - q].pstride = 2 * (long long)gpl;
+				for (int q = 0; q < np; ++q) P.plane[P.nplanes - 1 - q].pstride = 2 * (int)gpl;
 			}
 			if (cc_sory_planes(cc.relax)) P.off[l].sory = stage(L.sory, L.tpitch, (size_t)L.tpitch * ii, jj, ii, 2);
 			const size_t a = (size_t)((L.ny + 1) / 2) * L.nx, b = (size_t)((L.nx + 1) / 2) * L.ny;
@@ -187,7 +189,7 @@ __device__ __forceinline__ void cc_stage(const CcPlan<T> &P, T *base)
 		const T *src = static_cast<const T *>(c.src) + prob * c.pstride;
 		unsigned dst = sbase + (unsigned)c.dst * (unsigned)sizeof(T);
 		const int rowlen = c.rowlen, rows = c.rows, spitch = c.spitch;
-		const unsigned drow = (unsigned)(c.dpitch * (int)sizeof(T));
+		const unsigned drow = (unsigned)(rowlen * (int)sizeof(T));
 		if (sizeof(T) == 4 && c.pairs) {
 			for (int j = 0; j < rows; ++j, src += spitch, dst += drow)
 				for (int i = lane; i < rowlen / 2; i += 32) cp_async<8>(dst + 8 * i, src + 2 * i);

@@ -139,7 +139,7 @@ constexpr size_t kNormScratchBytes = 2048 * sizeof(double);
 // right-hand side and a zero iterate (or, with x0, its iterate) on entry; the last level is the coarsest
 // (banded Cholesky factor abd).  Arrays of a batch lie back to back (problem
 // blockIdx.x * bstep; the pointers are those of the first problem).
-constexpr int kMaxCoarseLevels = 12;
+constexpr int kMaxCoarseLevels = 7;  // 64 points a side down to one
 template <typename T>
 struct CoarseLevel {
 	const T *so = nullptr, *sor = nullptr, *sory = nullptr, *ci = nullptr;
