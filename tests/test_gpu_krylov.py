@@ -160,6 +160,25 @@ def test_fp32_levels_hybrid_cycle_converges(oracle):
     assert abs(len(hist[1]) - len(hist[0])) <= 2
 
 
+@pytest.mark.parametrize("n,f32l", [(101, 2), (101, 3), (101, 4), (400, 4)])
+def test_fp32_levels_below_the_fused_edge(n, f32l):
+    """gpu.fp32-levels whose hand-over lies below the first level that an FP32 cycle would fuse
+    (51^2 and 50^2 here): the coarse levels still run in FP64, fused (line-solve sequential: the
+    same bits as the separate launches) or not, so the histories agree and are not the all-FP32
+    cycle's."""
+    from cedar_b200.solver import Solver2D
+    so, b = P.hetero_diffusion(n, sigma=1.0, n_incl=4, contrast=100.0, aniso=0.5)
+    hist = {}
+    for key in ((32, f32l), (0, f32l), (32, 0)):
+        s = Solver2D(so, Config({"solver": {"relaxation": "line-xy", "max-iter": 4, "tol": 1e-14},
+                                 "gpu": {"precision": "fp32-ir", "line-solve": "sequential", "autotune": False,
+                                         "fuse-coarse": key[0], "fp32-levels": key[1]}}))
+        s.solve(b)
+        hist[key] = s.history.copy()
+    assert np.array_equal(hist[32, f32l], hist[0, f32l])
+    assert not np.array_equal(hist[32, f32l], hist[32, 0])
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32-ir"])
 def test_fcg_residual_replacement(oracle, prec):
     """gpu.fcg-replace = m: the residual is formed as b - A x every m-th
