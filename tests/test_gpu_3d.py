@@ -497,3 +497,29 @@ def test_fused_planes3(lib, oracle, nx, ny, nz, precision):
         assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     else:
         assert out[0][1][-1] < 1e-9 and abs(len(out[0][1]) - len(out[1][1])) <= 1
+
+
+@pytest.mark.parametrize("ns", [14, 4])
+@pytest.mark.parametrize("iters", [1, 2, 3])
+def test_solver3_fp32_ir_keeps_ghost_layer(lib, oracle, ns, iters):
+    """An operator that couples to the ghost layer and an initial guess that holds values there: every
+    step's residual of the refined solve takes them, as the FP64 solve does (norms of the oracle's
+    residual of the returned iterate, which carries the caller's ghosts)."""
+    from cedar_b200.solver import Solver3D
+    n = 17
+    so = make_op3(n, n, n) if ns == 14 else make_op7(n, n, n, seed=3)
+    for plane, axis in ((1, 2), (2, 1), (3, 0)):  # the stored coupling to the point before, first interior layer
+        at = [slice(1, -1)] * 3
+        at[axis] = 1
+        inner = list(at)
+        inner[axis] = 2
+        so[plane][tuple(at)] = so[plane][tuple(inner)]
+    b, x0 = grid3(n, n, n, 5), np.random.default_rng(6).standard_normal((n + 2,) * 3)
+    s = Solver3D(so, Config({"solver": {"relaxation": "point", "max-iter": iters, "tol": 1e-14},
+                             "gpu": {"precision": "fp32-ir"}}))
+    x = s.solve(b, x0.copy())
+    inner = np.zeros(x0.shape, bool)
+    inner[1:-1, 1:-1, 1:-1] = True
+    assert np.array_equal(x[~inner], x0[~inner])
+    rel = oracle.l2norm3(oracle.residual3(so, x, b)) / oracle.l2norm3(oracle.residual3(so, x0, b))
+    assert abs(s.history[-1] - rel) <= 1e-10 * rel
