@@ -99,3 +99,46 @@ def test_batch_rejects_bad_arguments():
     st.relaxation = 7  # a 3D smoother
     assert lib.cdr_gpu_batch2d_create(ctypes.byref(st), ctypes.c_void_p(16), 5, 9, 9, 16, 2, None,
                                       ctypes.byref(h)) == 1
+
+
+@pytest.mark.parametrize("iters", [1, 2, 3])
+def test_refinement_keeps_ghost_layer(oracle, iters):
+    """Operators that couple to the ghost ring and initial guesses that hold values there: every step's
+    residual of a refined solve (single problem, batch, mixed batch) and of flexible CG takes them, as
+    the FP64 solve does, and the returned iterate carries them."""
+    import torch
+    from cedar_b200.solver import BatchSolver2D, MixedBatchSolver2D, Solver2D
+    nx, ny, nb = 31, 25, 3
+    ops, rhs = _batch(nx, ny, nb, 5, seed=60)
+    for so in ops:  # w and s of the first interior column and row couple to the ring
+        so[1][1:-1, 1] = so[1][1:-1, 2]
+        so[2][1, 1:-1] = so[2][2, 1:-1]
+    x0 = [np.random.default_rng(p).standard_normal((ny + 2, nx + 2)) for p in range(nb)]
+    conf = Config({"solver": {"relaxation": "line-xy", "max-iter": iters, "tol": 1e-14},
+                   "gpu": {"precision": "fp32-ir"}})
+
+    def check(x, p, rel):
+        want = np.linalg.norm(oracle.residual(ops[p], x, rhs[p])) / np.linalg.norm(oracle.residual(ops[p], x0[p], rhs[p]))
+        assert abs(rel - want) <= 1e-10 * want
+        ring = np.ones(x.shape, bool)
+        ring[1:-1, 1:-1] = False
+        assert np.array_equal(x[ring], x0[p][ring])
+
+    fcg = [Config({"solver": {"relaxation": "line-xy", "max-iter": iters, "tol": 1e-14},
+                   "gpu": {"precision": prec, "krylov": "fcg"}}) for prec in ("fp64", "fp32-ir")]
+    for p in range(nb):
+        for c in (conf, *fcg):
+            s = Solver2D(ops[p], c)
+            check(s.solve(rhs[p], x0[p]), p, s.history[-1])
+    pitch = ((nx + 2 + 7) // 8) * 8
+    so, b = _device(ops, pitch), _device(rhs, pitch)
+    for mix in (False, True):
+        x = _device(x0, pitch)
+        if mix:
+            s = MixedBatchSolver2D([(so.data_ptr(), 5, nx, ny, pitch, nb)], conf)
+            s.solve_device([b.data_ptr()], [x.data_ptr()])
+        else:
+            s = BatchSolver2D(so.data_ptr(), 5, nx, ny, pitch, nb, conf)
+            s.solve_device(b.data_ptr(), x.data_ptr())
+        for p in range(nb):
+            check(np.ascontiguousarray(host(x)[p, :, :nx + 2]), p, s.rel[p])
