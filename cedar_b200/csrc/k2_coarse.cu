@@ -76,6 +76,9 @@ struct CcPlan {
 	CcPlane plane[kMaxCcPlanes];
 };
 
+// Byte counts stay in size_t until a level is known to fit: the plan is also the
+// fit test for levels of any size, and its table holds ints.  bytes = SIZE_MAX:
+// beyond the shared-memory limit.
 template <typename T>
 static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 {
@@ -84,7 +87,9 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 	static_assert(sizeof(CcPlan<T>) <= 4096, "plan within 4 KB");
 	CcPlan<T> P;
 	P.cc = cc;
+	P.bytes = SIZE_MAX;
 	size_t at = 0, ln = 0;
+	auto fits = [&]() { return at * sizeof(T) <= kCoarseSmemMax; };
 	auto take = [&](size_t n) {
 		const size_t o = at;
 		at += n;
@@ -99,15 +104,17 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 		if (!last) P.off[l].r = take(pl);
 		if (l > 0) P.off[l].b = take(pl);
 	}
+	if (!fits()) return P;
 	P.nzero = (int)at;
 	for (int l = 0; l < cc.nl; ++l) {
 		const CoarseLevel<T> &L = cc.lv[l];
 		const int ii = L.nx + 2, jj = L.ny + 2;
-		const size_t pl = (size_t)ii * jj, gpl = (size_t)L.pitch * jj;
+		const size_t gpl = (size_t)L.pitch * jj;
 		const bool last = l == cc.nl - 1;
 		// planes of one array: rowlen x rows elements each, back to back in shared memory
 		auto stage = [&](const T *src, int spitch, size_t splane, int rowlen, int rows, int planes) {
 			const int o = take((size_t)rowlen * rows * planes);
+			if (!fits()) return o;
 			for (int q = 0; q < planes && P.nplanes < kMaxCcPlanes; ++q) {
 				CcPlane &c = P.plane[P.nplanes++];
 				c.src = src + q * splane;
@@ -127,7 +134,7 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 			const int np = cc_sor_planes(cc.relax);
 			if (np) {
 				P.off[l].sor = stage(L.sor, L.pitch, gpl, ii, jj, np);
-				for (int q = 0; q < np; ++q) P.plane[P.nplanes - 1 - q].pstride = 2 * (int)gpl;
+				for (int q = 0; q < np && fits(); ++q) P.plane[P.nplanes - 1 - q].pstride = 2 * (int)gpl;
 			}
 			if (cc_sory_planes(cc.relax)) P.off[l].sory = stage(L.sory, L.tpitch, (size_t)L.tpitch * ii, jj, ii, 2);
 			const size_t a = (size_t)((L.ny + 1) / 2) * L.nx, b = (size_t)((L.nx + 1) / 2) * L.ny;
@@ -137,9 +144,10 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 		if (l > 0) P.off[l].ci = stage(L.ci, L.pitch, gpl, ii, jj, 8);
 		if (l == 0) P.off[l].b = stage(L.b, L.pitch, gpl, ii, jj, 1);
 		if (l == 0 && cc.x0) P.off[l].x = stage(L.x, L.pitch, gpl, ii, jj, 1);
-		(void)pl;
+		if (!fits()) return P;
 	}
 	P.lines = take(ln);
+	if (!fits()) return P;
 	P.dbl_byte = (int)((at * sizeof(T) + 7) / 8 * 8);
 	const CoarseLevel<T> &Cg = cc.lv[cc.nl - 1];
 	const size_t n = (size_t)Cg.nx * Cg.ny;
@@ -497,7 +505,7 @@ __device__ void cc_smooth(const CoarseCycle<T> &cc, const CoarseLevel<T> &L, int
 template <typename T>
 __device__ void cc_cg(const CoarseLevel<T> &L, double *xs)
 {
-	const int ldab = L.nx + 2, kd = L.nx + 1, n = L.nx * L.ny;
+	const int ldab = L.nx + 2, n = L.nx * L.ny;
 	const double *abs = xs + n;
 	cc_rows(1, L.nx, 1, L.ny, [&](int i, int j) { xs[(j - 1) * L.nx + i - 1] = (double)L.b[(size_t)j * L.pitch + i]; });
 	__syncthreads();
