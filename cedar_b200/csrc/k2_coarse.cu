@@ -63,7 +63,9 @@ struct CcPlane {
 	unsigned short rowlen, rows : 15, pairs : 1;
 };
 static_assert(sizeof(CcPlane) == 24, "one plane of the kernel parameter");
-constexpr int kMaxCcPlanes = 18 * kMaxCoarseLevels;
+// a level stages at most its operator (5), both directions' factors (2 + 2) and
+// its weights (8); the first one b and x in place of the weights
+constexpr int kMaxCcPlanes = (5 + 2 + 2 + 8) * kMaxCoarseLevels;
 // What a launch needs beside the levels, laid out on the host: the levels' x, r
 // and restricted b first (zeroed as one range), then the staged planes, the line
 // right-hand sides, and the coarsest solve's vector and factor in FP64.
@@ -78,7 +80,7 @@ struct CcPlan {
 
 // Byte counts stay in size_t until a level is known to fit: the plan is also the
 // fit test for levels of any size, and its table holds ints.  bytes = SIZE_MAX:
-// beyond the shared-memory limit.
+// beyond the shared-memory limit or the plane table.
 template <typename T>
 static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 {
@@ -89,7 +91,8 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 	P.cc = cc;
 	P.bytes = SIZE_MAX;
 	size_t at = 0, ln = 0;
-	auto fits = [&]() { return at * sizeof(T) <= kCoarseSmemMax; };
+	int nplanes = 0;  // wanted, in the table or not
+	auto fits = [&]() { return at * sizeof(T) <= kCoarseSmemMax && nplanes <= kMaxCcPlanes; };
 	auto take = [&](size_t n) {
 		const size_t o = at;
 		at += n;
@@ -114,8 +117,9 @@ static CcPlan<T> cc_plan(const CoarseCycle<T> &cc)
 		// planes of one array: rowlen x rows elements each, back to back in shared memory
 		auto stage = [&](const T *src, int spitch, size_t splane, int rowlen, int rows, int planes) {
 			const int o = take((size_t)rowlen * rows * planes);
+			nplanes += planes;
 			if (!fits()) return o;
-			for (int q = 0; q < planes && P.nplanes < kMaxCcPlanes; ++q) {
+			for (int q = 0; q < planes; ++q) {
 				CcPlane &c = P.plane[P.nplanes++];
 				c.src = src + q * splane;
 				c.pstride = (int)(splane * planes);

@@ -14,22 +14,22 @@ PROGRAM = r"""
 #include <cstdlib>
 #include "kernels2d.cuh"
 using namespace cdrgpu;
-template <typename T> static unsigned long long bytes(int nx, int ny, int nl, int relax)
+template <typename T> static unsigned long long bytes(int nx, int ny, int nl, int relax, int ns)
 {
 	CoarseCycle<T> cc;
 	cc.nl = nl;
 	cc.relax = relax;
 	for (int l = 0; l < nl; ++l) {
-		cc.lv[l].nx = nx; cc.lv[l].ny = ny; cc.lv[l].ns = 5;
+		cc.lv[l].nx = nx; cc.lv[l].ny = ny; cc.lv[l].ns = ns;
 		cc.lv[l].pitch = (nx + 2 + 31) / 32 * 32; cc.lv[l].tpitch = (ny + 2 + 31) / 32 * 32;
 		nx = (nx - 1) / 2 + 1; ny = (ny - 1) / 2 + 1;
 	}
 	return coarse_cycle_bytes<T>(cc);
 }
-int main(int, char **a)
+int main(int n, char **a)
 {
-	const int nx = atoi(a[2]), ny = atoi(a[3]), nl = atoi(a[4]), relax = atoi(a[5]);
-	printf("%llu %llu\n", a[1][0] == 'd' ? bytes<double>(nx, ny, nl, relax) : bytes<float>(nx, ny, nl, relax),
+	const int nx = atoi(a[2]), ny = atoi(a[3]), nl = atoi(a[4]), relax = atoi(a[5]), ns = n > 6 ? atoi(a[6]) : 5;
+	printf("%llu %llu\n", a[1][0] == 'd' ? bytes<double>(nx, ny, nl, relax, ns) : bytes<float>(nx, ny, nl, relax, ns),
 	       (unsigned long long)kCoarseSmemMax);
 	return 0;
 }
@@ -47,8 +47,8 @@ def program(tmp_path_factory):
                     "-I", os.path.join(cuda, "include"), str(d / "plan.cpp"), "-o", exe, _lib.LIB_PATH,
                     "-Wl,-rpath," + os.path.dirname(_lib.LIB_PATH)], check=True)
 
-    def run(prec, nx, ny, nl, relax):
-        out = subprocess.run([exe, prec] + [str(v) for v in (nx, ny, nl, relax)], capture_output=True, text=True,
+    def run(prec, *numbers):
+        out = subprocess.run([exe, prec] + [str(v) for v in numbers], capture_output=True, text=True,
                              check=True).stdout.split()
         return int(out[0]), int(out[1])
     return run
@@ -89,3 +89,11 @@ def test_fit_test_of_any_size(program, prec, relax):
         got, limit = program(prec, nx, ny, nl, relax)
         want = wanted(prec, nx, ny, nl, relax)
         assert got == want if want <= limit else got > limit, (nx, ny, nl, got, want)
+
+
+def test_more_planes_than_the_table(program):
+    """A hierarchy with more planes to stage than the launch's table holds does not fit, however small."""
+    got, limit = program("f", 20, 20, 5, 3, 5)
+    assert got <= limit
+    got, limit = program("f", 20, 20, 5, 3, 30)  # 4 levels of 30 + 4 planes, 4 of 8, and b
+    assert got > limit
