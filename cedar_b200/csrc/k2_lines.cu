@@ -992,10 +992,12 @@ static int tune_dir(const T *so, T *x, const T *b, const T *sor, Dims2 d, int tp
 	const int TPL = 1 << tpl_log2_of(n, K);
 	const int caps_x[4] = {32, 64, 128, 256};
 	const int caps_y[4] = {TPL, 2 * TPL, 4 * TPL, 8 * TPL};
-	// Each candidate is timed as a cycle runs it: captured in a graph (launches of
-	// the host would add a gap between the colours that a cycle does not have), two
-	// sweeps of both colours after L2 has been overwritten -- the first finds the
-	// level's arrays in DRAM, the second what L2 keeps of them -- best of three.
+	// Each candidate is timed as a cycle runs it: in a graph (launches of the host
+	// would add a gap between the colours that a cycle does not have), two sweeps of
+	// both colours after L2 has been overwritten -- the first finds the level's
+	// arrays in DRAM, the second what L2 keeps of them -- best of three.  The graph
+	// is captured on a stream of its own, since the caller's may be one that cannot
+	// be captured or that other threads use; without it the sweeps are launched.
 	int dev = 0, l2 = 0;
 	CDR_CUDA_TRY(cudaGetDevice(&dev));
 	CDR_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
@@ -1005,39 +1007,58 @@ static int tune_dir(const T *so, T *x, const T *b, const T *sor, Dims2 d, int tp
 		cudaGetLastError();
 		flush = nullptr;
 	}
+	cudaStream_t cst = nullptr;
+	if (cudaStreamCreateWithFlags(&cst, cudaStreamNonBlocking) != cudaSuccess) {
+		cudaGetLastError();
+		cst = nullptr;
+	}
 	cudaEvent_t e0, e1;
 	CDR_CUDA_TRY(cudaEventCreate(&e0));
 	CDR_CUDA_TRY(cudaEventCreate(&e1));
 	int rc = CDR_OK;
-	auto sweep = [&](const LineShape &sh) -> int {
-		if (DIR == CDR_DIR_Y && ysync && d.nb == 1 && sh.pair)  // both colours in one launch
-			return sh.K == 16 ? launch_ypair<T, NS, 16>(so, x, b, sor, d, tpitch, CDR_DOWN, sh.cap, ysync, st, false, yc)
-			                  : launch_ypair<T, NS, 8>(so, x, b, sor, d, tpitch, CDR_DOWN, sh.cap, ysync, st, false, yc);
+	auto sweeps = [&](const LineShape &sh, cudaStream_t q) -> int {  // two
 		int r = CDR_OK;
-		for (int f = 1; f <= 2 && r == CDR_OK; ++f)
-			r = launch_lines<T, NS, DIR>(so, x, b, sor, d, tpitch, f, false, st, &sh, false, yc);
+		for (int it = 0; it < 2 && r == CDR_OK; ++it) {
+			if (DIR == CDR_DIR_Y && ysync && d.nb == 1 && sh.pair) {  // both colours in one launch
+				r = sh.K == 16 ? launch_ypair<T, NS, 16>(so, x, b, sor, d, tpitch, CDR_DOWN, sh.cap, ysync, q, false, yc)
+				               : launch_ypair<T, NS, 8>(so, x, b, sor, d, tpitch, CDR_DOWN, sh.cap, ysync, q, false, yc);
+			} else {
+				for (int f = 1; f <= 2 && r == CDR_OK; ++f)
+					r = launch_lines<T, NS, DIR>(so, x, b, sor, d, tpitch, f, false, q, &sh, false, yc);
+			}
+		}
 		return r;
 	};
 	auto time_shape = [&](const LineShape &sh) -> float {
 		float ms = 1e30f;
 		cudaGraph_t g = nullptr;
 		cudaGraphExec_t ge = nullptr;
-		if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-			rc = CDR_ERR_CUDA;
-			return ms;
+		long long launches = 0;
+		if (cst && cudaStreamBeginCapture(cst, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+			const long long before = cdr_gpu_launch_count();
+			rc = sweeps(sh, cst);
+			launches = cdr_gpu_launch_count() - before;
+			count_launches(-launches);  // captured, not launched
+			if (cudaStreamEndCapture(cst, &g) != cudaSuccess || cudaGraphInstantiate(&ge, g, 0) != cudaSuccess) ge = nullptr;
+			if (g) cudaGraphDestroy(g);
 		}
-		rc = sweep(sh);
-		if (rc == CDR_OK) rc = sweep(sh);
-		if (cudaStreamEndCapture(st, &g) != cudaSuccess && rc == CDR_OK) rc = CDR_ERR_CUDA;
-		if (rc == CDR_OK && cudaGraphInstantiate(&ge, g, 0) != cudaSuccess) rc = CDR_ERR_CUDA;
-		if (g) cudaGraphDestroy(g);
+		if (!ge) cudaGetLastError();  // refused: the sweeps are launched below
 		for (int rep = 0; rep < 3 && rc == CDR_OK; ++rep) {
 			float t = 0.f;
-			if ((flush && cudaMemsetAsync(flush, rep, flush_bytes, st) != cudaSuccess) ||
-			    cudaEventRecord(e0, st) != cudaSuccess || cudaGraphLaunch(ge, st) != cudaSuccess ||
-			    cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
-			    cudaEventElapsedTime(&t, e0, e1) != cudaSuccess)
+			cudaError_t e = flush ? cudaMemsetAsync(flush, rep, flush_bytes, st) : cudaSuccess;
+			if (e == cudaSuccess) e = cudaEventRecord(e0, st);
+			if (ge && e == cudaSuccess) {
+				e = cudaGraphLaunch(ge, st);
+				count_launches(launches);
+			}
+			if (!ge) rc = sweeps(sh, st);
+			if (e == cudaSuccess) e = cudaEventRecord(e1, st);
+			if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+			if (e == cudaSuccess) e = cudaEventElapsedTime(&t, e0, e1);
+			if (e != cudaSuccess && rc == CDR_OK) {
+				set_error(CDR_ERR_CUDA, "line tuner: %s", cudaGetErrorString(e));
 				rc = CDR_ERR_CUDA;
+			}
 			ms = t < ms ? t : ms;
 		}
 		if (ge) cudaGraphExecDestroy(ge);
@@ -1070,6 +1091,7 @@ static int tune_dir(const T *so, T *x, const T *b, const T *sor, Dims2 d, int tp
 	}
 	cudaStreamSynchronize(st);
 	if (flush) cudaFree(flush);
+	if (cst) cudaStreamDestroy(cst);
 	cudaEventDestroy(e0);
 	cudaEventDestroy(e1);
 	if (rc != CDR_OK) return rc;

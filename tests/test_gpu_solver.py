@@ -248,3 +248,29 @@ def test_fcycle_fp32_ir_converges_in_fewer_cycles():
         assert s.history[-1] < 1e-8, cyc
         its[cyc] = s.iters
     assert its["f"] <= its["v"]
+
+
+def test_line_tuner_on_a_stream_that_cannot_be_captured():
+    """Without graphs a solver on the legacy default stream's handle, which refuses captures, is set up
+    with tuned line kernels and solves as on a stream of its own.  The launch counter takes the
+    tuner's launches as they run: three times two sweeps per candidate."""
+    from cedar_b200 import _lib
+    from cedar_b200.solver import Solver2D
+    lib = _lib.load()
+    legacy = 1  # cudaStreamLegacy
+    out = []
+    for stream, nx in ((legacy, 203), (0, 203), (legacy, 205)):
+        so, b = P.hetero_diffusion(nx, sigma=1.0, n_incl=4, contrast=100.0, aniso=0.5)
+        counts = []
+        for tune in (True, False):
+            conf = Config({"solver": {"relaxation": "line-xy", "max-iter": 5, "tol": 1e-14},
+                           "gpu": {"graph": False, "autotune": tune}})
+            before = lib.cdr_gpu_launch_count()
+            s = Solver2D(so, conf, stream=stream)
+            counts.append(lib.cdr_gpu_launch_count() - before)
+            out.append((nx, s.solve(b), s.history.copy()))
+        assert (counts[0] - counts[1]) % 6 == 0
+        assert counts[0] > counts[1] or (stream, nx) == (0, 203)  # shapes are tuned once per process
+    for nx, x, h in out[1:]:
+        if nx == 203:
+            assert np.array_equal(x, out[0][1]) and np.array_equal(h, out[0][2])
