@@ -403,134 +403,12 @@ int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Di
 {
 	dim3 blk(TX, TY);
 	const bool perx = per & 1, pery = (per >> 1) & 1;
-	// Nine-point rows, two colours per launch: W pairs of points per row and segment
-	// (equal segments of at most 256), rows to a block of 128 threads or one longer
-	// row.  A row of three segments or more is a chain of them in one block, so few
-	// such rows leave the chip idle: they go by colours, which tile x as well.  The
-	// line: 32 rows of a parity per segment, two to an SM at most.  Both sides, FP64
-	// us a sweep, colours | rows: 1024 x 128 7.5 | 9.4, x 320 11.0 | 9.6; 2048 x 256
-	// 11.2 | 13.5, x 384 15.4 | 15.1; 4096 x 512 37 | 47, x 640 74 | 58; 16384 x 16
-	// 8.4 | 78, x 256 122 | 164, x 768 348 | 233; FP32 4096 x 256 11.8 | 16.5, 8192 x
-	// 512 45 | 57, x 640 78 | 67.  Within a fifth of the line it costs some levels:
-	// FP64 3000 x 600 29.5 | 32.7, 8192 x 512 124 | 99.  Rows of one or two segments
-	// are the faster ones at any height (700 x 16 8.4 | 6.7).
-	const int nT = d.nx / 2 + 1, nseg = (nT + W - 1) / W, p = d.pitch;
-	auto pair = [&](const T *x, T(&v)[2]) {
-		if constexpr (VEC) {
-			const V2 u = *reinterpret_cast<const V2 *>(x);
-			v[0] = u.x;
-			v[1] = u.y;
-		} else {
-			v[0] = x[0];
-			v[1] = x[1];
-		}
-	};
-	for (int s = 0; s < nseg; ++s) {
-		const int t = (SECOND_A ? s : nseg - 1 - s) * W + t0;
-		const bool live = j <= d.ny && t < nT, va = live && t >= 1, vb = live && 2 * t + 1 <= d.nx;
-		const size_t k = (size_t)j * p + 2 * t;
-		T f[2], ds[2], w[3], s0[2], s1[2], sw0[2], nw0[2], nw1[2], sw1[2], Y[4], M[4], P[4];
-		T first = T(0);
-		// point e (0: a, 1: b) from its row neighbours, in gs_at's operand order
-		auto point = [&](int e, T left, T right) -> T {
-			T acc = madd(w[e], left, f[e]);
-			acc = madd(w[e + 1], right, acc);
-			acc = madd(s0[e], M[1 + e], acc);
-			acc = madd(s1[e], P[1 + e], acc);
-			acc = madd(sw0[e], M[e], acc);
-			acc = madd(nw0[e], M[2 + e], acc);
-			acc = madd(nw1[e], P[e], acc);
-			acc = madd(sw1[e], P[2 + e], acc);
-			return acc * ds[e];
-		};
-		if (live) {
-			auto row4 = [&](const T *x, T(&v)[4]) {  // left neighbour of a, a, b, right neighbour of b
-				T c[2];
-				pair(x, c);
-				v[0] = t >= 1 ? x[-1] : T(0);
-				v[1] = c[0];
-				v[2] = c[1];
-				v[3] = vb ? x[2] : T(0);
-			};
-			auto right = [&](const T *x, T(&v)[2]) {  // a plane at the right neighbours
-				v[0] = x[1];
-				v[1] = vb ? x[2] : T(0);
-			};
-			const T *cw = so + ps + k, *cs = so + 2 * ps + k, *csw = so + 3 * ps + k, *cnw = so + 4 * ps + k;
-			T c[2];
-			pair(cw, c);
-			w[0] = c[0];
-			w[1] = c[1];
-			w[2] = vb ? cw[2] : T(0);
-			pair(cs, s0);
-			pair(cs + p, s1);
-			pair(csw, sw0);
-			right(cnw, nw0);
-			pair(cnw + p, nw1);
-			right(csw + p, sw1);
-			pair(qf + k, f);
-			pair(sor + k, ds);
-			row4(q + k, Y);
-			row4(q + k - p, M);
-			row4(q + k + p, P);
-			// a point outside the interior keeps its value
-			if (SECOND_A) first = vb ? point(1, Y[1], Y[3]) : Y[2];
-			else first = va ? point(0, Y[0], Y[2]) : Y[1];
-		}
-		sh[threadIdx.x] = first;
-		__syncthreads();  // the segment's row is read, its first colour formed
-		if (live) {
-			T second;
-			if (SECOND_A) second = va ? point(0, t0 > 0 ? sh[threadIdx.x - 1] : edge[r], first) : T(0);
-			else second = vb ? point(1, first, t + 1 >= nT ? Y[3] : t0 + 1 < W ? sh[threadIdx.x + 1] : edge[r]) : T(0);
-			const T na = SECOND_A ? second : first, nb = SECOND_A ? first : second;
-			T *qo = q + k;
-			if (VEC && va && vb) {
-				V2 v;
-				v.x = na;
-				v.y = nb;
-				*reinterpret_cast<V2 *>(qo) = v;
-			} else {
-				if (va) qo[0] = na;
-				if (vb) qo[1] = nb;
-			}
-		}
-		if (nseg > 1) {
-			__syncthreads();  // edge and sh are read
-			if (t0 == (SECOND_A ? W - 1 : 0)) edge[r] = first;
-		}
-	}
-}
-
-
-// Periodic branch (BMG2_SymStd_relax_GS.f90:139-226): the reference copies a
-// row's x ghosts after the row's points of a colour and the y ghost rows after
-// the whole sweep.  Points of a colour never read another row's x ghosts that
-// the same colour changes (five-point: no diagonal couplings; nine-point: the
-// rows of one colour are two apart), so one copy launch after each colour
-// launch gives the same values.
-template <typename T>
-int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Dims2 d, int updown,
-                   cudaStream_t st, int per)
-{
-	dim3 blk(TX, TY);
-	const bool perx = per & 1, pery = (per >> 1) & 1;
-	// Nine-point rows, two colours per launch: W pairs of points per row and segment
-	// (equal segments of at most 256), rows to a block of 128 threads or one longer
-	// row.  A row of three segments or more is a chain of them in one block, so few
-	// such rows leave the chip idle: they go by colours, which tile x as well.  The
-	// line: 32 rows of a parity per segment, two to an SM at most.  Both sides, FP64
-	// us a sweep, colours | rows: 1024 x 128 8.7 | 9.5, x 320 9.9 | 9.4; 2048 x 256
-	// 12.5 | 13.8, x 384 15.3 | 14.6; 4096 x 512 37 | 47, x 640 75 | 58; 16384 x 16
-	// 8.8 | 78, x 768 347 | 232; FP32 4096 x 256 12.5 | 16.7, 8192 x 512 46 | 58, x 640
-	// 78 | 67.  Rows of one or two segments are the faster ones at any height (700 x 16
-	// 7.8 | 6.4).
-	const int nT = d.nx / 2 + 1, nseg = ceil_div(nT, 256), W = ceil_div(nT, nseg), R = W < 128 ? 128 / W : 1;
-	const long row_blocks = (long)(d.ny / 2) / R * d.nb;
-	const bool rows = !per && (nseg <= 2 || row_blocks >= (32 * nseg < 296 ? 32 * nseg : 296));
-	if (nstencil == 5 && rows) {
+	if (nstencil == 5 && !per) {
+		// two colours per launch; W pairs of points per row and segment (equal segments
+		// of at most 256), rows to a block of 128 threads or one longer row
 		const bool vec = d.pitch % 2 == 0 &&
 		                 ((uintptr_t)so | (uintptr_t)x | (uintptr_t)b | (uintptr_t)sor) % (2 * sizeof(T)) == 0;
+		const int nT = d.nx / 2 + 1, W = ceil_div(nT, ceil_div(nT, 256)), R = W < 128 ? 128 / W : 1;
 		for (int c = 0; c < 2; ++c) {
 			// DOWN: rows of odd 0-based j first, i odd then even; UP: the reverse
 			const int j0 = (updown == CDR_DOWN) == (c == 0) ? 1 : 2;
