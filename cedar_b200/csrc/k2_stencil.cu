@@ -403,12 +403,23 @@ int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Di
 {
 	dim3 blk(TX, TY);
 	const bool perx = per & 1, pery = (per >> 1) & 1;
-	if (nstencil == 5 && !per) {
-		// two colours per launch; W pairs of points per row and segment (equal segments
-		// of at most 256), rows to a block of 128 threads or one longer row
+	// Nine-point rows, two colours per launch: W pairs of points per row and segment
+	// (equal segments of at most 256), rows to a block of 128 threads or one longer
+	// row.  A row of three segments or more is a chain of them in one block, so few
+	// such rows leave the chip idle: they go by colours, which tile x as well.  The
+	// line: 32 rows of a parity per segment, two to an SM at most.  Both sides, FP64
+	// us a sweep, colours | rows: 1024 x 128 7.5 | 9.4, x 320 11.0 | 9.6; 2048 x 256
+	// 11.2 | 13.5, x 384 15.4 | 15.1; 4096 x 512 37 | 47, x 640 74 | 58; 16384 x 16
+	// 8.4 | 78, x 256 122 | 164, x 768 348 | 233; FP32 4096 x 256 11.8 | 16.5, 8192 x
+	// 512 45 | 57, x 640 78 | 67.  Within a fifth of the line it costs some levels:
+	// FP64 3000 x 600 29.5 | 32.7, 8192 x 512 124 | 99.  Rows of one or two segments
+	// are the faster ones at any height (700 x 16 8.4 | 6.7).
+	const int nT = d.nx / 2 + 1, nseg = ceil_div(nT, 256), W = ceil_div(nT, nseg), R = W < 128 ? 128 / W : 1;
+	const long row_blocks = (long)(d.ny / 2) / R * d.nb;
+	const bool rows = !per && (nseg <= 2 || row_blocks >= (32 * nseg < 296 ? 32 * nseg : 296));
+	if (nstencil == 5 && rows) {
 		const bool vec = d.pitch % 2 == 0 &&
 		                 ((uintptr_t)so | (uintptr_t)x | (uintptr_t)b | (uintptr_t)sor) % (2 * sizeof(T)) == 0;
-		const int nT = d.nx / 2 + 1, W = ceil_div(nT, ceil_div(nT, 256)), R = W < 128 ? 128 / W : 1;
 		for (int c = 0; c < 2; ++c) {
 			// DOWN: rows of odd 0-based j first, i odd then even; UP: the reverse
 			const int j0 = (updown == CDR_DOWN) == (c == 0) ? 1 : 2;

@@ -607,3 +607,22 @@ def test_gs_rows_edges(lib, oracle, nx, ny, extra):
     # two sweeps of 9-term sums of inputs rounded to 2^-24, on values of the size of x and b / c
     size = np.abs(x).max() + np.abs(b * sor).max()
     assert np.abs(host(d32[1])[:, :nx + 2] - x).max() <= 2 * 4 * 10 * 2.0 ** -24 * size
+
+
+@pytest.mark.parametrize("nx,ny", [(1030, 191), (1030, 192), (2050, 319), (2050, 320), (4100, 575), (4100, 576)])
+def test_gs_rows_or_colours(lib, oracle, nx, ny):
+    """Rows of three segments and more at the height where the nine-point sweep goes from single colours
+    to whole rows: FP64 bits of the oracle either way."""
+    rng = np.random.default_rng(nx)
+    so, x, b = np.abs(rng.standard_normal((5, ny + 2, nx + 2))), grid(nx, ny, 1), grid(nx, ny, 2)
+    so[0] += 8.0
+    sor = np.zeros_like(x)
+    sor[1:-1, 1:-1] = 1.0 / so[0][1:-1, 1:-1]
+    both = np.zeros((2,) + x.shape)
+    both[1] = sor
+    dev = [padded(a, nx + 2) for a in (so, x, b, sor)]
+    for updown in (_lib.DOWN, _lib.UP):
+        oracle.relax_gs(so, x, b, both, updown)
+        _lib.check(lib.cdr_gpu_relax_point_2d_f64(ptr(dev[0]), 5, ptr(dev[1]), ptr(dev[2]), ptr(dev[3]), nx, ny, nx + 2,
+                                                  updown, stream()))
+    assert np.array_equal(host(dev[1]), x)
