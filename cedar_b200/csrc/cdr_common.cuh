@@ -84,7 +84,8 @@ inline double &launch_before()
 }
 
 template <typename... P, typename... A>
-inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+inline void launch_as(bool may_be_early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                      A... args)
 {
 	cudaLaunchAttribute attr[1];
 	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -96,9 +97,14 @@ inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
 	cfg.stream = st;
 	cfg.attrs = attr;
 	const LaunchSize z = launch_size(grid, block, smem);
-	cfg.numAttrs = launch_early(z, launch_before()) ? 1 : 0;
+	cfg.numAttrs = may_be_early && launch_early(z, launch_before()) ? 1 : 0;
 	launch_before() = z.sms;
 	(void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // CDR_LAUNCH_CHECK reads the error
+}
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+	launch_as(true, kernel, grid, block, smem, st, args...);
 }
 
 #ifdef __CUDACC__

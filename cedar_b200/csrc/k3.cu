@@ -632,6 +632,22 @@ template int residual_3d<double>(const double *, const double *, const double *,
 template int residual_3d<float>(const float *, const float *, const float *, float *, Dims3, double *, double *,
                                 cudaStream_t, int);
 
+// One colour of the 27-point branch (BMG3_SymStd_relax_GS.f90:94-136): points of
+// parities (pi, pj, pk).
+template <typename T>
+__global__ void __launch_bounds__(TX *TY) k3_gs_colour(const T *__restrict__ so, T *__restrict__ q,
+                                                       const T *__restrict__ qf, const T *__restrict__ sor, Dims3 F,
+                                                       int pi, int pj, int pk)
+{
+	await_previous();
+	const int i = 2 + pi + 2 * (blockIdx.x * TX + threadIdx.x);
+	const int j = 2 + pj + 2 * (blockIdx.y * TY + threadIdx.y);
+	const int k = 2 + pk + 2 * blockIdx.z;
+	if (i > F.nx + 1 || j > F.ny + 1 || k > F.nz + 1) return;
+	const T acc = nb27<T>(so, Load3<T>{q, F}, QF(i, j, k), F, i, j, k);
+	Q(i, j, k) = acc * sor[F.at1(i, j, k)];
+}
+
 // One colour of the seven-point branch of BMG3_SymStd_relax_GS
 // (BMG3_SymStd_relax_GS.f90:141-180): colour pts (0 or 1) holds the points
 // with I + J + K + pts even.
@@ -647,6 +663,26 @@ __global__ void __launch_bounds__(TX *TY) k3_gs7_colour(const T *__restrict__ so
 	Q(i, j, k) = nb7<T>(so, Load3<T>{q, F}, QF(i, j, k), F, i, j, k) * sor[F.at1(i, j, k)];
 }
 
+// Whether a level whose rows cannot be staged goes by single colours, not by rows
+// in nseg segments.  A row of several segments is a chain of them in one block, so
+// rows need many blocks (two to an SM) and a level beyond L2 (126 MB), where each
+// operator line read once instead of twice pays; and about the size of L2 the
+// rows' order keeps less of the level there.  Level sizes count the operator, x, b
+// and 1/c.  Both sides, us a sweep, colours | rows.  One segment: FP64 79^3 (67 MB)
+// 38 | 24, 95^3 54 | 58, 103^3 69 | 84, 111^3 (186 MB) 87 | 95, 119^3 155 | 111; FP32
+// 103^3 (74 MB) 38 | 37, 111^3 43 | 48, 119^3 (115 MB) 53 | 57, 127^3 63 | 62.
+// Several: FP64 8192 x 8 x 8 33 | 319, 700 x 32 x 32 43 | 52, 1024 x 32 x 32 64 | 82,
+// 600 x 64 x 64 210 | 179, 4096 x 24 x 24 202 | 281, 1024 x 64 x 64 346 | 381 (a row
+// pitch of 1026), 1100 x 64 x 64 367 | 337; FP32 1500 x 32 x 32 49 | 75, 600 x 64 x 64
+// 96 | 102, 1500 x 48 x 48 142 | 104.
+template <typename T>
+static bool gs3_by_colours(Dims3 F, int nseg)
+{
+	const double mb = 17e-6 * sizeof(T) * F.nx * F.ny * F.nz, hi = sizeof(T) == 8 ? 190.0 : 126.0;
+	if (nseg == 1) return mb > 84.0 && mb < hi;
+	return mb < hi || (long)(F.ny / 2) * (F.nz / 2) < 296;
+}
+
 template <typename T>
 int relax_point_3d(const T *so, T *x, const T *b, const T *sor, Dims3 F, int updown, cudaStream_t st, int ns)
 {
@@ -660,16 +696,25 @@ int relax_point_3d(const T *so, T *x, const T *b, const T *sor, Dims3 F, int upd
 	}
 	// colours 1..8 (UP) or 8..1 (DOWN) are the parities (i, j, k), i fastest: pairs
 	// of colours share the rows of one (j, k) parity.  Staged rows where they fit
-	// (see staged_ok); else W pairs of points per row and
-	// segment, as many rows to a block of 256 threads as fit; two-element accesses
-	// where rows start aligned.
+	// (see staged_ok); else single colours (see gs3_by_colours) or W pairs of points
+	// per row and segment (equal segments), as many rows to a block of 256 threads as
+	// fit; two-element accesses where rows start aligned.
 	const bool staged = staged_ok<T>(F, so, x, b, sor);
 	const size_t smem = staged_smem<T>(F);
 	if (staged)
 		CDR_TRY(staged_opt_in(updown == CDR_UP ? (const void *)k3_gs_staged<T, true>
 		                                       : (const void *)k3_gs_staged<T, false>, smem));
 	const bool vec = F.pitch % 2 == 0 && aligned_to(2 * sizeof(T), so, x, b, sor);
-	const int W = F.nx / 2 + 1 < 256 ? F.nx / 2 + 1 : 256, R = 256 / W;
+	const int nT = F.nx / 2 + 1, nseg = ceil_div(nT, 256), W = ceil_div(nT, nseg), R = 256 / W;
+	if (!staged && gs3_by_colours<T>(F, nseg)) {
+		const dim3 blk(TX, TY), grd(ceil_div((F.nx + 1) / 2, TX), ceil_div((F.ny + 1) / 2, TY), (F.nz + 1) / 2);
+		for (int c = 0; c < 8; ++c) {  // not early: 300 x 64 x 64 FP64 74 us a sweep, 100 with early launches
+			const int bits = updown == CDR_UP ? c : 7 - c;
+			launch_as(false, k3_gs_colour<T>, grd, blk, 0, st, so, x, b, sor, F, bits & 1, (bits >> 1) & 1, bits >> 2);
+			CDR_LAUNCH_CHECK();
+		}
+		return CDR_OK;
+	}
 	for (int c = 0; c < 4; ++c) {
 		const int bits = updown == CDR_UP ? c : 3 - c, pj = bits & 1, pk = bits >> 1;
 		const int nrj = (F.ny - pj + 1) / 2, nrows = nrj * ((F.nz - pk + 1) / 2);

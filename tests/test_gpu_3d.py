@@ -523,3 +523,21 @@ def test_solver3_fp32_ir_keeps_ghost_layer(lib, oracle, ns, iters):
     assert np.array_equal(x[~inner], x0[~inner])
     rel = oracle.l2norm3(oracle.residual3(so, x, b)) / oracle.l2norm3(oracle.residual3(so, x0, b))
     assert abs(s.history[-1] - rel) <= 1e-10 * rel
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(85, 85, 85), (86, 85, 85), (112, 111, 112), (113, 112, 112),  # one segment, 84 and 190 MB
+                                      (515, 51, 52), (515, 52, 53), (1300, 33, 33), (1300, 34, 36)])  # several: 190 MB, 296 blocks
+def test_gs3_rows_or_colours(lib, oracle, nx, ny, nz):
+    """The 27-point sweep of rows that are not staged, at the sizes where it goes from rows to single
+    colours and back: FP64 bits of the oracle either way."""
+    rng = np.random.default_rng(nx)
+    so, x, b = rng.random((14, nz + 2, ny + 2, nx + 2)), grid3(nx, ny, nz, 3), grid3(nx, ny, nz, 4)
+    so[0] += 27.0
+    sor = oracle.setup_recip3(so)
+    p = nx + 2 + (nx + 1) % 2  # odd: not aligned
+    d = [padded(a, p) for a in (so, x, b, sor)]
+    for updown in (_lib.UP, _lib.DOWN):
+        oracle.relax_gs3(so, x, b, sor, updown)
+        _lib.check(lib.cdr_gpu_relax_point_3d_f64(ptr(d[0]), 14, ptr(d[1]), ptr(d[2]), ptr(d[3]), nx, ny, nz, p, updown,
+                                                  stream()))
+    assert np.array_equal(unpad(d[1], nx), x)
