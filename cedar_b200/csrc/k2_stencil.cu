@@ -425,12 +425,18 @@ int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Di
 			const int j0 = (updown == CDR_DOWN) == (c == 0) ? 1 : 2;
 			if (j0 > d.ny) continue;
 			const dim3 grd(ceil_div((d.ny - j0) / 2 + 1, R), 1, d.nb);
+			// not early where the blocks crowd on the SMs that the launch before leaves free
+			// (early | not, us a sweep): FP64 1200 x 1080 16.2 | 14.5, unaligned 1400 x 1260
+			// 34.7 | 30.8; FP32 1000 x 900 9.6 | 8.5, 2048 x 1024 17.2 | 14.1; but 850 x 765
+			// (40 SMs' worth) 6.7 | 7.5, FP64 2048 x 2048 (103) 74.1 | 75.4
+			const double sms = launch_size(grd, R * W, 0).sms;
+			const bool early = sms < 45.0 || (sizeof(T) == 8 && sms > 90.0);
 			if (updown == CDR_DOWN) {
-				if (vec) launch(k_gs_rows<T, true, true>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
-				else launch(k_gs_rows<T, false, true>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
+				if (vec) launch_as(early, k_gs_rows<T, true, true>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
+				else launch_as(early, k_gs_rows<T, false, true>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
 			} else {
-				if (vec) launch(k_gs_rows<T, true, false>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
-				else launch(k_gs_rows<T, false, false>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
+				if (vec) launch_as(early, k_gs_rows<T, true, false>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
+				else launch_as(early, k_gs_rows<T, false, false>, grd, R * W, 0, st, so, x, b, sor, d, j0, W);
 			}
 			CDR_LAUNCH_CHECK();
 		}
@@ -439,9 +445,12 @@ int relax_point_2d(const T *so, int nstencil, T *x, const T *b, const T *sor, Di
 		// Fortran index 2 is 0-based 1 (odd), 3 is 0-based 2 (even).
 		const int order[4][2] = {{1, 1}, {1, 0}, {0, 1}, {0, 0}};  // (j odd?, i odd?)
 		dim3 grd(ceil_div((d.nx + 1) / 2, TX), ceil_div((d.ny + 1) / 2, TY), d.nb);
+		// FP64 beyond 90 SMs' worth not early, as the rows above (3000 x 300 18.6 | 16.6,
+		// 4096 x 256 18.4 | 17.4; FP32 11.6 | 12.5)
+		const bool early = sizeof(T) == 4 || launch_size(grd, blk, 0).sms <= 90.0;
 		for (int c = 0; c < 4; ++c) {
 			int o = updown == CDR_DOWN ? c : 3 - c;
-			launch(k_gs_colour<T, 5>, grd, blk, 0, st, so, x, b, sor, d, order[o][1], order[o][0]);
+			launch_as(early, k_gs_colour<T, 5>, grd, blk, 0, st, so, x, b, sor, d, order[o][1], order[o][0]);
 			CDR_LAUNCH_CHECK();
 			if (perx) CDR_TRY(ghost_copy_2d<T>(x, d, 1, 1, 0, order[o][0], st));
 		}

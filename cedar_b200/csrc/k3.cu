@@ -726,12 +726,18 @@ int relax_point_3d(const T *so, T *x, const T *b, const T *sor, Dims3 F, int upd
 			continue;
 		}
 		const int grd = ceil_div(nrows, R), blk = R * W;
+		// not early where the blocks crowd on the SMs that the launch before leaves free
+		// (unaligned, early | not, us a sweep): FP64 79^3 26.1 | 23.1; FP32 79^3 21.3 | 19.3,
+		// 300 x 64 x 64 41.3 | 34.8; but 71^3 (22 SMs' worth) 23.9 | 24.2, FP64 119^3 (102)
+		// 111.1 | 113.1
+		const double sms = launch_size(grd, blk, 0).sms;
+		const bool early = sms < 28.0 || sms > 90.0;
 		if (updown == CDR_UP) {
-			if (vec) launch(k3_gs_rows<T, true, true>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
-			else launch(k3_gs_rows<T, false, true>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			if (vec) launch_as(early, k3_gs_rows<T, true, true>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			else launch_as(early, k3_gs_rows<T, false, true>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
 		} else {
-			if (vec) launch(k3_gs_rows<T, true, false>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
-			else launch(k3_gs_rows<T, false, false>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			if (vec) launch_as(early, k3_gs_rows<T, true, false>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
+			else launch_as(early, k3_gs_rows<T, false, false>, grd, blk, 0, st, so, x, b, sor, F, pj, pk, nrj, nrows, W);
 		}
 		CDR_LAUNCH_CHECK();
 	}
