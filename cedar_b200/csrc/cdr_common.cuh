@@ -115,6 +115,12 @@ __device__ __forceinline__ void await_previous()
 {
 	asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }
+// The wait alone: for launches of many short blocks, where letting the next kernel
+// in costs each block more than it hides.  The next one follows when this is done.
+__device__ __forceinline__ void await_previous_only()
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 #endif
 
 #define CDR_CUDA_TRY(expr)                                                          \

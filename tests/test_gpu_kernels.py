@@ -626,3 +626,21 @@ def test_gs_rows_or_colours(lib, oracle, nx, ny):
         _lib.check(lib.cdr_gpu_relax_point_2d_f64(ptr(dev[0]), 5, ptr(dev[1]), ptr(dev[2]), ptr(dev[3]), nx, ny, nx + 2,
                                                   updown, stream()))
     assert np.array_equal(host(dev[1]), x)
+
+
+@pytest.mark.parametrize("nx,ny", [(1300, 896), (1300, 897)])
+def test_gs_five_point_fp32_waves(lib, oracle, nx, ny):
+    """The FP32 red-black sweep on either side of two waves of blocks, within the rounding of its 5-term
+    sums (relative to the oracle's FP64 sweep of the unrounded inputs)."""
+    import torch
+    so, x, b = np.ascontiguousarray(G.diag_diffusion(nx, ny, 1.0, 0.5)), grid(nx, ny, 1), grid(nx, ny, 2)
+    both = np.zeros((2,) + x.shape)
+    both[1, 1:-1, 1:-1] = 1.0 / so[0][1:-1, 1:-1]
+    d = [padded(a, nx + 2).to(torch.float32) for a in (so, x, b, both[1])]
+    for updown in (_lib.DOWN, _lib.UP):
+        oracle.relax_gs(so, x, b, both, updown)
+        _lib.check(lib.cdr_gpu_relax_point_2d_f32(ptr(d[0]), 3, ptr(d[1]), ptr(d[2]), ptr(d[3]), nx, ny, nx + 2, updown,
+                                                  stream()))
+    # two sweeps of 5-term sums of inputs rounded to 2^-24, on values of the size of x and b / c
+    size = np.abs(x).max() + np.abs(b * both[1]).max()
+    assert np.abs(host(d[1]) - x).max() <= 2 * 4 * 6 * 2.0 ** -24 * size
