@@ -826,7 +826,7 @@ static int solve_fcg(cdr_gpu_solver *h, int *iters, double *hist, int maxhist)
 	const size_t bytes = sizeof(double) * F.d.plane();
 	CDR_CUDA_TRY(cudaMemcpyAsync(h->kb, F.b, bytes, cudaMemcpyDeviceToDevice, st));
 	// both buffers: the steps write the interior only, each reads the caller's ghosts
-	for (double *x : h->kx) CDR_CUDA_TRY(cudaMemcpyAsync(x, F.x, bytes, cudaMemcpyDeviceToDevice, st));
+	CDR_TRY(copy_to_both(F.x, h->kx[0], h->kx[1], F.d.plane(), st));
 	CDR_TRY(residual_2d<double>(F.so, F.ns, h->kx[0], h->kb, h->kr, F.d, h->norm, h->partial, st));
 	CDR_CUDA_TRY(cudaMemcpyAsync(h->h_norm, h->norm, sizeof(double), cudaMemcpyDeviceToHost, st));
 	CDR_CUDA_TRY(cudaStreamSynchronize(st));
@@ -903,8 +903,7 @@ static int solve_loaded(cdr_gpu_solver *h, int *iters, double *hist, int maxhist
 		// x64 = x (both: the steps write the interior only, each reads the caller's
 		// ghosts); r = b - A x (FP64), r32 -> level-0 FP32 right-hand side
 		int cur = 0;
-		for (double *x : h->x64)
-			CDR_CUDA_TRY(cudaMemcpyAsync(x, F.x, sizeof(double) * F.d.plane(), cudaMemcpyDeviceToDevice, st));
+		CDR_TRY(copy_to_both(F.x, h->x64[0], h->x64[1], F.d.plane(), st));
 		CDR_TRY(ir_residual_2d(F.so, F.ns, h->x64[0], F.x32, F.b, h->x64[1], F.b32, F.d, F.d, h->norm, h->partial, 0,
 		                       st));
 		CDR_CUDA_TRY(cudaMemcpyAsync(h->h_norm, h->norm, sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -377,8 +377,7 @@ static int solve3_loaded(cdr_gpu_solver3 *h, int *iters, double *hist, int maxhi
 		CDR_TRY(residual_3d<double>(F.so, F.x, F.b, F.r, F.d, h->norm, h->partial, st, F.ns));
 	} else {
 		// both buffers: the steps write the interior only, each reads the caller's ghost layer
-		for (double *x : h->x64)
-			CDR_CUDA_TRY(cudaMemcpyAsync(x, F.x, sizeof(double) * F.d.plane(), cudaMemcpyDeviceToDevice, st));
+		CDR_TRY(copy_to_both(F.x, h->x64[0], h->x64[1], F.d.plane(), st));
 		CDR_TRY(ir_residual_3d(F.so, h->x64[0], F.x32, F.b, h->x64[1], F.b32, F.d, h->norm, h->partial, 0, st,
 		                       F.ns));
 	}
