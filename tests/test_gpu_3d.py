@@ -434,7 +434,7 @@ def test_gs3_rows_edges(lib, oracle, nx, ny, nz, extra):
     so, x, b = make_op3(nx, ny, nz), grid3(nx, ny, nz, 3), grid3(nx, ny, nz, 4)
     sor = oracle.setup_recip3(so)
     sor[~np.isfinite(sor)] = 0.0
-    t = __import__("torch")
+    import torch as t
     p = nx + 2 + (nx + extra) % 2
     d64 = [padded(a, p) for a in (so, x, b, sor)]
     d32 = [a.to(t.float32) for a in d64]
@@ -448,11 +448,12 @@ def test_gs3_rows_edges(lib, oracle, nx, ny, nz, extra):
     assert np.abs(unpad(d32[1], nx) - xr).max() <= 60 * 2.0 ** -24 * max(np.abs(xr).max(), np.abs(x).max()) * 4
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(1, 2, 2), (2, 3, 1), (61, 2, 3), (62, 3, 2), (63, 4, 2), (331, 2, 2), (368, 2, 2),
-                                      (712, 2, 2), (1100, 2, 2)])
+@pytest.mark.parametrize("nx,ny,nz", [(1, 2, 2), (2, 3, 1), (61, 2, 3), (62, 3, 2), (63, 4, 2), (331, 2, 2), (366, 2, 2),
+                                      (367, 2, 2), (368, 2, 2), (712, 2, 2), (734, 2, 2), (735, 2, 2), (1100, 2, 2)])
 def test_staged_rows3_edges(lib, oracle, nx, ny, nz):
-    """Residual (and its norm) and sweep of aligned levels around the limits of the staged rows
-    (whole warps of points, the shared-memory limit in FP64 and FP32) against the oracle's bits."""
+    """Residual (and its norm) and sweep of aligned levels around the limits of the staged rows (whole
+    warps of points; the shared-memory limit, 366 points in FP64 and 734 in FP32): FP64 against
+    the oracle's bits, FP32 within the rounding of its sums."""
     so, x, b = make_op3(nx, ny, nz), grid3(nx, ny, nz, 3), grid3(nx, ny, nz, 4)
     p = -(-(nx + 2) // 4) * 4
     dso, dx, db, dr = padded(so, p), padded(x, p), padded(b, p), padded(np.zeros_like(x), p)
@@ -462,7 +463,7 @@ def test_staged_rows3_edges(lib, oracle, nx, ny, nz):
     ref = oracle.residual3(so, x, b)
     assert np.array_equal(unpad(dr, nx), ref)
     assert abs(host(nrm)[0, 0] - oracle.l2norm3(ref)) <= 1e-13 * oracle.l2norm3(ref)
-    t = __import__("torch")
+    import torch as t
     d32 = [a.to(t.float32) for a in (dso, dx, db)]
     r32 = t.zeros_like(d32[1])
     _lib.check(lib.cdr_gpu_residual_3d_f32(ptr(d32[0]), 14, ptr(d32[1]), ptr(d32[2]), ptr(r32), nx, ny, nz, p, None,
@@ -471,12 +472,44 @@ def test_staged_rows3_edges(lib, oracle, nx, ny, nz):
     scale = np.abs(so).max() * np.abs(x).max() + np.abs(b).max()
     assert np.abs(unpad(r32, nx) - ref).max() <= 28 * 32 * 2.0 ** -24 * scale
     sor = oracle.setup_recip3(so)
-    dsor = padded(sor, p)
+    sor[~np.isfinite(sor)] = 0.0
+    dsor, x0 = padded(sor, p), np.abs(x).max()
+    s32 = dsor.to(t.float32)
     for updown in (_lib.UP, _lib.DOWN):
         oracle.relax_gs3(so, x, b, sor, updown)
         _lib.check(lib.cdr_gpu_relax_point_3d_f64(ptr(dso), 14, ptr(dx), ptr(db), ptr(dsor), nx, ny, nz, p, updown,
                                                   stream()))
+        _lib.check(lib.cdr_gpu_relax_point_3d_f32(ptr(d32[0]), 14, ptr(d32[1]), ptr(d32[2]), ptr(s32), nx, ny, nz, p,
+                                                  updown, stream()))
     assert np.array_equal(unpad(dx, nx), x)
+    # 2 sweeps of 27-term sums: 2 * 30 roundings of 2^-24 on values of the size of x
+    assert np.abs(unpad(d32[1], nx) - x).max() <= 60 * 2.0 ** -24 * max(np.abs(x).max(), x0) * 4
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(30, 50, 45), (62, 47, 44), (366, 46, 46), (735, 46, 46), (1, 1, 1)])
+def test_staged_residual3_norm_fp32(lib, oracle, nx, ny, nz):
+    """The FP32 residual with its norm: staged rows walked by 2048 blocks (more rows than that), one
+    row, and rows that are not staged.  The norm is the FP64 one of the stored residual, in
+    another order of its sum (a relative 1e-12 for up to 1.6 million terms); the residual is the
+    one without a norm, bit for bit, and the FP64 one within the rounding of its sums."""
+    import torch as t
+    rng = np.random.default_rng(nx)
+    so, x, b = rng.standard_normal((14, nz + 2, ny + 2, nx + 2)), grid3(nx, ny, nz, 3), grid3(nx, ny, nz, 4)
+    p = -(-(nx + 2) // 4) * 4
+    d = [padded(a, p).to(t.float32) for a in (so, x, b)]
+    r, plain = t.zeros_like(d[1]), t.zeros_like(d[1])
+    nrm, scratch = padded(np.zeros((1, 1)), 1), padded(np.zeros((1, 2048)), 2048)
+    _lib.check(lib.cdr_gpu_residual_3d_f32(ptr(d[0]), 14, ptr(d[1]), ptr(d[2]), ptr(r), nx, ny, nz, p, ptr(nrm),
+                                           ptr(scratch), stream()))
+    _lib.check(lib.cdr_gpu_residual_3d_f32(ptr(d[0]), 14, ptr(d[1]), ptr(d[2]), ptr(plain), nx, ny, nz, p, None, None,
+                                           stream()))
+    got = unpad(r, nx)
+    assert np.array_equal(got, unpad(plain, nx))
+    want = np.sqrt((got[1:-1, 1:-1, 1:-1] ** 2).sum())
+    assert abs(host(nrm)[0, 0] - want) <= 1e-12 * want
+    ref = oracle.residual3(so, x, b)
+    scale = np.abs(so).max() * np.abs(x).max() + np.abs(b).max()
+    assert np.abs(got - ref)[1:-1, 1:-1, 1:-1].max() <= 28 * 32 * 2.0 ** -24 * scale
 
 
 @pytest.mark.parametrize("nx,ny,nz", [(17, 9, 12), (32, 33, 31), (48, 40, 5), (64, 56, 9), (65, 33, 20)])
