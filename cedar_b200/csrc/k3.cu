@@ -409,6 +409,18 @@ __device__ __forceinline__ void stage_rows(T *rows, int nch, const T *__restrict
 	__syncthreads();
 }
 
+constexpr size_t kStageSmemMax = 104 * 1024;  // two blocks to an SM
+// threads of a block at that limit (a pair of points each, whole warps): 384 in FP32
+// (rows of 734 points), 192 in FP64 (366).  The kernels' launch bounds ask for more,
+// which caps their registers at 64 and 128: with bounds of 384 and 192 threads they
+// take 80 and 168, fewer blocks share an SM, and most sizes lose (FP32 sweep 95^3 20.7
+// -> 22.5 us, 159^3 103.5 -> 105.7, 255^3 365 -> 372, norm 200^3 131 -> 148; FP64 sweep
+// 95^3 40.5 -> 42.9, 255^3 820 -> 750).
+template <typename T>
+constexpr int kStagedThreads =
+    ((int)(kStageSmemMax / (GS_ROWS * 16)) * (16 / (int)sizeof(T)) - 2) / 2 / 32 * 32 + 32;
+static_assert(kStagedThreads<float> == 384 && kStagedThreads<double> == 192, "within the launch bounds");
+
 // k3_gs_rows with the row staged; block = row.
 template <typename T, bool SECOND_A>
 __global__ void __launch_bounds__(512, sizeof(T) == 4 ? 2 : 1)
@@ -532,7 +544,7 @@ __global__ void __launch_bounds__(512, 2)
 {
 	await_previous();
 	extern __shared__ __align__(16) unsigned char k3_raw[];
-	__shared__ double sh[16];
+	__shared__ double sh[kStagedThreads<T> / 32];
 	T *rows = reinterpret_cast<T *>(k3_raw);
 	const int nch = staged_chunks<T>(F), rl = nch * (16 / (int)sizeof(T)), t = threadIdx.x;
 	const bool live = t < F.nx / 2 + 1, va = live && t >= 1, vb = live && 2 * t + 1 <= F.nx;
@@ -566,11 +578,11 @@ __global__ void __launch_bounds__(512, 2)
 }
 
 // Shared memory of a staged row, and whether a level's rows can be staged: one
-// row to a block, two blocks to an SM at the least, rows on 16 bytes.  The
-// sweep is faster so at every size but a narrow middle: 31^3 FP32 15.0 -> 9.3 us
-// a sweep, 95^3 19.8 -> 21.8 (L2 holds the level), 127^3 56.7 -> 44.1, 255^3
-// 445 -> 363; FP64 31^3 17.6 -> 10.9, 63^3 18.0 -> 20.1, 191^3 444 -> 317.
-constexpr size_t kStageSmemMax = 104 * 1024;
+// row to a block, two blocks to an SM at the least, rows on 16 bytes.  Against the
+// rows with loads into registers, us a sweep: FP32 31^3 16.2 -> 8.2, 63^3 16.6 ->
+// 14.4, 95^3 21.7 -> 20.6, 127^3 65 -> 45, 191^3 244 -> 166; FP64 31^3 17.8 -> 9.3,
+// 79^3 27.6 -> 26.4, 95^3 65 -> 40, 127^3 151 -> 116, 191^3 543 -> 323.  At 63^3 FP64
+// alone it was slower (19.1 -> 21.5; single colours 27): not worth a rule.
 template <typename T>
 static size_t staged_smem(Dims3 F)
 {
@@ -579,8 +591,7 @@ static size_t staged_smem(Dims3 F)
 template <typename T, typename... P>
 static bool staged_ok(Dims3 F, const P *...p)
 {
-	return F.pitch % (16 / (int)sizeof(T)) == 0 && F.nx / 2 + 1 <= 512 &&
-	       staged_smem<T>(F) <= kStageSmemMax && aligned_to(16, p...);
+	return F.pitch % (16 / (int)sizeof(T)) == 0 && staged_smem<T>(F) <= kStageSmemMax && aligned_to(16, p...);
 }
 static int staged_block(Dims3 F) { return (F.nx / 2 + 1 + 31) / 32 * 32; }
 // opts a staged kernel into its dynamic shared memory
