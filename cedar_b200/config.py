@@ -9,7 +9,7 @@ solvers, does not change the coarsest-level solve (only its MPI solvers read it)
 GPU options live under the ``"gpu"`` object: ``precision`` ("fp64" | "fp32-ir"),
 ``graph`` (bool), ``fuse-coarse`` (levels with both edges at most this many
 points run as one fused kernel, FP32 levels of single problems and plane smoothers from twice that edge where
-shared memory holds them; 0 = off; default 32), ``line-solve`` ("scan": parallel line substitutions, the
+shared memory holds them, with ``fp32-levels`` none above the hand-over; 0 = off; default 32), ``line-solve`` ("scan": parallel line substitutions, the
 default; "sequential": DPTTRS order, bit-identical to the reference), ``autotune`` (bool, default true: time
 the line kernels' launch shapes per level at setup, once per shape and process), ``line-stream`` (bool,
 default false: x-line sweeps of 256-2048 points by the persistent kernel whose rows arrive in shared memory

@@ -314,17 +314,17 @@ CoarseCycle<T> coarse_desc(std::vector<Level> &lv, int l0, const cdr_gpu_setting
 // FP32 cycles fuse from twice that edge: their lines of up to 64 points stay in a
 // warp's registers (a colour under a microsecond), where a level's 15 launches
 // take about 5 us each; FP64 lines run DPTTS2's sequential order there and do not
-// gain.  The fused cycle ends at the coarsest level, so an FP32 one would run the
-// levels from fp32_levels on in FP32: cycles that hand over to FP64 fuse in FP64
-// only.
+// gain.  The fused cycle ends at the coarsest level, so an FP32 one that began above
+// the hand-over to FP64 (fp32_levels) would skip it: it begins at that level or
+// below, which only an F cycle's first leg reaches in FP32.
 template <typename T>
 int pick_fused_level(std::vector<Level> &lv, const cdr_gpu_settings &s)
 {
 	const int L = (int)lv.size();
 	if (s.fuse_coarse <= 0) return -1;
-	if (sizeof(T) == 4 && s.fp32_levels > 0 && s.fp32_levels < L) return -1;
 	const int edge = sizeof(T) == 4 && s.fuse_coarse < 1 << 20 ? 2 * s.fuse_coarse : s.fuse_coarse;
-	for (int l = 1; l + 1 < L; ++l) {
+	const bool hands_over = sizeof(T) == 4 && s.fp32_levels > 0 && s.fp32_levels < L;
+	for (int l = hands_over ? s.fp32_levels : 1; l + 1 < L; ++l) {
 		if (lv[l].nx > edge || lv[l].ny > edge || L - l > kMaxCoarseLevels) continue;
 		if (coarse_cycle_bytes(coarse_desc<T>(lv, l, s)) <= kCoarseSmemMax) return l;
 	}

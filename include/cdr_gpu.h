@@ -373,7 +373,8 @@ typedef struct cdr_gpu_settings {
 	int use_graph;    /* replay the cycle as a CUDA graph (default 1)                  */
 	int line_flags;   /* CDR_LINES_EXACT: sequential line substitutions; CDR_LINES_NOTUNE (default 0) */
 	int fuse_coarse;  /* levels with both edges <= this run as one fused kernel (default 32, 0 = off); FP32
-	                     levels of single problems and plane smoothers from twice that edge where they fit */
+	                     levels of single problems and plane smoothers from twice that edge where they fit, but
+	                     none above the hand-over of fp32_levels */
 	int krylov;       /* CDR_KRYLOV_NONE (default) or CDR_KRYLOV_FCG; 2D solver only    */
 	int coarse_solve; /* CDR_COARSE_BANDED (default) or CDR_COARSE_INVERSE; 2D solver only */
 	int fp32_levels;  /* CDR_PREC_F32_IR, 2D solver: the FP32 cycle runs this many finest levels in FP32 and

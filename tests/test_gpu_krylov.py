@@ -179,6 +179,23 @@ def test_fp32_levels_below_the_fused_edge(n, f32l):
     assert not np.array_equal(hist[32, f32l], hist[32, 0])
 
 
+@pytest.mark.parametrize("f32l", [1, 3, 5])
+def test_fp32_levels_f_cycle(f32l):
+    """F cycles with gpu.fp32-levels: their first leg reaches levels below the hand-over in FP32, where
+    a fused launch may begin (at 64^2, below it for fp32-levels 1); converging as unfused."""
+    from cedar_b200.solver import Solver2D
+    so, b = P.hetero_diffusion(255, sigma=1.0, n_incl=4, contrast=100.0, aniso=0.5)
+    its = []
+    for fuse in (32, 0):
+        s = Solver2D(so, Config({"solver": {"relaxation": "line-xy", "cycle": {"type": "f"}, "max-iter": 30, "tol": 1e-9},
+                                 "gpu": {"precision": "fp32-ir", "autotune": False, "fuse-coarse": fuse,
+                                         "fp32-levels": f32l}}))
+        s.solve(b)
+        assert s.history[-1] < 1e-9
+        its.append(s.iters)
+    assert abs(its[0] - its[1]) <= 1
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32-ir"])
 def test_fcg_residual_replacement(oracle, prec):
     """gpu.fcg-replace = m: the residual is formed as b - A x every m-th
