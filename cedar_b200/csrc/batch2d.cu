@@ -558,8 +558,9 @@ int cdr_gpu_batch2d_solve_device(cdr_gpu_batch2d *h, const double *b_dev, double
 	double *xw = mixed ? h->x64[0] : F.x;  // the iterate the cycles update
 	CDR_CUDA_TRY(cudaMemcpy2DAsync(xw, F.pitch * sizeof(double), x_dev, pitch * sizeof(double), w, rows,
 	                               cudaMemcpyDeviceToDevice, st));
-	// the refinement's second buffer as well: its steps write the interior only, each reads the caller's ghosts
-	CDR_CUDA_TRY(cudaMemcpyAsync(h->x64[mixed], xw, sizeof(double) * pl * nb, cudaMemcpyDeviceToDevice, st));
+	// the refinement's steps write the interior of the other buffer, each reads the caller's ghosts
+	if (mixed) CDR_TRY(copy_rings(xw, h->x64[1], d, st));
+	else CDR_CUDA_TRY(cudaMemcpyAsync(h->x64[0], F.x, sizeof(double) * pl * nb, cudaMemcpyDeviceToDevice, st));
 	CDR_CUDA_TRY(cudaMemcpyAsync(h->active, h->h_active, sizeof(int) * nb, cudaMemcpyHostToDevice, st));
 	CDR_CUDA_TRY(cudaEventRecord(h->ev[0], st));
 	if (mixed) CDR_TRY(ir_residual_2d(F.so, F.ns, h->x64[0], F.x32, F.b, h->x64[1], F.b32, d, d, h->norm, h->partial, 0, st));

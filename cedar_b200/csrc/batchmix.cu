@@ -558,10 +558,10 @@ int cdr_gpu_batchmix_solve_device(cdr_gpu_batchmix *h, const double *const *b_de
 		const size_t w = (F.nx + 2) * sizeof(double), rows = (size_t)(F.ny + 2) * C.nb;
 		CDR_CUDA_TRY(cudaMemcpy2DAsync(F.b, F.pitch * sizeof(double), b_dev[c], pitch[c] * sizeof(double), w, rows,
 		                               cudaMemcpyDeviceToDevice, st));
-		// both buffers: the steps write the interior only, each reads the caller's ghosts
-		for (double *x : C.x64)
-			CDR_CUDA_TRY(cudaMemcpy2DAsync(x, F.pitch * sizeof(double), x_dev[c], pitch[c] * sizeof(double), w, rows,
-			                               cudaMemcpyDeviceToDevice, st));
+		CDR_CUDA_TRY(cudaMemcpy2DAsync(C.x64[0], F.pitch * sizeof(double), x_dev[c], pitch[c] * sizeof(double), w, rows,
+		                               cudaMemcpyDeviceToDevice, st));
+		// the steps write the interior of the other buffer, each reads the caller's ghosts
+		CDR_TRY(copy_rings(C.x64[0], C.x64[1], F.dims(Sel{0, 1, C.nb}), st));
 		for (int p = 0; p < C.nb; ++p) {
 			iters[first[c] + p] = 0;
 			rel[first[c] + p] = 1.0;

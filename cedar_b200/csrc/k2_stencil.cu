@@ -1189,6 +1189,24 @@ int copy_to_both(const double *x, double *a, double *b, size_t n, cudaStream_t s
 	return CDR_OK;
 }
 
+__global__ void __launch_bounds__(256) k_copy_rings(const double *__restrict__ x, double *__restrict__ y, Dims2 d)
+{
+	await_previous();
+	const int w = d.nx + 2, t = blockIdx.x * 256 + threadIdx.x;
+	if (t >= 2 * w + 2 * d.ny) return;
+	const int s = t - 2 * w;  // rows 0 and ny + 1, then columns 0 and nx + 1
+	const int i = s < 0 ? t % w : s % 2 * (d.nx + 1), j = s < 0 ? t / w * (d.ny + 1) : s / 2 + 1;
+	const size_t k = d.bofs(d.plane()) + d.at(i, j);
+	y[k] = x[k];
+}
+
+int copy_rings(const double *x, double *y, Dims2 d, cudaStream_t st)
+{
+	launch(k_copy_rings, dim3(ceil_div(2 * (d.nx + 2) + 2 * d.ny, 256), 1, d.nb), 256, 0, st, x, y, d);
+	CDR_LAUNCH_CHECK();
+	return CDR_OK;
+}
+
 // Outer refinement step of the mixed-precision solve:
 //   x_out = x_in + e32 on the interior, r64 = b64 - A64 x_out, r32 = (float) r64
 //   and ||r64||^2 per block.  The residual at a point needs the corrected x at

@@ -107,6 +107,8 @@ int solve_cg_inv_2d(const T *ainv, T *x, const T *b, Dims2 d, cudaStream_t st);
 int convert_f64_f32(const double *in, float *out, size_t n, cudaStream_t st);
 // a = b = x (16-byte aligned arrays)
 int copy_to_both(const double *x, double *a, double *b, size_t n, cudaStream_t st);
+// the ghost rings of y = those of x (every problem of a batch)
+int copy_rings(const double *x, double *y, Dims2 d, cudaStream_t st);
 int ir_residual_2d(const double *so, int nstencil, const double *x, const float *e, const double *b, double *xo,
                    float *r32, Dims2 d, Dims2 d32, double *norm_out, double *partial, int apply, cudaStream_t st,
                    const int *active = nullptr);
