@@ -15,9 +15,10 @@
 // compact rows): the operators, smoother factors and interpolation weights are
 // staged once at entry, b of the first level is read and its x written back at
 // exit, and nothing else touches global memory.  Loops map rows to warps and
-// positions to lanes (no per-element division).  Levels of at most 32^2 are
-// fused by default (the levels of the 2047^2 hierarchy below 63^2 need 83 KB in
-// FP32, 166 KB in FP64; from 63^2 on they would not fit).
+// positions to lanes (no per-element division).  By default a cycle of a single
+// problem or a plane fuses the levels of at most 32^2 in FP64 and 64^2 in FP32, as
+// far as shared memory holds them (the callers' rules: pick_fused_level,
+// Batch2::pick_fused); batches fuse from 32^2 in both.
 #include <algorithm>
 
 #include "k2_point.cuh"
